@@ -83,3 +83,25 @@ def test_srgb8_equals_the_exact_oetf_of_the_linear_output(ctx, ref_oetf):
     want = (v * np.float32(255.0) + np.float32(0.5)).to(torch.uint8).cpu().numpy()
     assert len(np.unique(want)) == (248 if ref_oetf else 256)
     np.testing.assert_array_equal(s8, want)
+
+
+# Tiles of the column-walking NLM kernels are 16 rows by 32 - 2P columns (28 for the reference's
+# filter): images smaller than a tile, exactly one, and one pixel more each way; search radii
+# on both sides of the staged pitches (10, 32), patch radii inside and outside 1..3.
+# Tolerance: a weight's exponent is a mean of up to 147 terms, its FP32 error some 20 ulp, and
+# matters up to about 20 (e^-20): 20 * 20 * 2^-24 = 2.4e-5 relative, taken as 1e-4.
+@pytest.mark.parametrize("h,w", [(5, 7), (16, 26), (17, 27), (33, 61)])
+@pytest.mark.parametrize("search_r,patch_r", [(2, 1), (5, 2), (10, 3), (11, 3), (0, 1), (3, 0), (2, 4)])
+def test_variance_nlm_at_tile_edges(ctx, oracle, h, w, search_r, patch_r):
+    rng = np.random.default_rng(1000 * h + 10 * search_r + patch_r)
+    img = rng.random((h, w, 3), dtype=np.float32)
+    var = (0.02 * rng.random((h, w, 3), dtype=np.float32) + 1e-3).astype(np.float32)
+    out = ctx.nlm(img, var, search_r=search_r, patch_r=patch_r, k=0.6)
+    np.testing.assert_allclose(out, oracle.nlm_var(img, var, search_r, patch_r, 0.6), rtol=1e-4, atol=1e-5)
+
+
+# The exponent here is at most about 10 with 25 non-negative terms: 10 * 10 * 2^-24 = 6e-6.
+@pytest.mark.parametrize("h,w", [(3, 5), (16, 28), (17, 29), (40, 57)])
+def test_nlm_ref_at_tile_edges(ctx, oracle, h, w):
+    rgba = np.random.default_rng(h).random((h, w, 4), dtype=np.float32)
+    np.testing.assert_allclose(ctx.nlm_ref(rgba, 0.6), oracle.nlm_ref(rgba, 0.6), rtol=1e-5, atol=1e-6)
