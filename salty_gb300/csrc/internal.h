@@ -303,6 +303,7 @@ struct salty_ctx {
     salty::WaveStore waves;
     salty::BatchArena arena;
     salty::DevBuf<unsigned char> slots;  // SceneSlot table of the current render
+    salty::DevBuf<unsigned char> build_ws;  // BVH build workspace (bvh_build.cu)
 };
 
 namespace salty {

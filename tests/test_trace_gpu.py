@@ -226,3 +226,40 @@ def test_autotune_trace_keeps_results(ctx, gpu_soup_1m):
     gpu_soup_1m.trace_raw(rays, hits)
     np.testing.assert_array_equal(hits.cpu().numpy().view(np.int32), ref)
     ctx.tuning = default
+
+
+def _layout(kind, n):
+    rng = np.random.default_rng(n)
+    if kind == "soup":
+        c = rng.random((n, 3))
+    elif kind == "stacked":    # one centroid: no bin separates anything, halves by position
+        c = np.full((n, 3), 0.5)
+    else:                      # "chain": geometric spacing, each split peels off a few
+        c = np.zeros((n, 3))
+        c[:, 0] = 1.02 ** -np.arange(n)
+    size = 0.02 if kind != "chain" else 0.01 * c[:, :1, None]
+    return (c[:, None, :] + size * (rng.random((n, 3, 3)) - 0.5)).reshape(n, 9).astype(np.float32)
+
+
+# Sizes around the builder's limits: one to a leaf (3), the 8- and 16-lane ranges, a block's
+# subtree (512), a work item of the top levels (2048); every build must give the oracle's hits.
+@pytest.mark.parametrize("kind", ["soup", "stacked", "chain"])
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 8, 9, 16, 17, 33, 512, 513, 2049, 5000])
+@pytest.mark.parametrize("bins,max_leaf", [(32, 3), (8, 1)])
+def test_build_at_size_limits(ctx, oracle, kind, n, bins, max_leaf):
+    tris = _layout(kind, min(n, 2049) if kind == "chain" else n)
+    n = tris.shape[0]
+    rng = np.random.default_rng(5)
+    org = rng.uniform(-1, 2, (512, 3))
+    to = tris.reshape(-1, 3, 3).mean(1)[rng.integers(0, n, 512)] + rng.normal(0, 0.003, (512, 3))
+    rays = np.zeros((512, 8), np.float32)
+    rays[:, :3], rays[:, 4:7] = org, (to - org) / np.linalg.norm(to - org, axis=1, keepdims=True)
+    rays[:, 3], rays[:, 7] = 1e-4, np.inf
+    s = ctx.upload_scene(tris)
+    info = s.build(bins=bins, max_leaf=max_leaf)
+    assert info["n_binary"] <= 2 * n - 1 and info["n_nodes"] >= 1
+    res = s.trace(rays)
+    oid, ot, _, _ = oracle.trace(tris, rays, mode=0)
+    np.testing.assert_array_equal(res.ids, oid)
+    np.testing.assert_array_equal(res.t[oid >= 0], ot[oid >= 0])
+    s.close()
