@@ -24,31 +24,40 @@
 // Every wait is bounded (2 s of the global timer); a wait that gives up sets
 // status[0] |= 1, skips the rest of the strip, frees the CTA's TMEM and returns.
 //
-// k_conv3x3_tma is the same convolution for inputs held in one tensor, as a persistent,
-// warp-specialised kernel (one CTA per SM looping over strips):
+// k_conv3x3_tma is the same convolution as a persistent, warp-specialised kernel (one CTA per
+// SM looping over strips):
 //   warp 0    one lane issues TMA tensor copies (cp.async.bulk.tensor): per 16-channel
 //             chunk the halo (a box of 16 channels x 130 pixels x R+2 rows, the image
-//             border zero-filled by the copy engine) and the weights (16 channels x Npad
-//             rows x 9 taps) into a ring of up to 4 stages, each guarded by a "full"
-//             (transaction bytes) and an "empty" (MMAs done) mbarrier.  A layer whose
-//             weights fit in 48 KB has them copied once, before the first strip, into a
-//             region of their own (its own mbarrier), and its stages hold only halos.  Both land in the
-//             tensor core's 32-byte-swizzled K-major layout: one 32-byte row per pixel (or
-//             weight row), the two 16-byte halves of a row exchanged where address bit 7 is
-//             set.  The MMA unit undoes the exchange from the absolute shared-memory
+//             border zero-filled by the copy engine) and the weights (per kx the three
+//             vertical taps' Npad rows, one after the other) into a ring of up to 4 stages, each
+//             guarded by a "full" (transaction bytes) and an "empty" (MMAs done) mbarrier.  A
+//             layer whose weights fit in kResidentMaxBytes has them copied once, chunk by
+//             chunk, into a region of their own, and its stages hold only halos.  Both land
+//             in the tensor core's 32-byte-swizzled K-major layout: one 32-byte row per pixel
+//             (or weight row), the two 16-byte halves of a row exchanged where address bit 7
+//             is set.  The MMA unit undoes the exchange from the absolute shared-memory
 //             address, so a tap's A operand still starts at any pixel of the halo (32-byte
 //             steps, descriptor base offset 0) -- measured on this GPU with exact integer
 //             products at row offsets 0-131.
-//   warps 1-8 one lane each issues the MMAs of its row of the strip (r = m) and commits
-//             them to the stage's "empty" barrier, and after a strip's last chunk to its
-//             accumulator's barrier: one thread issues an MMA about every 100 cycles,
-//             several issuing threads keep the tensor pipe fed with these small N <= 96
-//             MMAs (measured: 4 issuers 1.35x faster than 1 on the 32-channel layers)
-//   warps 9-12 the epilogue: TMEM -> bias, ReLU, BF16 -> global, one warp per TMEM lane
-//             quarter, then release the accumulator
+//   warp 1    issues the MMAs.  A 128 x N x 16 MMA takes max(32 + N/4, N/2) cycles (measured:
+//             its operands are read from shared memory at 128 bytes a cycle, 4 KB of pixels
+//             and 32 N bytes of weights), so at N = 32 most of it is the pixel operand; the
+//             vertical taps of one halo row therefore run as one MMA of N = up to 3 x Npad
+//             whose columns are three neighbouring rows' accumulators (rows stored in
+//             descending order, so ky ascends with the columns).  Every accumulator still sees
+//             its products in the order chunk, ky, kx.  The whole warp stays converged and one
+//             elected lane issues, which keeps the descriptors in uniform registers: issued
+//             from a single diverged lane an MMA cost 233 cycles, and eight such lanes 46.
+//   warps 2-9 the epilogue: TMEM -> bias, ReLU, BF16 -> global, two warps per TMEM lane
+//             quarter, then release the accumulator; optionally also the 2x2 max-pooled
+//             output (rows paired in the strip, columns by a shuffle)
+//   warps 10-13 (decoder layers only) fill the chunks that come from the coarse level: each
+//             coarse pixel is loaded once and stored to its up to four places in the
+//             swizzled halo, so the up-sampled tensor is never written
 // Two accumulators of R x Npad columns (512 TMEM columns) let the epilogue of one strip
 // overlap the MMAs of the next.  Waits are bounded as above; a wait that gives up raises
 // a shared abort flag that ends every role's loop.
+// Measured (GB300, 1088 x 1920): see the comment at the kernel.
 #include <cuda.h>  // CUtensorMap and its enums (the encoder is fetched from the driver at run time)
 #include <cuda_bf16.h>
 
@@ -283,14 +292,15 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_conv3x3_tc(const TcConvArgs a
 }
 
 // ---------------------------------------------------------------- persistent TMA kernel
-// warp 0: TMA; warps 1..MW: MMA issue (rows r = m, m + MW, ... of a strip for MMA warp m);
-// warps MW+1..MW+4: epilogue
-__host__ __device__ constexpr int tma_threads(int mw) { return 32 * (mw + 5); }
 constexpr int kMaxStages = 4;
-constexpr int kTmaMmaWarps = 8;
+constexpr int kTmaMmaWarps = 1;
+constexpr int kTmaEpiWarps = 8;            // two per TMEM lane quarter
+constexpr int kTmaCoarseWarps = 4;         // expand the coarse level (decoder layers)
+constexpr int kTmaThreads = 32 * (1 + kTmaMmaWarps + kTmaEpiWarps);
+constexpr int kTmaMaxChunks = 16;          // input channel chunks with their own weight barrier
 constexpr int kTmaHeader = 2048;   // barriers, TMEM address, abort flag, bias
 constexpr int kTmaMinSmem = 120 * 1024;  // above half an SM's shared memory: one CTA per SM owns all 512 TMEM columns
-constexpr int kResidentMaxBytes = 48 * 1024;  // weights kept resident up to this size
+constexpr int kResidentMaxBytes = 100 * 1024;  // weights kept resident up to this size
 
 __host__ __device__ constexpr int tma_halo(int R) { return ((R + 2) * kHaloW * 32 + 1023) / 1024 * 1024; }
 __host__ __device__ constexpr int tma_wts(int npad) { return (9 * npad * 32 + 1023) / 1024 * 1024; }
@@ -304,11 +314,14 @@ __device__ __forceinline__ uint64_t sdesc_sw32(uint32_t addr) {
 }
 
 struct TmaConvArgs {
-    int cin, npad, R, cout, relu, out_cs, out_co;
+    int cin, npad, R, cout, relu, out_cs;
     int N, H, W, tiles, stages;
     int resident, wres;  // weights staged once for the whole kernel; bytes reserved for them
     const float* bias;
     bf16* out;
+    bf16* pool;          // 2x2 max-pooled output [N][H/2][W/2][out_cs] or null (R even then)
+    const bf16* coarse;  // decoder layers: input channels [0, coarse_ch) at half resolution
+    int coarse_cs, coarse_ch;
     int* status;
 };
 
@@ -327,11 +340,6 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map
         "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
         :: "r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar) : "memory");
 }
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-        :: "r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(bar) : "memory");
-}
 
 // Bounded wait that also gives up when another role has raised the abort flag.
 __device__ __forceinline__ bool wait_or_abort(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status) {
@@ -348,64 +356,107 @@ __device__ __forceinline__ bool wait_or_abort(uint32_t bar, uint32_t parity, vol
     }
 }
 
-template <int MW>
-__global__ void __launch_bounds__(tma_threads(MW), 1)
+// One lane of the converged warp (always the same one).
+__device__ __forceinline__ uint32_t elect_lane() {
+    uint32_t e;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(e));
+    return e;
+}
+
+// An MMA issued by the elected lane of a converged warp; descriptors as their low words and
+// the common high word.
+__device__ __forceinline__ void umma_elect(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi, uint32_t idesc,
+                                           uint32_t elected, uint32_t accumulate) {
+    asm volatile(
+        "{\n.reg .pred q, p;\n.reg .b64 a, b;\nsetp.ne.b32 q, %5, 0;\nsetp.ne.b32 p, %6, 0;\n"
+        "mov.b64 a, {%1, %3};\nmov.b64 b, {%2, %3};\n"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p;\n}\n"
+        :: "r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(elected), "r"(accumulate));
+}
+__device__ __forceinline__ void umma_commit_elect(uint32_t bar, uint32_t elected) {
+    asm volatile(
+        "{\n.reg .pred q;\nsetp.ne.b32 q, %1, 0;\n"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n"
+        :: "r"(bar), "r"(elected) : "memory");
+}
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status) {
+    return __all_sync(0xffffffffu, wait_or_abort(bar, parity, abort_flag, status));
+}
+
+// 16 BF16 channels of a pixel (32-byte aligned) or 8 of them
+__device__ __forceinline__ void store_pixel16(bf16* p, const uint32_t (&v)[8], bool full) {
+    if (full)
+        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                     :: "l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                     : "memory");
+    else
+        *reinterpret_cast<uint4*>(p) = make_uint4(v[0], v[1], v[2], v[3]);
+}
+
+struct TmaHeader {
+    uint64_t full[kMaxStages], empty[kMaxStages];
+    uint64_t acc_full[2], acc_empty[2];
+    uint64_t wbar[kTmaMaxChunks];  // a resident chunk's weights landed
+    uint32_t tmem;
+    int abort_flag;
+};
+static_assert(sizeof(TmaHeader) <= 512, "the bias table starts at byte 512");
+
+template <bool COARSE>
+__global__ void __launch_bounds__(kTmaThreads + (COARSE ? 32 * kTmaCoarseWarps : 0), 1)
 k_conv3x3_tma(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_w, const TmaConvArgs a) {
     extern __shared__ __align__(1024) unsigned char smem[];
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem);  // [kMaxStages]
-    uint64_t* empty = full + kMaxStages;                 // [kMaxStages]
-    uint64_t* acc_full = empty + kMaxStages;             // [2]
-    uint64_t* acc_empty = acc_full + 2;                  // [2]
-    uint64_t* wbar = acc_empty + 2;                      // resident weights landed
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + 128);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + 132);
-    float* sbias = reinterpret_cast<float*>(smem + 256);  // [npad]
+    TmaHeader& hd = *reinterpret_cast<TmaHeader*>(smem);
+    volatile int* abort_flag = &hd.abort_flag;
+    float* sbias = reinterpret_cast<float*>(smem + 512);  // [npad]
     unsigned char* wres = smem + kTmaHeader;
     unsigned char* ring = smem + kTmaHeader + a.wres;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     // TMA destinations and the descriptors below assume a 1024-byte aligned base
     if (saddr(smem) & 1023u) {
         if (tid == 0) atomicOr(a.status, 2);
         return;
     }
+    constexpr int kFullCount = COARSE ? kTmaCoarseWarps : 1;  // arrivals per "full" phase
     const int R = a.R, npad = a.npad, S = a.stages;
     const int hbytes = tma_halo(R), sbytes = a.resident ? tma_halo(R) : tma_stage(R, npad);
-    const uint32_t tx_bytes = (uint32_t)(R + 2) * kHaloW * 32u + (a.resident ? 0u : 9u * npad * 32u);
-    const int nchunks = a.cin / 16;
+    const uint32_t wchunk = 9u * npad * 32u;                  // one chunk's weights
+    const uint32_t halo_tx = (uint32_t)(R + 2) * kHaloW * 32u;
+    const int nchunks = a.cin / 16, ncoarse = COARSE ? a.coarse_ch / 16 : 0;
     const int strips_x = (a.W + kStrip - 1) / kStrip, strips_y = (a.H + R - 1) / R;
     if (tid == 0) {
         for (int s = 0; s < kMaxStages; ++s) {
-            mbar_init(saddr(full + s), 1);
-            mbar_init(saddr(empty + s), MW);  // one commit per MMA warp
+            mbar_init(saddr(hd.full + s), kFullCount);
+            mbar_init(saddr(hd.empty + s), 1);
         }
         for (int b = 0; b < 2; ++b) {
-            mbar_init(saddr(acc_full + b), MW);
-            mbar_init(saddr(acc_empty + b), 4);  // one arrival per epilogue warp
+            mbar_init(saddr(hd.acc_full + b), 1);
+            mbar_init(saddr(hd.acc_empty + b), kTmaEpiWarps);
         }
-        mbar_init(saddr(wbar), 1);
-        *abort_flag = 0;
+        for (int c = 0; c < kTmaMaxChunks; ++c) mbar_init(saddr(hd.wbar + c), 1);
+        hd.abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    for (int i = tid; i < npad; i += tma_threads(MW)) sbias[i] = (a.bias && i < a.cout) ? a.bias[i] : 0.0f;
+    for (int i = tid; i < npad; i += blockDim.x) sbias[i] = (a.bias && i < a.cout) ? a.bias[i] : 0.0f;
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" :: "r"(saddr(tmem_slot)) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" :: "r"(saddr(&hd.tmem)) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, hd.tmem, 0);
+
+    // weights of chunk c: per kx the three vertical taps' rows
+    auto load_weights = [&](uint32_t dst, int c, uint32_t bar) {
+        for (int kx = 0; kx < 3; ++kx) tma_load_4d(dst + kx * 3 * npad * 32, &tm_w, c * 16, 0, kx, 0, bar);
+    };
 
     if (warp == 0) {
         if (lane == 0) {
             asm volatile("prefetch.tensormap [%0];" :: "l"(reinterpret_cast<uint64_t>(&tm_in)) : "memory");
             asm volatile("prefetch.tensormap [%0];" :: "l"(reinterpret_cast<uint64_t>(&tm_w)) : "memory");
-            // resident weights: every chunk's nine taps once, before the first strip
-            if (a.resident) {
-                mbar_expect_tx(saddr(wbar), (uint32_t)nchunks * 9u * npad * 32u);
-                for (int c = 0; c < nchunks; ++c)
-                    tma_load_3d(saddr(wres) + c * 9 * npad * 32, &tm_w, c * 16, 0, 0, saddr(wbar));
-            }
             int k = 0;
             for (int t = blockIdx.x; t < a.tiles; t += gridDim.x) {
                 int tt = t;
@@ -416,56 +467,75 @@ k_conv3x3_tma(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__
                 const int x0 = sx * kStrip, y0 = sy * R;
                 bool ok = true;
                 for (int c = 0; c < nchunks; ++c, ++k) {
+                    if (a.resident && t == (int)blockIdx.x) {  // the chunk's weights, once
+                        const uint32_t wb = saddr(hd.wbar + c);
+                        mbar_expect_tx(wb, wchunk);
+                        load_weights(saddr(wres) + c * wchunk, c, wb);
+                    }
                     const int s = k % S;
                     const uint32_t ph = (uint32_t)(k / S) & 1u;
-                    if (!wait_or_abort(saddr(empty + s), ph ^ 1u, abort_flag, a.status)) { ok = false; break; }
-                    const uint32_t bar = saddr(full + s);
-                    mbar_expect_tx(bar, tx_bytes);
+                    // every chunk's stage is waited for, whoever fills it: a parity tells two
+                    // successive uses of a stage apart, not a use from the next but one
+                    if (!wait_or_abort(saddr(hd.empty + s), ph ^ 1u, abort_flag, a.status)) { ok = false; break; }
+                    if (c < ncoarse) continue;  // filled by the coarse warps
+                    const uint32_t bar = saddr(hd.full + s);
+                    mbar_expect_tx(bar, halo_tx + (a.resident ? 0u : wchunk));
                     const uint32_t dst = saddr(ring + s * sbytes);
-                    tma_load_4d(dst, &tm_in, c * 16, x0 - 1, y0 - 1, n, bar);
-                    if (!a.resident) tma_load_3d(dst + hbytes, &tm_w, c * 16, 0, 0, bar);
+                    tma_load_4d(dst, &tm_in, c * 16 - (COARSE ? a.coarse_ch : 0), x0 - 1, y0 - 1, n, bar);
+                    if (!a.resident) load_weights(dst + hbytes, c, bar);
+                    for (int i = 1; i < kFullCount; ++i) mbar_arrive(bar);
                 }
                 if (!ok) break;
             }
         }
-    } else if (warp <= MW) {
-        const int m = warp - 1;
-        if (lane == 0 && (!a.resident || wait_or_abort(saddr(wbar), 0u, abort_flag, a.status))) {
-            const uint32_t idesc = idesc_bf16(kStrip, npad);
-            int k = 0, i = 0;
-            for (int t = blockIdx.x; t < a.tiles; t += gridDim.x, ++i) {
-                const int ab = i & 1;
-                if (!wait_or_abort(saddr(acc_empty + ab), ((uint32_t)(i >> 1) & 1u) ^ 1u, abort_flag, a.status)) break;
+    } else if (warp == 1) {
+        const uint32_t el = elect_lane();
+        const uint64_t d0 = sdesc_sw32(0);
+        const uint32_t dlo = (uint32_t)d0, dhi = (uint32_t)(d0 >> 32);
+        const uint32_t idesc = idesc_bf16(kStrip, 0), nbit = (uint32_t)(npad >> 3) << 17;  // + n * nbit: N = n * npad
+        int k = 0, i = 0;
+        for (int t = blockIdx.x; t < a.tiles; t += gridDim.x, ++i) {
+            const int ab = i & 1;
+            if (!warp_wait(saddr(hd.acc_empty + ab), ((uint32_t)(i >> 1) & 1u) ^ 1u, abort_flag, a.status)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t acc = tmem + (uint32_t)ab * 256u;  // row r in columns (R - 1 - r) npad ..
+            bool ok = true;
+            for (int c = 0; c < nchunks; ++c, ++k) {
+                const int s = k % S;
+                if (a.resident && i == 0) ok = warp_wait(saddr(hd.wbar + c), 0u, abort_flag, a.status);
+                if (!ok || !warp_wait(saddr(hd.full + s), (uint32_t)(k / S) & 1u, abort_flag, a.status)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t d0 = tmem + (uint32_t)ab * 256u;
-                bool ok = true;
-                for (int c = 0; c < nchunks; ++c, ++k) {
-                    const int s = k % S;
-                    if (!wait_or_abort(saddr(full + s), (uint32_t)(k / S) & 1u, abort_flag, a.status)) { ok = false; break; }
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t hs = saddr(ring + s * sbytes);
-                    const uint32_t ws = a.resident ? saddr(wres) + c * 9 * npad * 32 : hs + hbytes;
-                    for (int tap = 0; tap < 9; ++tap) {
-                        const int ky = tap / 3, kx = tap - ky * 3;
-                        const uint64_t bd = sdesc_sw32(ws + tap * npad * 32);
-                        for (int r = m; r < R; r += MW) {
-                            const uint64_t ad = sdesc_sw32(hs + ((r + ky) * kHaloW + kx) * 32);
-                            umma_bf16(d0 + r * npad, ad, bd, idesc, (c > 0 || tap > 0) ? 1u : 0u);
-                        }
+                const uint32_t hs = saddr(ring + s * sbytes);
+                const uint32_t ws = a.resident ? saddr(wres) + c * wchunk : hs + hbytes;
+                const uint32_t a0 = dlo + (hs >> 4), b0 = dlo + (ws >> 4);
+                for (int h = 0; h < R + 2; ++h) {
+                    // halo row h is tap ky of output row h - ky
+                    const int ky0 = h < R ? 0 : h - R + 1, n = (h < 2 ? h : 2) - ky0 + 1;
+                    const uint32_t col = acc + (uint32_t)((R - 1 - h + ky0) * npad);
+                    const uint32_t ah = a0 + (uint32_t)(h * kHaloW) * 2u, bh = b0 + (uint32_t)(ky0 * npad) * 2u;
+                    const uint32_t kxs = (uint32_t)(3 * npad) * 2u;
+                    if (c == 0 && ky0 == 0) {  // row h's first products overwrite its columns
+                        umma_elect(col, ah, bh, dhi, idesc + nbit, el, 0u);
+                        if (n > 1)
+                            umma_elect(col + npad, ah, bh + (uint32_t)npad * 2u, dhi, idesc + (uint32_t)(n - 1) * nbit, el, 1u);
+                    } else {
+                        umma_elect(col, ah, bh, dhi, idesc + (uint32_t)n * nbit, el, 1u);
                     }
-                    umma_commit(saddr(empty + s));
+                    umma_elect(col, ah + 2u, bh + kxs, dhi, idesc + (uint32_t)n * nbit, el, 1u);
+                    umma_elect(col, ah + 4u, bh + 2u * kxs, dhi, idesc + (uint32_t)n * nbit, el, 1u);
                 }
-                if (!ok) break;
-                umma_commit(saddr(acc_full + ab));
+                umma_commit_elect(saddr(hd.empty + s), el);
             }
+            if (!ok) break;
+            umma_commit_elect(saddr(hd.acc_full + ab), el);
         }
-    } else {
-        const int q = warp & 3;  // this warp's TMEM lane quarter
+    } else if (!COARSE || warp < 2 + kTmaEpiWarps) {
+        const int q = warp & 3, sub = (warp - 2) >> 2;  // TMEM lane quarter; which of its two warps
+        const int J = npad / 16;
         int i = 0;
         for (int t = blockIdx.x; t < a.tiles; t += gridDim.x, ++i) {
             const int ab = i & 1;
-            const bool got = wait_or_abort(saddr(acc_full + ab), (uint32_t)(i >> 1) & 1u, abort_flag, a.status);
-            if (!__all_sync(0xffffffffu, got)) break;
+            if (!warp_wait(saddr(hd.acc_full + ab), (uint32_t)(i >> 1) & 1u, abort_flag, a.status)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             int tt = t;
             const int sx = tt % strips_x;
@@ -473,33 +543,118 @@ k_conv3x3_tma(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__
             const int sy = tt % strips_y;
             const int n = tt / strips_y;
             const int x = sx * kStrip + q * 32 + lane;
-            for (int r = 0; r < R; ++r) {
-                const int y = sy * R + r;
-                for (int j = 0; j < npad / 16; ++j) {
-                    uint32_t v[16];
-                    tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)ab * 256u + r * npad + j * 16, v);
-                    if (y >= a.H || x >= a.W) continue;
+            const uint32_t acc = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)ab * 256u;
+            // 16 channels of row r of this lane's pixel, stored; left in pk
+            auto item = [&](int r, int j, uint32_t (&pk)[8]) {
+                uint32_t v[16];
+                tmem_ld16(acc + (uint32_t)((R - 1 - r) * npad + j * 16), v);
+                const float4* b4 = reinterpret_cast<const float4*>(sbias + j * 16);
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const int co = j * 16 + h * 8;
-                        if (co >= a.cout) continue;
-                        uint32_t pk[4];
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            float v0 = __uint_as_float(v[h * 8 + 2 * e]) + sbias[co + 2 * e];
-                            float v1 = __uint_as_float(v[h * 8 + 2 * e + 1]) + sbias[co + 2 * e + 1];
-                            if (a.relu) { v0 = fmaxf(v0, 0.0f); v1 = fmaxf(v1, 0.0f); }
-                            const __nv_bfloat162 p2 = __floats2bfloat162_rn(v0, v1);
-                            pk[e] = *reinterpret_cast<const uint32_t*>(&p2);
-                        }
-                        *reinterpret_cast<uint4*>(a.out + (((size_t)n * a.H + y) * a.W + x) * a.out_cs + a.out_co + co) =
-                            make_uint4(pk[0], pk[1], pk[2], pk[3]);
+                for (int e = 0; e < 4; ++e) {
+                    const float4 b = b4[e];
+                    float f0 = __uint_as_float(v[4 * e]) + b.x, f1 = __uint_as_float(v[4 * e + 1]) + b.y;
+                    float f2 = __uint_as_float(v[4 * e + 2]) + b.z, f3 = __uint_as_float(v[4 * e + 3]) + b.w;
+                    if (a.relu) {
+                        f0 = fmaxf(f0, 0.0f); f1 = fmaxf(f1, 0.0f);
+                        f2 = fmaxf(f2, 0.0f); f3 = fmaxf(f3, 0.0f);
                     }
+                    const __nv_bfloat162 p0 = __floats2bfloat162_rn(f0, f1), p1 = __floats2bfloat162_rn(f2, f3);
+                    pk[2 * e] = *reinterpret_cast<const uint32_t*>(&p0);
+                    pk[2 * e + 1] = *reinterpret_cast<const uint32_t*>(&p1);
                 }
+                const int y = sy * R + r;
+                if (y < a.H && x < a.W && j * 16 < a.cout)
+                    store_pixel16(a.out + (((size_t)n * a.H + y) * a.W + x) * a.out_cs + j * 16, pk, j * 16 + 16 <= a.cout);
+            };
+            if (a.pool) {
+                for (int r = 0; r < R; r += 2)
+                    for (int j = 0; j < J; ++j) {
+                        if ((((r >> 1) * J + j) & 1) != sub) continue;
+                        uint32_t p0[8], p1[8];
+                        item(r, j, p0);
+                        item(r + 1, j, p1);
+                        const int y = sy * R + r;
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) {
+                            __nv_bfloat162 m = __hmax2(*reinterpret_cast<__nv_bfloat162*>(&p0[e]),
+                                                       *reinterpret_cast<__nv_bfloat162*>(&p1[e]));
+                            const uint32_t o = __shfl_xor_sync(0xffffffffu, *reinterpret_cast<uint32_t*>(&m), 1);
+                            m = __hmax2(m, *reinterpret_cast<const __nv_bfloat162*>(&o));
+                            p0[e] = *reinterpret_cast<uint32_t*>(&m);
+                        }
+                        if (y < a.H && x < a.W && !(lane & 1) && j * 16 < a.cout)
+                            store_pixel16(a.pool + (((size_t)n * (a.H / 2) + y / 2) * (a.W / 2) + x / 2) * a.out_cs + j * 16,
+                                          p0, j * 16 + 16 <= a.cout);
+                    }
+            } else {
+                for (int r = 0; r < R; ++r)
+                    for (int j = 0; j < J; ++j) {
+                        if (((r * J + j) & 1) != sub) continue;
+                        uint32_t pk[8];
+                        item(r, j, pk);
+                    }
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive(saddr(acc_empty + ab));
+            if (lane == 0) mbar_arrive(saddr(hd.acc_empty + ab));
+        }
+    } else {
+        // coarse chunks: halo pixel (hy, hx) shows coarse pixel ((y0 - 1 + hy) >> 1, (x0 - 1 + hx) >> 1)
+        constexpr int kJobs = 7;  // coarse pixel halves per thread: up to 6 rows x 66 pixels x 2 halves / 128 threads
+        constexpr int kCoarseW = kStrip / 2 + 2;
+        const int ct = tid - kTmaThreads;
+        const int Hc = a.H >> 1, Wc = a.W >> 1;
+        int k = 0;
+        for (int t = blockIdx.x; t < a.tiles; t += gridDim.x) {
+            int tt = t;
+            const int sx = tt % strips_x;
+            tt /= strips_x;
+            const int sy = tt % strips_y;
+            const int n = tt / strips_y;
+            const int x0 = sx * kStrip, y0 = sy * R;
+            const int cy0 = (y0 - 1) >> 1, cx0 = (x0 - 1) >> 1, ncy = ((y0 + R) >> 1) - cy0 + 1;
+            bool ok = true;
+            for (int c = 0; c < nchunks; ++c, ++k) {
+                const int s = k % S;
+                if (c >= ncoarse) {  // filled by TMA; waited for here too (see warp 0)
+                    if (!warp_wait(saddr(hd.empty + s), ((uint32_t)(k / S) & 1u) ^ 1u, abort_flag, a.status)) { ok = false; break; }
+                    continue;
+                }
+                uint4 v[kJobs];
+#pragma unroll
+                for (int u = 0; u < kJobs; ++u) {
+                    const int i = ct + u * 32 * kTmaCoarseWarps, half = i & 1, p = i >> 1;
+                    const int cy = cy0 + p / kCoarseW, cx = cx0 + p % kCoarseW;
+                    v[u] = make_uint4(0, 0, 0, 0);
+                    if (p < ncy * kCoarseW && cy >= 0 && cy < Hc && cx >= 0 && cx < Wc)
+                        v[u] = __ldg(reinterpret_cast<const uint4*>(a.coarse + (((size_t)n * Hc + cy) * Wc + cx) * a.coarse_cs +
+                                                                    c * 16 + half * 8));
+                }
+                if (!warp_wait(saddr(hd.empty + s), ((uint32_t)(k / S) & 1u) ^ 1u, abort_flag, a.status)) { ok = false; break; }
+                const uint32_t bar = saddr(hd.full + s);
+                unsigned char* dst = ring + s * sbytes;
+                if (!a.resident && ct == 0) {
+                    asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" :: "r"(bar), "r"(wchunk) : "memory");
+                    load_weights(saddr(dst + hbytes), c, bar);
+                }
+#pragma unroll
+                for (int u = 0; u < kJobs; ++u) {
+                    const int i = ct + u * 32 * kTmaCoarseWarps, half = i & 1, p = i >> 1;
+                    if (p >= ncy * kCoarseW) continue;
+                    const int hy0 = 2 * (cy0 + p / kCoarseW) - (y0 - 1), hx0 = 2 * (cx0 + p % kCoarseW) - (x0 - 1);
+#pragma unroll
+                    for (int d = 0; d < 4; ++d) {
+                        const int hy = hy0 + (d >> 1), hx = hx0 + (d & 1);
+                        if (hy < 0 || hy >= R + 2 || hx < 0 || hx >= kHaloW) continue;
+                        const int px = hy * kHaloW + hx;
+                        *reinterpret_cast<uint4*>(dst + px * 32 + ((half ^ ((px >> 2) & 1)) << 4)) = v[u];
+                    }
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // these stores -> tensor core reads
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar);
+            }
+            if (!ok) break;
         }
     }
     __syncthreads();
@@ -749,17 +904,24 @@ salty_status conv3x3_tc(salty_ctx* ctx, const ConvSrc& in, int cin, const bf16* 
     return SALTY_OK;
 }
 
-salty_status conv3x3_tma(salty_ctx* ctx, const bf16* in, int in_cs, int cin, const bf16* wt, int wrows,
-                         const float* bias, bf16* out, int out_cs, int out_co, int cout, int N, int H, int W, int relu,
-                         int* d_status) {
+salty_status conv3x3_tma(salty_ctx* ctx, const ConvSrc& in, int cin, const bf16* wt, int wrows, const float* bias,
+                         bf16* out, bf16* pool, int out_cs, int cout, int N, int H, int W, int relu, int* d_status) {
     const int npad = (cout + 15) / 16 * 16;
-    if (cin % 16 || cin <= 0 || cin > in_cs || in_cs % 8 || npad > 256 || npad < 16 || cout % 8 || out_cs % 8 ||
-        out_co % 8 || wrows < 1 || wrows > 256 || reinterpret_cast<uintptr_t>(in) % 16 ||
-        reinterpret_cast<uintptr_t>(wt) % 16)
+    const bool coarse = in.a_ch < cin;  // [up2(a) | b]
+    const bf16* src = coarse ? in.b : in.a;
+    const int src_cs = coarse ? in.b_cs : in.a_cs;
+    auto unaligned = [](const void* p, int by) { return reinterpret_cast<uintptr_t>(p) % by != 0; };
+    if (cin % 16 || cin <= 0 || cin > 16 * kTmaMaxChunks || npad > 256 || npad < 16 || cout % 8 || wrows < 1 || wrows > 256 ||
+        (coarse ? in.a_shift != 1 || in.a_ch % 16 || in.a_cs % 8 || H % 2 || W % 2 || unaligned(in.a, 16)
+                : in.a_shift != 0) ||
+        src_cs % 8 || (cout >= 16 ? out_cs % 16 != 0 : out_cs % 8 != 0) || unaligned(src, 16) || unaligned(wt, 16) ||
+        unaligned(out, 32) || (pool && (unaligned(pool, 32) || H % 2 || W % 2)))
         return ctx->err.fail(SALTY_ERR_INVALID_ARG, "conv3x3_tma: unsupported shape (cin %d, cout %d)", cin, cout);
     EncodeTiledFn enc = tensor_map_encoder();
     if (!enc) return ctx->err.fail(SALTY_ERR_CUDA, "conv3x3_tma: cuTensorMapEncodeTiled is not available");
-    const int R = conv_tc_rows(cout);
+    int R = conv_tc_rows(cout);
+    if (pool && (R & 1)) --R;  // pooled rows are pairs within a strip
+    if (pool && R < 2) return ctx->err.fail(SALTY_ERR_INVALID_ARG, "conv3x3_tma: no pooled output for cout %d", cout);
     // the layer's weights stay in shared memory for the whole kernel when they are small
     const int wbytes = (cin / 16) * 9 * npad * 32;
     const bool resident = wbytes <= kResidentMaxBytes;
@@ -772,29 +934,29 @@ salty_status conv3x3_tma(salty_ctx* ctx, const bf16* in, int in_cs, int cin, con
     if (smem < (size_t)kTmaMinSmem) smem = kTmaMinSmem;
     // input: 4-D (channels, x, y, image), boxes of 16 channels x 130 pixels x R + 2 rows
     CUtensorMap tm_in, tm_w;
-    const cuuint64_t gdim[4] = {(cuuint64_t)in_cs, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)N};
-    const cuuint64_t gstride[3] = {(cuuint64_t)in_cs * 2, (cuuint64_t)W * in_cs * 2, (cuuint64_t)H * W * in_cs * 2};
+    const cuuint64_t gdim[4] = {(cuuint64_t)src_cs, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)N};
+    const cuuint64_t gstride[3] = {(cuuint64_t)src_cs * 2, (cuuint64_t)W * src_cs * 2, (cuuint64_t)H * W * src_cs * 2};
     const cuuint32_t box[4] = {16, (cuuint32_t)kHaloW, (cuuint32_t)(R + 2), 1};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
-    if (enc(&tm_in, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<bf16*>(in), gdim, gstride, box, estr,
+    if (enc(&tm_in, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<bf16*>(src), gdim, gstride, box, estr,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return ctx->err.fail(SALTY_ERR_CUDA, "conv3x3_tma: input tensor map");
-    // weights: 3-D (input channel, row, tap), boxes of 16 channels x npad rows x 9 taps
-    const cuuint64_t wdim[3] = {(cuuint64_t)cin, (cuuint64_t)wrows, 9};
-    const cuuint64_t wstride[2] = {(cuuint64_t)cin * 2, (cuuint64_t)wrows * cin * 2};
-    const cuuint32_t wbox[3] = {16, (cuuint32_t)npad, 9};
-    if (enc(&tm_w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<bf16*>(wt), wdim, wstride, wbox, estr,
+    // weights: 4-D (input channel, row, kx, ky), boxes of 16 channels x npad rows x the three ky
+    const cuuint64_t wdim[4] = {(cuuint64_t)cin, (cuuint64_t)wrows, 3, 3};
+    const cuuint64_t wstride[3] = {(cuuint64_t)cin * 2, (cuuint64_t)wrows * cin * 2, (cuuint64_t)3 * wrows * cin * 2};
+    const cuuint32_t wbox[4] = {16, (cuuint32_t)npad, 1, 3};
+    if (enc(&tm_w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<bf16*>(wt), wdim, wstride, wbox, estr,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return ctx->err.fail(SALTY_ERR_CUDA, "conv3x3_tma: weight tensor map");
-    constexpr int MW = kTmaMmaWarps;
-    SALTY_TRY_CUDA(ctx->err, cudaFuncSetAttribute(k_conv3x3_tma<MW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const long long tiles = (long long)N * ((H + R - 1) / R) * ((W + kStrip - 1) / kStrip);
     const int grid = (int)(tiles < ctx->num_sms ? tiles : ctx->num_sms);
-    TmaConvArgs a{cin, npad, R, cout, relu, out_cs, out_co, N, H, W, (int)tiles, S, resident ? 1 : 0, wres, bias, out,
-                  d_status};
-    k_conv3x3_tma<MW><<<grid, tma_threads(MW), smem, ctx->stream>>>(tm_in, tm_w, a);
+    TmaConvArgs a{cin, npad, R, cout, relu, out_cs, N, H, W, (int)tiles, S, resident ? 1 : 0, wres, bias, out, pool,
+                  coarse ? in.a : nullptr, coarse ? in.a_cs : 0, coarse ? in.a_ch : 0, d_status};
+    auto kern = coarse ? k_conv3x3_tma<true> : k_conv3x3_tma<false>;
+    SALTY_TRY_CUDA(ctx->err, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<grid, kTmaThreads + (coarse ? 32 * kTmaCoarseWarps : 0), smem, ctx->stream>>>(tm_in, tm_w, a);
     SALTY_TRY_CUDA(ctx->err, cudaGetLastError());
     return SALTY_OK;
 }

@@ -734,11 +734,18 @@ void init_layers(Unet& u) {
 }
 
 salty_status launch_conv(salty_ctx* ctx, int kind, const ConvSrc& in, int cin, const bf16* w, int rows, int nt,
-                         const float* bias, bf16* out, int out_cs, int cout, int N, int H, int W, int relu) {
-    if (kind == SALTY_CONV_TCGEN05 && in.a_shift == 0 && in.a_ch >= cin && rows <= 256)
-        return conv3x3_tma(ctx, in.a, in.a_cs, cin, w, rows, bias, out, out_cs, 0, cout, N, H, W, relu,
-                           ctx->status.p + 8);
-    if (kind == SALTY_CONV_TCGEN05 || kind == SALTY_CONV_TCGEN05_CP_ASYNC)
+                         const float* bias, bf16* out, int out_cs, int cout, int N, int H, int W, int relu,
+                         bf16* pool = nullptr) {
+    if (kind == SALTY_CONV_TCGEN05)
+        return conv3x3_tma(ctx, in, cin, w, rows, bias, out, pool, out_cs, cout, N, H, W, relu, ctx->status.p + 8);
+    if (pool) {
+        SALTY_TRY(launch_conv(ctx, kind, in, cin, w, rows, nt, bias, out, out_cs, cout, N, H, W, relu));
+        const long long groups = (long long)N * (H / 2) * (W / 2) * (cout / 8);
+        k_pool<<<gsz(groups), 256, 0, ctx->stream>>>(out, pool, N, H, W, cout);
+        SALTY_TRY_CUDA(ctx->err, cudaGetLastError());
+        return SALTY_OK;
+    }
+    if (kind == SALTY_CONV_TCGEN05_CP_ASYNC)
         return conv3x3_tc(ctx, in, cin, w, rows, bias, out, out_cs, 0, cout, N, H, W, relu, ctx->status.p + 8);
     const int tiles = N * ((W + kTileX - 1) / kTileX) * ((H + kTileY - 1) / kTileY);
     dim3 grid(tiles, rows / (nt * 8));
@@ -831,31 +838,24 @@ salty_status forward(salty_ctx* ctx, Unet& u, const float* d_feat, int N, int H,
     cudaStream_t st = ctx->stream;
     const long long P0 = (long long)N * H * W;
     k_prep_input<<<gsz(P0), 256, 0, st>>>(d_feat, P0, F.t[T_X]);
-    auto conv = [&](int li, const ConvSrc& in, int out, int h, int w) {
+    // pool: the tensor that takes the 2x2 max-pooled output too, or -1
+    auto conv = [&](int li, const ConvSrc& in, int out, int h, int w, int pool = -1) {
         const UnetLayer& L = u.layers[li];
         return launch_conv(ctx, u.conv_kind, in, L.cin, u.wf.p + L.wf_off, L.rows_fwd, L.nt, u.params.p + L.b_off,
-                           F.t[out], L.cout, L.cout, N, h, w, L.relu);
-    };
-    auto pool = [&](int in, int out, int h, int w, int c) {
-        const long long groups = (long long)N * (h / 2) * (w / 2) * (c / 8);
-        k_pool<<<gsz(groups), 256, 0, st>>>(F.t[in], F.t[out], N, h, w, c);
+                           F.t[out], L.cout, L.cout, N, h, w, L.relu, pool >= 0 ? F.t[pool] : nullptr);
     };
     auto x = [&](int t, int c) { return conv_src(F.t[t], c, c); };
     // decoder inputs: [up2(coarse) | skip], read by the convolutions from both tensors
     auto cat = [&](int coarse, int cc, int skip, int cs) { return conv_src_cat(F.t[coarse], cc, F.t[skip], cs); };
     const int H1 = H / 2, W1 = W / 2, H2 = H / 4, W2 = W / 4, H3 = H / 8, W3 = W / 8, H4 = H / 16, W4 = W / 16;
     SALTY_TRY(conv(0, x(T_X, 16), T_A0, H, W));
-    SALTY_TRY(conv(1, x(T_A0, 32), T_E0, H, W));
-    pool(T_E0, T_P0, H, W, 32);
+    SALTY_TRY(conv(1, x(T_A0, 32), T_E0, H, W, T_P0));
     SALTY_TRY(conv(2, x(T_P0, 32), T_A1, H1, W1));
-    SALTY_TRY(conv(3, x(T_A1, 48), T_E1, H1, W1));
-    pool(T_E1, T_P1, H1, W1, 48);
+    SALTY_TRY(conv(3, x(T_A1, 48), T_E1, H1, W1, T_P1));
     SALTY_TRY(conv(4, x(T_P1, 48), T_A2, H2, W2));
-    SALTY_TRY(conv(5, x(T_A2, 64), T_E2, H2, W2));
-    pool(T_E2, T_P2, H2, W2, 64);
+    SALTY_TRY(conv(5, x(T_A2, 64), T_E2, H2, W2, T_P2));
     SALTY_TRY(conv(6, x(T_P2, 64), T_A3, H3, W3));
-    SALTY_TRY(conv(7, x(T_A3, 80), T_E3, H3, W3));
-    pool(T_E3, T_P3, H3, W3, 80);
+    SALTY_TRY(conv(7, x(T_A3, 80), T_E3, H3, W3, T_P3));
     SALTY_TRY(conv(8, x(T_P3, 80), T_B, H4, W4));
     SALTY_TRY(conv(9, cat(T_B, 96, T_E3, 80), T_D3, H3, W3));
     SALTY_TRY(conv(10, cat(T_D3, 80, T_E2, 64), T_D2, H2, W2));

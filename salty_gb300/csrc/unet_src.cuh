@@ -4,7 +4,7 @@
 // [0, a_ch) are the coarse level's, nearest-up-sampled (read at (y >> 1, x >> 1) of an image
 // half as tall and wide), channels [a_ch, cin) the skip connection's at (y, x).  The
 // convolution kernels read both where they stage their input tiles, so the concatenated
-// tensor is never written.  A plain input is source a alone (a_shift 0, a_ch = cin).
+// tensor is never written in a forward pass.  A plain input is source a alone (a_shift 0, a_ch = cin).
 #pragma once
 
 #include <cuda_bf16.h>
@@ -43,10 +43,12 @@ int conv_tc_rows(int cout);
 salty_status conv3x3_tc(salty_ctx* ctx, const ConvSrc& in, int cin, const __nv_bfloat16* wt, int wrows,
                         const float* bias, __nv_bfloat16* out, int out_cs, int out_co, int cout, int N, int H, int W,
                         int relu, int* d_status);
-// The same for an input held in one tensor [N][H][W][in_cs] (16-byte aligned), by TMA in a
-// persistent warp-specialised kernel; wrows <= 256.
-salty_status conv3x3_tma(salty_ctx* ctx, const __nv_bfloat16* in, int in_cs, int cin, const __nv_bfloat16* wt,
-                         int wrows, const float* bias, __nv_bfloat16* out, int out_cs, int out_co, int cout, int N,
+// The same by TMA in a persistent warp-specialised kernel, for an input held in one tensor or
+// a decoder's [up2(coarse) | skip] (16-byte aligned; H and W even then); wrows <= 256, out
+// [N][H][W][out_cs] 32-byte aligned with out_cs % 16 == 0 (cout = 8: % 8).  pool (may be
+// null): also the 2x2 max-pooled output [N][H/2][W/2][out_cs].
+salty_status conv3x3_tma(salty_ctx* ctx, const ConvSrc& in, int cin, const __nv_bfloat16* wt, int wrows,
+                         const float* bias, __nv_bfloat16* out, __nv_bfloat16* pool, int out_cs, int cout, int N,
                          int H, int W, int relu, int* d_status);
 
 // Weight gradient of a 3x3 convolution on tcgen05, deterministic (partial sums per CTA,

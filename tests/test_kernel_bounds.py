@@ -140,3 +140,35 @@ def test_channel_counts_fit_the_sixteen_channel_chunks(launches):
     assert len(cats) >= 4
     for cc, cs in cats:
         assert int(cc) % 16 == 0 and int(cs) % 8 == 0
+
+
+def test_tma_kernel_grouped_taps(k, launches):
+    """k_conv3x3_tma issues the vertical taps of a halo row as one MMA: halo row h, taps
+    ky0..ky0 + n - 1 go to rows h - ky0, h - ky0 - 1, ..., whose accumulators are stored in
+    descending row order.  Every row must get its nine taps, in (ky, kx) order, from
+    weights and pixels inside the stage and columns inside its accumulator."""
+    s = _src("conv_tc.cu")
+    assert _const(s, "kTmaMaxChunks") >= max(c for _, c, _, _ in launches) // 16
+    for kind, cin, cout, wrows in launches:
+        R0, npad = rows(k, cout)
+        for R in {R0, R0 - (R0 & 1)} - {0}:      # pooled outputs take an even number of rows
+            got = {r: [] for r in range(R)}
+            for h in range(R + 2):
+                ky0 = 0 if h < R else h - R + 1
+                n = min(h, 2) - ky0 + 1
+                col = (R - 1 - h + ky0) * npad
+                assert n >= 1 and n * npad <= 256 and n * npad % 16 == 0
+                assert 0 <= col and col + n * npad <= 256
+                for kx in range(3):
+                    # B: rows [ky][npad] of the kx block, A: 128 pixels from (h, kx)
+                    assert (kx * 3 + ky0 + n) * npad * 32 <= 9 * npad * 32
+                    assert (h * k["kHaloW"] + kx) * 32 + k["kStrip"] * 32 <= (R + 2) * k["kHaloW"] * 32
+                    for i in range(n):
+                        r = R - 1 - (col // npad + i)
+                        assert r == h - (ky0 + i)
+                        got[r].append((ky0 + i, kx))
+            assert all(g == [(ky, kx) for ky in range(3) for kx in range(3)] for g in got.values())
+        # coarse pixels of a strip (both halves of 16 channels) against the expanders' jobs
+        jobs = max(((y0 + R0) // 2 - (y0 - 1) // 2 + 1) * (k["kStrip"] // 2 + 2) * 2 for y0 in range(0, 16 * R0, R0))
+        m = re.search(r"constexpr int kJobs = (\d+);", s)
+        assert jobs <= int(m.group(1)) * 32 * _const(s, "kTmaCoarseWarps")
