@@ -57,7 +57,10 @@
 // Two accumulators of R x Npad columns (512 TMEM columns) let the epilogue of one strip
 // overlap the MMAs of the next.  Waits are bounded as above; a wait that gives up raises
 // a shared abort flag that ends every role's loop.
-// Measured (GB300, 1088 x 1920): see the comment at the kernel.
+// Measured (GB300; film denoise at 1080p, 8 symmetries as two batches of 4 images): all
+// convolutions 5.81 -> 3.05 ms against one N = Npad MMA per tap and row from eight diverged
+// lanes, with the decoder inputs staged by k_conv3x3_tc.  The 32 -> 32 layer at full
+// resolution now moves 1.2 GB in 213 us (5.6 TB/s, 0.83 of the copy peak).
 #include <cuda.h>  // CUtensorMap and its enums (the encoder is fetched from the driver at run time)
 #include <cuda_bf16.h>
 
@@ -699,8 +702,9 @@ EncodeTiledFn tensor_map_encoder() {
 // scheduling, unlike atomics.
 //
 // Warp roles: one lane of warp 0 issues the TMA copies of each strip into a ring of
-// kWgStages buffers (a "full" barrier per buffer counts the bytes), one lane of warp 1
-// issues the MMAs and commits them to the buffer's "empty" barrier, and after the last
+// kWgStages buffers (a "full" barrier per buffer counts the bytes), warp 1, converged, issues
+// the MMAs from one elected lane (a diverged lane took about 75 cycles per MMA against 28 of
+// operand reads at M = 64, N = 48; gradients of 16 x 256 x 256: 2.81 -> 2.38 ms) and commits them to the buffer's "empty" barrier, and after the last
 // strip to the accumulator barrier; then all four warps move the accumulators from TMEM to
 // this CTA's slice.  Every wait is bounded.
 constexpr int kWgStrip = 64;
@@ -745,7 +749,7 @@ k_wgrad_tc(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUt
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + 128);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + 132);
     unsigned char* stage0 = smem + kWgHeader;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     if (saddr(smem) & 1023u) {  // the swizzled boxes need 1 KB aligned destinations
         if (tid == 0) atomicOr(a.status, 2);
         return;
@@ -773,7 +777,7 @@ k_wgrad_tc(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUt
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
     bool ok = true;
     if (warp == 0 && lane == 0) {
@@ -796,28 +800,32 @@ k_wgrad_tc(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUt
             for (int k = 0; k < ndy; ++k) tma_load_4d(dyb + k * kWgDyBox, &tm_dy, k * 16, x0, y0, n, bar);
             for (int k = 0; k < nx; ++k) tma_load_4d(xb + k * kWgXBox, &tm_x, c0 + k * 16, x0 - 1, y0 - 1, n, bar);
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1) {  // converged, one elected lane issues (see k_conv3x3_tma)
+        const uint32_t el = elect_lane();
         const uint32_t idesc = idesc_bf16_mn(a.m, ch);
+        const uint64_t da = sdesc_sw32_mn(0, kWgDyBox), db = sdesc_sw32_mn(0, kWgXBox);
+        const uint32_t alo = (uint32_t)da, blo = (uint32_t)db, dhi = (uint32_t)(da >> 32);
         for (int it = 0; it < count; ++it) {
             const int b = it % kWgStages;
-            if (!wait_or_abort(saddr(full + b), (uint32_t)(it / kWgStages) & 1u, abort_flag, a.status)) {
+            if (!warp_wait(saddr(full + b), (uint32_t)(it / kWgStages) & 1u, abort_flag, a.status)) {
                 ok = false;
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t dyb = saddr(stage0 + b * kWgStage), xb = dyb + 8 * kWgDyBox;
+            const uint32_t a0 = alo + (dyb >> 4), b0 = blo + (xb >> 4);
             for (int r = 0; r < kWgRows; ++r)
                 for (int k = 0; k < kWgStrip / 16; ++k) {
-                    const uint64_t ad = sdesc_sw32_mn(dyb + (r * kWgStrip + 16 * k) * 32, kWgDyBox);
-                    for (int tap = 0; tap < 9; ++tap) {
-                        const int ky = tap / 3, kx = tap - ky * 3;
-                        const uint64_t bd = sdesc_sw32_mn(xb + ((r + ky) * kWgHaloW + kx + 16 * k) * 32, kWgXBox);
-                        umma_bf16(tmem + tap * ch, ad, bd, idesc, (it > 0 || r > 0 || k > 0) ? 1u : 0u);
-                    }
+                    const uint32_t ak = a0 + (uint32_t)(r * kWgStrip + 16 * k) * 2u;
+                    const uint32_t bk = b0 + (uint32_t)(r * kWgHaloW + 16 * k) * 2u;
+#pragma unroll
+                    for (int tap = 0; tap < 9; ++tap)
+                        umma_elect(tmem + tap * ch, ak, bk + (uint32_t)((tap / 3) * kWgHaloW + tap % 3) * 2u, dhi, idesc, el,
+                                   (it > 0 || r > 0 || k > 0) ? 1u : 0u);
                 }
-            umma_commit(saddr(empty + b));
+            umma_commit_elect(saddr(empty + b), el);
         }
-        if (ok && count > 0) umma_commit(saddr(acc));
+        if (ok && count > 0) umma_commit_elect(saddr(acc), el);
     }
     __syncwarp();
     // epilogue: TMEM lane (warp * 32 + lane) holds output channel co for every tap
