@@ -330,8 +330,7 @@ salty_status render_batch(salty_ctx* ctx, salty_scene* const* scenes, const salt
 salty_status check_render_opts(salty_ctx* ctx, const salty_scene* sc, const salty_render_opts* o);
 salty_status film_outputs(salty_ctx* ctx, salty_scene* sc, const salty_render_opts& o,
                           float* d_mean, float* d_var, uint8_t* d_srgb);
-salty_status film_features(salty_ctx* ctx, salty_scene* sc, float* d_mean, float* d_var, float* d_albedo,
-                           float* d_normal, float* d_depth);
+salty_status film_records(salty_ctx* ctx, salty_scene* sc, void* d_rec);
 // post.cu
 salty_status tonemap_device(salty_ctx* ctx, int type, int w, int h, const float* d_rgb,
                             float* d_out, uint8_t* d_srgb, int ref_oetf, float* ave, float* mx);

@@ -38,6 +38,9 @@
 #include <cstdlib>
 #include <cstring>
 
+#include <cuda_bf16.h>
+
+#include "film.cuh"
 #include "internal.h"
 
 namespace salty {
@@ -1237,16 +1240,46 @@ __global__ void k_aov_out(const float* __restrict__ aov, long long npx, double c
 }
 
 __global__ void k_film_out(const float* sum, const float* sumsq, const double* sum64, const double* sumsq64,
-                           long long n, double count, float* mean, float* var) {
+                           long long n, FilmScale F, float* mean, float* var) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        double s = sum64 ? sum64[i] : (double)sum[i];
-        double q = sum64 ? sumsq64[i] : (double)sumsq[i];
-        double m = count > 0 ? s / count : 0.0;
-        if (mean) mean[i] = (float)m;
-        if (var) {
-            double v = count > 1 ? (q / count - m * m) * count / (count - 1.0) / count : 0.0;
-            var[i] = (float)(v > 0 ? v : 0.0);
+        float m, v;
+        if (sum64) film_value64(sum64[i], sumsq64[i], F.count, m, v);
+        else film_value(sum[i], sumsq[i], F, m, v);
+        if (mean) mean[i] = m;
+        if (var) var[i] = v;
+    }
+}
+
+// The learned denoiser's input of every film pixel, 16 BF16 channels (32 bytes): log(1 + mean),
+// mean first-hit albedo and normal, 1/(1+t), the noise level mean_c sqrt(var_c) / (1 +
+// mean_c), zeros.
+__global__ void k_film_records(const float* __restrict__ sum, const float* __restrict__ sumsq,
+                               const double* __restrict__ sum64, const double* __restrict__ sumsq64,
+                               const float* __restrict__ aov, float aov_inv, long long npx, FilmScale F,
+                               uint4* __restrict__ rec) {
+    for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < npx; p += (long long)gridDim.x * blockDim.x) {
+        float v[16], noise = 0.0f;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            float m, var;
+            if (sum64) film_value64(sum64[3 * p + c], sumsq64[3 * p + c], F.count, m, var);
+            else film_value(sum[3 * p + c], sumsq[3 * p + c], F, m, var);
+            v[c] = log1pf(fmaxf(m, 0.0f));
+            noise += sqrtf(fmaxf(var, 0.0f)) / (1.0f + fmaxf(m, 0.0f));
         }
+#pragma unroll
+        for (int k = 0; k < 7; ++k) v[3 + k] = aov[7 * p + k] * aov_inv;
+        v[10] = noise * (1.0f / 3.0f);
+#pragma unroll
+        for (int k = 11; k < 16; ++k) v[k] = 0.0f;
+        uint32_t w[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
+            w[k] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+        rec[2 * p] = make_uint4(w[0], w[1], w[2], w[3]);
+        rec[2 * p + 1] = make_uint4(w[4], w[5], w[6], w[7]);
     }
 }
 
@@ -1817,9 +1850,9 @@ salty_status film_outputs(salty_ctx* ctx, salty_scene* sc, const salty_render_op
         SALTY_TRY_CUDA(E, tmp.ensure(n));
         mean = tmp.p;
     }
-    k_film_out<<<ctx->num_sms * 4, 256, 0, ctx->stream>>>(F.fp64 ? nullptr : F.sum.p, F.fp64 ? nullptr : F.sumsq.p,
+    k_film_out<<<grid_of(n, 8, ctx->num_sms), 256, 0, ctx->stream>>>(F.fp64 ? nullptr : F.sum.p, F.fp64 ? nullptr : F.sumsq.p,
                                                          F.fp64 ? F.sum64.p : nullptr, F.fp64 ? F.sumsq64.p : nullptr,
-                                                         n, (double)F.samples, mean, d_var);
+                                                         n, film_scale(F.samples, F.fp64), mean, d_var);
     SALTY_TRY_CUDA(E, cudaGetLastError());
     if (d_srgb) {
         int tm = o.tonemap < 0 ? SALTY_TM_REINHARD : o.tonemap;
@@ -1828,20 +1861,16 @@ salty_status film_outputs(salty_ctx* ctx, salty_scene* sc, const salty_render_op
     return SALTY_OK;
 }
 
-// Mean, variance of the mean and mean first-hit features of the film, all on the device
-// (any output may be null).  The film must hold samples.
-salty_status film_features(salty_ctx* ctx, salty_scene* sc, float* d_mean, float* d_var, float* d_albedo,
-                           float* d_normal, float* d_depth) {
+// The learned denoiser's input records of the film (k_film_records; 32 bytes per pixel).
+// The film must hold samples.
+salty_status film_records(salty_ctx* ctx, salty_scene* sc, void* d_rec) {
     Film& F = sc->film;
     const long long npx = (long long)F.width * F.height;
     if (npx == 0 || F.samples == 0 || !F.aov.p) return ctx->err.fail(SALTY_ERR_NOT_BUILT, "the film is empty");
-    if (d_mean || d_var)
-        k_film_out<<<ctx->num_sms * 4, 256, 0, ctx->stream>>>(
-            F.fp64 ? nullptr : F.sum.p, F.fp64 ? nullptr : F.sumsq.p, F.fp64 ? F.sum64.p : nullptr,
-            F.fp64 ? F.sumsq64.p : nullptr, npx * 3, (double)F.samples, d_mean, d_var);
-    if (d_albedo || d_normal || d_depth)
-        k_aov_out<<<ctx->num_sms * 4, 256, 0, ctx->stream>>>(F.aov.p, npx, (double)F.samples, d_albedo, d_normal,
-                                                            d_depth);
+    k_film_records<<<grid_of(npx, 8, ctx->num_sms), 256, 0, ctx->stream>>>(
+        F.fp64 ? nullptr : F.sum.p, F.fp64 ? nullptr : F.sumsq.p, F.fp64 ? F.sum64.p : nullptr,
+        F.fp64 ? F.sumsq64.p : nullptr, F.aov.p, (float)(1.0 / (double)F.samples), npx,
+        film_scale(F.samples, F.fp64), static_cast<uint4*>(d_rec));
     SALTY_TRY_CUDA(ctx->err, cudaGetLastError());
     return SALTY_OK;
 }

@@ -429,22 +429,51 @@ __global__ void k_loss(const bf16* __restrict__ out, const bf16* __restrict__ x,
     if ((threadIdx.x & 31) == 0) atomicAdd(loss_sum, s);
 }
 
-// One pass of the self-ensemble: adds weight * (the prediction of pixel (px, py), found at
-// its mirrored place in the padded Wp x Hp output, or, with flip bit 2, at the transposed
-// place of the Hp-wide transposed output) to rgb [H][W][3].
-__global__ void k_output_flipped(const bf16* __restrict__ out, const bf16* __restrict__ x, int W, int H, int Wp,
-                                 int Hp, int flip, float weight, int first, float* __restrict__ rgb) {
-    const long long total = (long long)W * H;
-    for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < total; p += (long long)gridDim.x * blockDim.x) {
-        const int px = (int)(p % W), py = (int)(p / W);
-        const int qx = (flip & 1) ? W - 1 - px : px, qy = (flip & 2) ? H - 1 - py : py;
-        const long long q = (flip & 4) ? (long long)qx * Hp + qy : (long long)qy * Wp + qx;
+// Up to four symmetries of one shape, as the self-ensemble's forward passes take them.
+struct FlipSet {
+    int n, flip[4];
+};
+
+// Adds the predictions of a batch of images to rgb [H][W][3]: image j's prediction of pixel
+// (px, py) stands at its mirrored place in the padded Wp x Hp output, or, with flip bit 2, at
+// the transposed place of the Hp-wide transposed output; it is added times `weight`, in the
+// order of the images.  rec: the film's input records, whose first channels are the log
+// colour the network corrects.  Blocks of 16 x 16 pixels: transposed images are read down
+// columns of 16 neighbours.
+__global__ void __launch_bounds__(256) k_output_images(const bf16* __restrict__ out, const uint4* __restrict__ rec, int W,
+                                                       int H, int Wp, int Hp, FlipSet fs, float weight, int first,
+                                                       float* __restrict__ rgb) {
+    const int px = blockIdx.x * 16 + (threadIdx.x & 15), py = blockIdx.y * 16 + (threadIdx.x >> 4);
+    if (px >= W || py >= H) return;
+    const long long p = (long long)py * W + px;
+    const uint2 xr = *reinterpret_cast<const uint2*>(rec + 2 * p);
+    const __nv_bfloat162 x01 = *reinterpret_cast<const __nv_bfloat162*>(&xr.x),
+                         x2 = *reinterpret_cast<const __nv_bfloat162*>(&xr.y);
+    const float x[3] = {__low2float(x01), __high2float(x01), __low2float(x2)};
+    float v[3] = {0.0f, 0.0f, 0.0f};
+    if (!first)
+        for (int c = 0; c < 3; ++c) v[c] = rgb[3 * p + c];
+    uint2 o[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        if (j >= fs.n) break;
+        const int f = fs.flip[j], qx = (f & 1) ? W - 1 - px : px, qy = (f & 2) ? H - 1 - py : py;
+        const long long q = (long long)j * Wp * Hp + ((f & 4) ? (long long)qx * Hp + qy : (long long)qy * Wp + qx);
+        o[j] = __ldg(reinterpret_cast<const uint2*>(out + q * 8));
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        if (j >= fs.n) break;
+        const __nv_bfloat162 r01 = *reinterpret_cast<const __nv_bfloat162*>(&o[j].x),
+                             r2 = *reinterpret_cast<const __nv_bfloat162*>(&o[j].y);
+        const float r[3] = {__low2float(r01), __high2float(r01), __low2float(r2)};
+#pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const float v =
-                weight * fmaxf(expm1f(__bfloat162float(out[q * 8 + c]) + __bfloat162float(x[q * 16 + c])), 0.0f);
-            rgb[p * 3 + c] = first ? v : rgb[p * 3 + c] + v;
+            const float y = __fmul_rn(weight, fmaxf(expm1f(r[c] + x[c]), 0.0f));
+            v[c] = first && j == 0 ? y : __fadd_rn(v[c], y);
         }
     }
+    for (int c = 0; c < 3; ++c) rgb[3 * p + c] = v[c];
 }
 
 // prediction (input log colour + network correction) -> linear colour
@@ -604,33 +633,23 @@ __global__ void k_weights_to_bf16(const float* __restrict__ w, int Cout, int Cin
     }
 }
 
-// Film planes (W x H) -> network input (Wp x Hp, multiples of 16) with reflected borders:
-// colour, albedo, normal, 1/(1+t), noise level mean_c sqrt(var_c) / (1 + colour_c).  With
-// flip bit 0 (1) the frame is mirrored left-right (top-bottom) first; with bit 2 the input
-// is the transposed frame, Hp wide and Wp tall.
-__global__ void k_pack_features(const float* __restrict__ mean, const float* __restrict__ var,
-                                const float* __restrict__ albedo, const float* __restrict__ normal,
-                                const float* __restrict__ depth, int W, int H, int Wp, int Hp, int flip,
-                                float* __restrict__ f) {
-    const long long total = (long long)Wp * Hp;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-        const int x = (flip & 4) ? (int)(i / Hp) : (int)(i % Wp), y = (flip & 4) ? (int)(i % Hp) : (int)(i / Wp);
-        int sx = x < W ? x : max(2 * W - 2 - x, 0), sy = y < H ? y : max(2 * H - 2 - y, 0);
-        if (flip & 1) sx = W - 1 - sx;
-        if (flip & 2) sy = H - 1 - sy;
-        const long long p = (long long)sy * W + sx;
-        float* d = f + i * kFeatures;
-        float noise = 0.0f;
-        for (int c = 0; c < 3; ++c) {
-            const float m = mean[3 * p + c];
-            d[c] = m;
-            d[3 + c] = albedo[3 * p + c];
-            d[6 + c] = normal[3 * p + c];
-            noise += sqrtf(fmaxf(var[3 * p + c], 0.0f)) / (1.0f + fmaxf(m, 0.0f));
-        }
-        d[9] = depth[p];
-        d[10] = noise * (1.0f / 3.0f);
-    }
+// The film's input records (W x H, 32 bytes per pixel) placed as a batch of network inputs
+// (Wp x Hp, multiples of 16) with reflected borders.  With flip bit 0 (1) the frame is
+// mirrored left-right (top-bottom) first; with bit 2 the input is the transposed frame, Hp wide
+// and Wp tall.  Two threads per pixel, 16 x 8 pixels per block; the records (66 MB at 1080p)
+// are read from L2.
+__global__ void __launch_bounds__(256) k_place_inputs(const uint4* __restrict__ rec, int W, int H, int Wp, int Hp,
+                                                      FlipSet fs, uint4* __restrict__ x) {
+    const int half = threadIdx.x & 1, t = threadIdx.x >> 1, f = fs.flip[blockIdx.z];
+    // blocks run along the output's rows: (u, v) is the output pixel
+    const int Wo = (f & 4) ? Hp : Wp, Ho = (f & 4) ? Wp : Hp;
+    const int u = blockIdx.x * 16 + (t & 15), v = blockIdx.y * 8 + (t >> 4);
+    if (u >= Wo || v >= Ho) return;
+    const int px = (f & 4) ? v : u, py = (f & 4) ? u : v;
+    int sx = px < W ? px : max(2 * W - 2 - px, 0), sy = py < H ? py : max(2 * H - 2 - py, 0);
+    if (f & 1) sx = W - 1 - sx;
+    if (f & 2) sy = H - 1 - sy;
+    x[(((long long)blockIdx.z * Ho + v) * Wo + u) * 2 + half] = __ldg(rec + ((long long)sy * W + sx) * 2 + half);
 }
 
 inline int gsz(long long n, int block = 256) {
@@ -698,7 +717,7 @@ struct Unet {
     DevBuf<float> gbuf;
     long long act_off[T_COUNT], g_off[G_COUNT];
     DevBuf<float> io;       // device copies of host features / targets / outputs
-    DevBuf<float> film_ws;  // film planes, packed features and padded output of salty_denoise_unet
+    DevBuf<float> film_ws;  // a film's input records and the denoised image (salty_denoise_unet)
     DevBuf<double> loss;
     DevBuf<float> wg_ws;    // per-CTA partial weight and bias gradients (fixed-order sums)
     DevBuf<bf16> cat_ws;    // a decoder convolution's concatenated input, for its weight gradient
@@ -832,12 +851,13 @@ struct Fwd {
     bf16* t[T_COUNT];
 };
 
+// d_feat: the input features, or null when the input tensor T_X is in place already.
 salty_status forward(salty_ctx* ctx, Unet& u, const float* d_feat, int N, int H, int W, Fwd& F) {
     SALTY_TRY(ensure_workspace(ctx, u, N, H, W));
     for (int i = 0; i < T_COUNT; ++i) F.t[i] = u.act.p + u.act_off[i];
     cudaStream_t st = ctx->stream;
     const long long P0 = (long long)N * H * W;
-    k_prep_input<<<gsz(P0), 256, 0, st>>>(d_feat, P0, F.t[T_X]);
+    if (d_feat) k_prep_input<<<gsz(P0), 256, 0, st>>>(d_feat, P0, F.t[T_X]);
     // pool: the tensor that takes the 2x2 max-pooled output too, or -1
     auto conv = [&](int li, const ConvSrc& in, int out, int h, int w, int pool = -1) {
         const UnetLayer& L = u.layers[li];
@@ -1164,7 +1184,7 @@ salty_status salty_denoise_unet_ensemble(salty_ctx* ctx, salty_unet* net, salty_
     if ((long long)W * H == 0 || Fm.samples == 0) return ctx->err.fail(SALTY_ERR_NOT_BUILT, "the film is empty");
     const int Wp = (W + 15) / 16 * 16, Hp = (H + 15) / 16 * 16;
     SALTY_TRY(check_shape(ctx, 1, Hp, Wp));
-    const long long npx = (long long)W * H, npp = (long long)Wp * Hp;
+    const long long npx = (long long)W * H;
     // The symmetries run as batches of images of one shape: the mirror images (up to 4) in
     // one forward pass, their transposes in a second -- each convolution launch then has
     // that many times more strips to spread over the SMs.  An image's outputs do not depend
@@ -1172,30 +1192,24 @@ salty_status salty_denoise_unet_ensemble(salty_ctx* ctx, salty_unet* net, salty_
     // result in the order k = 0..mirrors-1, as one pass per image would add them.
     const int per = mirrors < 4 ? mirrors : 4;
     SALTY_TRY(check_shape(ctx, per, Hp, Wp));
-    // [mean 3 | var 3 | albedo 3 | normal 3 | depth 1] per film pixel, then features, then the image
-    SALTY_TRY_CUDA(ctx->err, u.film_ws.ensure((size_t)(npx * 16 + per * npp * kFeatures)));
-    float* mean = u.film_ws.p;
-    float* var = mean + npx * 3;
-    float* alb = var + npx * 3;
-    float* nrm = alb + npx * 3;
-    float* dep = nrm + npx * 3;
-    float* feat = dep + npx;
-    float* img = feat + per * npp * kFeatures;
-    SALTY_TRY(film_features(ctx, scene, mean, var, alb, nrm, dep));
+    // the film's input records (8 floats' worth of BF16 per pixel), then the image
+    SALTY_TRY_CUDA(ctx->err, u.film_ws.ensure((size_t)npx * 11));
+    uint4* rec = reinterpret_cast<uint4*>(u.film_ws.p);
+    float* img = u.film_ws.p + npx * 8;
+    SALTY_TRY(film_records(ctx, scene, rec));
     SALTY_TRY(conv_status_reset(ctx));
     for (int k0 = 0; k0 < mirrors; k0 += per) {
-        for (int j = 0; j < per; ++j)
-            k_pack_features<<<gsz(npp), 256, 0, ctx->stream>>>(mean, var, alb, nrm, dep, W, H, Wp, Hp, k0 + j,
-                                                               feat + j * npp * kFeatures);
+        FlipSet fs{per, {0, 0, 0, 0}};
+        for (int j = 0; j < per; ++j) fs.flip[j] = k0 + j;
+        const bool tr = (k0 & 4) != 0;  // the transposed frames: Hp wide, Wp tall
+        const int h = tr ? Wp : Hp, w = tr ? Hp : Wp;
+        SALTY_TRY(ensure_workspace(ctx, u, per, h, w));
+        k_place_inputs<<<dim3(w / 16, (h + 7) / 8, per), 256, 0, ctx->stream>>>(
+            rec, W, H, Wp, Hp, fs, reinterpret_cast<uint4*>(u.act.p + u.act_off[T_X]));
         Fwd F;
-        if (k0 & 4)
-            SALTY_TRY(forward(ctx, u, feat, per, Wp, Hp, F));  // the transposed frames: Hp wide, Wp tall
-        else
-            SALTY_TRY(forward(ctx, u, feat, per, Hp, Wp, F));
-        for (int j = 0; j < per; ++j)
-            k_output_flipped<<<gsz(npx), 256, 0, ctx->stream>>>(F.t[T_OUT] + j * npp * 8, F.t[T_X] + j * npp * 16, W,
-                                                               H, Wp, Hp, k0 + j, 1.0f / (float)mirrors,
-                                                               k0 + j == 0, img);
+        SALTY_TRY(forward(ctx, u, nullptr, per, h, w, F));
+        k_output_images<<<dim3((W + 15) / 16, (H + 15) / 16), 256, 0, ctx->stream>>>(
+            F.t[T_OUT], rec, W, H, Wp, Hp, fs, 1.0f / (float)mirrors, k0 == 0, img);
     }
     SALTY_TRY_CUDA(ctx->err, cudaGetLastError());
     SALTY_TRY_CUDA(ctx->err, cudaMemcpyAsync(out_rgb, img, (size_t)npx * 3 * sizeof(float), cudaMemcpyDefault,

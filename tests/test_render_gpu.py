@@ -275,3 +275,32 @@ def test_cancel_stops_a_render_and_the_context_recovers(ctx):
     assert err.get("status") == salty_gb300.ERR_CANCELLED, err
     r = s.render(32, 32, 4, 8, seed=2, want=("mean",))
     assert np.all(np.isfinite(r["mean"])) and r["samples"] == 4
+
+
+# The film's read-out: mean correctly rounded, variance of the mean within one unit in the last
+# place (pairs of FP32 numbers hold 48 bits; with var >= 2^-14 mean^2 at least 33 bits are left
+# after the cancellation, then one rounding).  Sizes: counts around the largest the pairs
+# take (2^24); values whose squares over- or underflow FP32, which take the 64-bit form.
+@pytest.mark.parametrize("samples", [1, 2, 3, 49, 1000, (1 << 24) - 1, 1 << 24])
+@pytest.mark.parametrize("scale", [1e-22, 1e-3, 1.0, 1e18])
+def test_film_read_out_rounding(ctx, samples, scale):
+    from salty_gb300 import scenes
+    rng = np.random.default_rng(samples)
+    w, h = 37, 5
+    m = (rng.lognormal(0.0, 1.0, (h, w, 3)) * scale).astype(np.float64)
+    s = (m * samples).astype(np.float32).astype(np.float64)
+    with np.errstate(over="ignore"):
+        q = ((s / samples) ** 2 * samples * (1.0 + rng.uniform(2.0 ** -13, 2.0, m.shape))).astype(np.float32)
+    q = q.astype(np.float64)
+    s[0, :3], q[0, :3] = 0.0, 0.0
+    sc = scenes.upload(ctx, scenes.cornell())
+    sc.build()
+    sc.restore({"sum": s, "sumsq": q, "comp": None, "aov": None, "samples": samples}, w, h)
+    r = sc.read(w, h)
+    np.testing.assert_array_equal(r["mean"], (s / samples).astype(np.float32))
+    n = float(samples)
+    v = np.maximum((q / n - (s / n) ** 2) / (n - 1.0), 0.0) if samples > 1 else np.zeros_like(q)
+    with np.errstate(over="ignore"):
+        v = v.astype(np.float32)
+    np.testing.assert_allclose(r["var"], v, rtol=2.0 ** -23, atol=2.0 ** -149)
+    sc.close()
