@@ -360,73 +360,182 @@ __global__ void k_pool(const bf16* __restrict__ in, bf16* __restrict__ out, int 
     }
 }
 
-// max-pool backward: the gradient goes to the first input equal to the max (ties: first).
-// One thread per output pixel and 8 channels (C % 8 == 0); din += at the chosen inputs.
-__global__ void k_pool_bwd(const bf16* __restrict__ in, const float* __restrict__ dout, float* __restrict__ din, int N,
-                           int H, int W, int C) {
-    const int Ho = H / 2, Wo = W / 2, G = C / 8;
-    const long long total = (long long)N * Ho * Wo * G;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-        const int c = (int)(i % G) * 8;
-        long long p = i / G;
-        const long long po = p;
-        const int xo = (int)(p % Wo);
-        p /= Wo;
-        const int yo = (int)(p % Ho);
-        const int n = (int)(p / Ho);
-        const size_t base = (((size_t)n * H + 2 * yo) * W + 2 * xo) * C + c;
-        const size_t off[4] = {0, (size_t)C, (size_t)W * C, (size_t)W * C + C};
-        float m[8], v[4][8];
-        int arg[8];
+// Block sums of the bias gradient: per-thread sums s[8] (8-channel group j of G, thread row r of
+// `per`) added in shared memory in row order into part[blockIdx.x][c], c < C; k_bias_reduce adds
+// the blocks' partials.
+__device__ __forceinline__ void bias_partials(float* sb, const float (&s)[8], int j, int r, int per, int C,
+                                              float* __restrict__ part) {
+    if (r < per && j * 8 < C) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) unpack_bf16x8(__ldg(reinterpret_cast<const uint4*>(in + base + off[k])), v[k]);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            m[e] = -INFINITY;
-            arg[e] = 0;
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (v[k][e] > m[e]) { m[e] = v[k][e]; arg[e] = k; }
-        }
-        const float4* dp = reinterpret_cast<const float4*>(dout + po * C + c);
-        const float4 d0 = __ldg(dp), d1 = __ldg(dp + 1);
-        const float d[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            float4* q = reinterpret_cast<float4*>(din + base + off[k]);
-            float4 a = q[0], b = q[1];
-            a.x += arg[0] == k ? d[0] : 0.0f; a.y += arg[1] == k ? d[1] : 0.0f;
-            a.z += arg[2] == k ? d[2] : 0.0f; a.w += arg[3] == k ? d[3] : 0.0f;
-            b.x += arg[4] == k ? d[4] : 0.0f; b.y += arg[5] == k ? d[5] : 0.0f;
-            b.z += arg[6] == k ? d[6] : 0.0f; b.w += arg[7] == k ? d[7] : 0.0f;
-            q[0] = a;
-            q[1] = b;
-        }
+        for (int k = 0; k < 8; ++k) sb[r * C + j * 8 + k] = s[k];
+    }
+    __syncthreads();
+    for (int c = threadIdx.x; c < C; c += blockDim.x) {
+        float t = 0.0f;
+        for (int i = 0; i < per; ++i) t += sb[i * C + c];
+        part[(size_t)blockIdx.x * C + c] = t;
     }
 }
 
 // L1 loss in log space on channels 0..2 of the prediction y = out + x (the network predicts
-// a correction of the input's log colour x, channels 0..2 of the 16-channel input [npx][16]);
-// grad dout [npx][8] (FP32, zero beyond channel 2)
-__global__ void k_loss(const bf16* __restrict__ out, const bf16* __restrict__ x, const float* __restrict__ target,
-                       long long npx, float* __restrict__ dout, double* __restrict__ loss_sum) {
+// a correction of the input's log colour x, channels 0..2 of the 16-channel input [npx][16]),
+// and its gradient as the next GEMMs' operand: g [npx][16] BF16, zero beyond channel 2, with
+// the output layer's bias partial sums (8 channels).
+__global__ void __launch_bounds__(256) k_loss_bwd(const bf16* __restrict__ out, const bf16* __restrict__ x,
+                                                  const float* __restrict__ target, long long npx, bf16* __restrict__ g,
+                                                  float* __restrict__ part, double* __restrict__ loss_sum) {
+    extern __shared__ float sb[];  // [256][8]
     double s = 0.0;
+    float bs[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     const float scale = 1.0f / (3.0f * (float)npx);
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < npx; p += (long long)gridDim.x * blockDim.x) {
-        for (int c = 0; c < 8; ++c) {
-            float g = 0.0f;
-            if (c < 3) {
-                const float y = __bfloat162float(out[p * 8 + c]) + __bfloat162float(x[p * 16 + c]);
-                const float t = log1pf(fmaxf(target[p * 3 + c], 0.0f));
-                const float d = y - t;
-                s += fabsf(d);
-                g = (d > 0.0f ? 1.0f : (d < 0.0f ? -1.0f : 0.0f)) * scale;
-            }
-            dout[p * 8 + c] = g;
+        const uint2 o = __ldg(reinterpret_cast<const uint2*>(out + p * 8)), xi = __ldg(reinterpret_cast<const uint2*>(x + p * 16));
+        const float2 o01 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&o.x)),
+                     o2 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&o.y)),
+                     x01 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&xi.x)),
+                     x2 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&xi.y));
+        const float y[3] = {o01.x + x01.x, o01.y + x01.y, o2.x + x2.x};
+        float v[8] = {0, 0, 0, 0, 0, 0, 0, 0}, w[8];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const float d = y[c] - log1pf(fmaxf(target[p * 3 + c], 0.0f));
+            s += fabsf(d);
+            v[c] = (d > 0.0f ? 1.0f : (d < 0.0f ? -1.0f : 0.0f)) * scale;
         }
+        const uint4 pk = pack_bf16x8(v);
+        reinterpret_cast<uint4*>(g + p * 16)[0] = pk;
+        reinterpret_cast<uint4*>(g + p * 16)[1] = make_uint4(0, 0, 0, 0);
+        unpack_bf16x8(pk, w);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) bs[c] += w[c];
     }
     for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
     if ((threadIdx.x & 31) == 0) atomicAdd(loss_sum, s);
+    bias_partials(sb, bs, 0, threadIdx.x, blockDim.x, 8, part);
+}
+
+// Where a layer's output gradient comes from: backward-data outputs in BF16, read in place.
+//   GRAD_PLAIN  a [npx][a_cs], channels 0..C-1
+//   GRAD_UP     the layer was up-sampled: the sum of its four children's gradients, channels
+//               0..C-1 of a [N][2h][2w][a_cs]
+//   GRAD_SKIP   the layer fed a skip connection and a max pool: channels a_off.. of
+//               a [npx][a_cs], plus at a 2x2 block's first maximum (of the layer's output) the
+//               block's gradient b [N][h/2][w/2][C]
+enum GradKind { GRAD_PLAIN, GRAD_UP, GRAD_SKIP };
+struct GradSrc {
+    const bf16* a;
+    int a_cs, a_off;
+    const bf16* b;
+};
+
+// A layer's output gradient summed in FP32, its ReLU mask (y > 0), the rounding to BF16 that
+// the next GEMMs read (g [npx][C]) and the bias gradient's partial sums, in one pass: the
+// FP32 copies of the gradients that three kernels wrote and read before are never stored
+// (gradients of 16 x 256 x 256: element-wise kernels 0.55 -> 0.2 ms).  Thread t of a block takes
+// 8-channel group t % G of the pixels (2x2 blocks for GRAD_SKIP) t / G, t / G + per, ... of
+// the block's grid stride.  C and the strides are multiples of 8.
+template <int KIND>
+__global__ void __launch_bounds__(256) k_grad_in(const bf16* __restrict__ y, GradSrc src, int C, int N, int H, int W,
+                                                 bf16* __restrict__ g, float* __restrict__ part) {
+    extern __shared__ float sb[];  // [per][C]
+    const int G = C / 8, per = blockDim.x / G;
+    const int j = threadIdx.x % G, r = threadIdx.x / G, c = j * 8;
+    float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    auto finish = [&](long long p, const float (&yv)[8], float (&v)[8]) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (!(yv[k] > 0.0f)) v[k] = 0.0f;
+        const uint4 pk = pack_bf16x8(v);
+        *reinterpret_cast<uint4*>(g + p * C + c) = pk;
+        float w[8];
+        unpack_bf16x8(pk, w);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) s[k] += w[k];
+    };
+    auto ld = [](const bf16* p) { return __ldg(reinterpret_cast<const uint4*>(p)); };
+    if (r < per) {
+        if (KIND == GRAD_SKIP) {
+            const int Ho = H / 2, Wo = W / 2;
+            const long long nb = (long long)N * Ho * Wo;
+            for (long long b = (long long)blockIdx.x * per + r; b < nb; b += (long long)gridDim.x * per) {
+                const int xo = (int)(b % Wo);
+                const long long t = b / Wo;
+                const int yo = (int)(t % Ho), n = (int)(t / Ho);
+                const long long p0 = ((long long)n * H + 2 * yo) * W + 2 * xo;
+                const long long px[4] = {p0, p0 + 1, p0 + W, p0 + W + 1};
+                uint4 yq[4], aq[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) yq[k] = ld(y + px[k] * C + c);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) aq[k] = ld(src.a + px[k] * src.a_cs + src.a_off + c);
+                float d[8], m[8], yv[8];
+                int arg[8];
+                unpack_bf16x8(ld(src.b + b * C + c), d);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) { m[e] = -INFINITY; arg[e] = 0; }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    unpack_bf16x8(yq[k], yv);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e)
+                        if (yv[e] > m[e]) { m[e] = yv[e]; arg[e] = k; }
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    float v[8];
+                    unpack_bf16x8(yq[k], yv);
+                    unpack_bf16x8(aq[k], v);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) v[e] += arg[e] == k ? d[e] : 0.0f;
+                    finish(px[k], yv, v);
+                }
+            }
+        } else {
+            const long long npx = (long long)N * H * W, step = (long long)gridDim.x * per;
+            for (long long p = (long long)blockIdx.x * per + r; p < npx; p += step) {
+                float v[8], yv[8];
+                const uint4 yq = ld(y + p * C + c);
+                if (KIND == GRAD_UP) {
+                    const int x = (int)(p % W);
+                    const long long t = p / W;
+                    const int yy = (int)(t % H), n = (int)(t / H);
+                    const bf16* a = src.a + (((long long)n * 2 * H + 2 * yy) * 2 * W + 2 * x) * src.a_cs + c;
+                    const uint4 q[4] = {ld(a), ld(a + src.a_cs), ld(a + (size_t)2 * W * src.a_cs),
+                                        ld(a + (size_t)2 * W * src.a_cs + src.a_cs)};
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) v[k] = 0.0f;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        float w[8];
+                        unpack_bf16x8(q[i], w);
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) v[k] += w[k];
+                    }
+                } else {
+                    unpack_bf16x8(ld(src.a + p * src.a_cs + c), v);
+                }
+                unpack_bf16x8(yq, yv);
+                finish(p, yv, v);
+            }
+        }
+    }
+    bias_partials(sb, s, j, r, per, C, part);
+}
+
+// db[c] += the blocks' partials: 32 threads per channel, each a strided share, then their sums
+// in a fixed order (one thread per channel took 36 us per layer for 608 blocks).
+__global__ void __launch_bounds__(256) k_bias_reduce(const float* __restrict__ part, int blocks, int C,
+                                                     float* __restrict__ db) {
+    __shared__ float sm[32][9];
+    const int cl = threadIdx.x & 7, r = threadIdx.x >> 3, c = blockIdx.x * 8 + cl;
+    float t = 0.0f;
+    for (int b = r; b < blocks; b += 32) t += part[(size_t)b * C + c];
+    sm[r][cl] = t;
+    __syncthreads();
+    if (r != 0) return;
+    t = 0.0f;
+    for (int i = 0; i < 32; ++i) t += sm[i][cl];
+    db[c] += t;
 }
 
 // Up to four symmetries of one shape, as the self-ensemble's forward passes take them.
@@ -483,126 +592,6 @@ __global__ void k_output(const bf16* __restrict__ out, const bf16* __restrict__ 
         for (int c = 0; c < 3; ++c)
             rgb[p * 3 + c] =
                 fmaxf(expm1f(__bfloat162float(out[p * 8 + c]) + __bfloat162float(x[p * 16 + c])), 0.0f);
-}
-
-// ReLU backward and the bias gradient in one pass over a layer's output gradient dy:
-// g = dy * (y > 0) in BF16 (the next GEMMs' operand, channels C..g_cs-1 zero), and per block
-// the sums of g's BF16 values per channel in a fixed order (no atomics).  Thread t of a
-// block takes 8-channel group j = t % G (G = g_cs / 8) of the pixels r = t / G, r + per,
-// ... of the block's grid stride (per = blockDim / G; threads beyond per * G idle) and sums
-// in registers; the per-thread sums are added in shared memory in thread order into
-// part[blockIdx.x][c], and k_bias_reduce adds the blocks' partials in block order.
-// dy is FP32 [npx][C], or, when dy16 is given, BF16 with dy16_cs channels per pixel (a
-// backward-data GEMM's output read directly; widening it to FP32 first would be exact).
-// (C, y_cs, g_cs, dy16_cs multiples of 8.)
-__global__ void k_relu_bwd_bias(const bf16* __restrict__ y, int y_cs, const float* __restrict__ dy,
-                                const bf16* __restrict__ dy16, int dy16_cs, int C, int relu, long long npx,
-                                bf16* __restrict__ g, int g_cs, float* __restrict__ part) {
-    extern __shared__ float sb[];  // [per][C]
-    const int G = g_cs / 8, per = blockDim.x / G, lanes = per * G;
-    if ((int)threadIdx.x < lanes) {
-        const int j = threadIdx.x % G, r = threadIdx.x / G, c = j * 8;
-        float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        for (long long p = (long long)blockIdx.x * per + r; p < npx; p += (long long)gridDim.x * per) {
-            float v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-            if (c < C) {
-                if (dy16) {
-                    unpack_bf16x8(__ldg(reinterpret_cast<const uint4*>(dy16 + p * dy16_cs + c)), v);
-                } else {
-                    const float4* d = reinterpret_cast<const float4*>(dy + p * C + c);
-                    const float4 a = __ldg(d), b = __ldg(d + 1);
-                    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-                }
-                if (relu) {
-                    float yv[8];
-                    unpack_bf16x8(__ldg(reinterpret_cast<const uint4*>(y + p * y_cs + c)), yv);
-#pragma unroll
-                    for (int k = 0; k < 8; ++k)
-                        if (!(yv[k] > 0.0f)) v[k] = 0.0f;
-                }
-            }
-            const uint4 pk = pack_bf16x8(v);
-            *reinterpret_cast<uint4*>(g + p * g_cs + c) = pk;
-            if (c < C) {
-                float w[8];
-                unpack_bf16x8(pk, w);
-#pragma unroll
-                for (int k = 0; k < 8; ++k) s[k] += w[k];
-            }
-        }
-        if (c < C) {
-#pragma unroll
-            for (int k = 0; k < 8; ++k) sb[r * C + c + k] = s[k];
-        }
-    }
-    __syncthreads();
-    for (int c = threadIdx.x; c < C; c += blockDim.x) {
-        float t = 0.0f;
-        for (int r = 0; r < per; ++r) t += sb[r * C + c];
-        part[(size_t)blockIdx.x * C + c] = t;
-    }
-}
-
-__global__ void k_bias_reduce(const float* __restrict__ part, int blocks, int C, float* __restrict__ db) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= C) return;
-    float t = 0.0f;
-    for (int b = 0; b < blocks; ++b) t += part[(size_t)b * C + c];
-    db[c] += t;
-}
-
-// BF16 activation gradient (from a backward-data GEMM) -> FP32, optionally accumulated;
-// channels [off, off + C) of src [npx][Cs]
-// (one thread per pixel and 8 channels; Cs, off, C multiples of 8)
-__global__ void k_grad_to_f32(const bf16* __restrict__ src, int Cs, int off, int C, long long npx, float* __restrict__ dst,
-                              int accumulate) {
-    const int G = C / 8;
-    const long long total = npx * G;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-        const long long p = i / G;
-        const int c = (int)(i % G) * 8;
-        float v[8];
-        unpack_bf16x8(__ldg(reinterpret_cast<const uint4*>(src + p * Cs + off + c)), v);
-        float4* d = reinterpret_cast<float4*>(dst + p * C + c);
-        float4 a = make_float4(v[0], v[1], v[2], v[3]), b = make_float4(v[4], v[5], v[6], v[7]);
-        if (accumulate) {
-            const float4 a0 = d[0], b0 = d[1];
-            a.x += a0.x; a.y += a0.y; a.z += a0.z; a.w += a0.w;
-            b.x += b0.x; b.y += b0.y; b.z += b0.z; b.w += b0.w;
-        }
-        d[0] = a;
-        d[1] = b;
-    }
-}
-
-// up-sampling backward: coarse grad = sum of its 2x2 children's grads (channels [0, Cc) of dcat)
-// (one thread per coarse pixel and 8 channels; Ccat, Cc multiples of 8)
-__global__ void k_upsample_bwd(const bf16* __restrict__ dcat, int Ccat, float* __restrict__ dcoarse, int Cc, int N,
-                               int H, int W) {
-    const int Hc = H / 2, Wc = W / 2, G = Cc / 8;
-    const long long total = (long long)N * Hc * Wc * G;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-        const int c = (int)(i % G) * 8;
-        long long p = i / G;
-        const long long pc = p;
-        const int x = (int)(p % Wc);
-        p /= Wc;
-        const int y = (int)(p % Hc);
-        const int n = (int)(p / Hc);
-        float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        for (int dy = 0; dy < 2; ++dy)
-            for (int dx = 0; dx < 2; ++dx) {
-                float v[8];
-                unpack_bf16x8(__ldg(reinterpret_cast<const uint4*>(
-                                  dcat + (((size_t)n * H + 2 * y + dy) * W + 2 * x + dx) * Ccat + c)),
-                              v);
-#pragma unroll
-                for (int k = 0; k < 8; ++k) s[k] += v[k];
-            }
-        float4* d = reinterpret_cast<float4*>(dcoarse + pc * Cc + c);
-        d[0] = make_float4(s[0], s[1], s[2], s[3]);
-        d[1] = make_float4(s[4], s[5], s[6], s[7]);
-    }
 }
 
 // Adam on FP32 masters, then the BF16 copies: forward layout [tap][co][ci] and the
@@ -693,17 +682,13 @@ int pick_nt(int c) {
 
 inline int round_up(int a, int b) { return (a + b - 1) / b * b; }
 
-// Activation workspace (BF16), by name; sizes in elements for N x H x W inputs.
+// Workspace (BF16), by name; sizes in elements for N x H x W inputs.  T_G: a layer's output
+// gradient, T_G2: its input gradient, T_C0..3: the decoder layers' input gradients (read twice,
+// as the coarse level's and the skip connection's).
 enum {
     T_X, T_A0, T_E0, T_P0, T_A1, T_E1, T_P1, T_A2, T_E2, T_P2, T_A3, T_E3, T_P3, T_B,
-    T_D3, T_D2, T_D1, T_D0, T_OUT, T_G, T_G2, T_COUNT
+    T_D3, T_D2, T_D1, T_D0, T_OUT, T_G, T_G2, T_C3, T_C2, T_C1, T_C0, T_COUNT
 };
-// FP32 gradients, by name.
-enum {
-    G_OUT, G_D0, G_C0S, G_D1, G_D2, G_D3, G_B, G_E0, G_E1, G_E2, G_E3, G_P3, G_A3, G_P2, G_A2, G_P1, G_A1, G_P0,
-    G_A0, G_COUNT
-};
-
 }  // namespace
 
 struct Unet {
@@ -714,8 +699,7 @@ struct Unet {
     long long step = 0;
     int N = 0, H = 0, W = 0;
     DevBuf<bf16> act;
-    DevBuf<float> gbuf;
-    long long act_off[T_COUNT], g_off[G_COUNT];
+    long long act_off[T_COUNT];
     DevBuf<float> io;       // device copies of host features / targets / outputs
     DevBuf<float> film_ws;  // a film's input records and the denoised image (salty_denoise_unet)
     DevBuf<double> loss;
@@ -811,16 +795,10 @@ salty_status ensure_workspace(salty_ctx* ctx, Unet& u, int N, int H, int W) {
     const long long P0 = (long long)N * H * W, P1 = P0 / 4, P2 = P0 / 16, P3 = P0 / 64, P4 = P0 / 256;
     const long long asz[T_COUNT] = {P0 * 16, P0 * 32, P0 * 32, P1 * 32, P1 * 48, P1 * 48, P2 * 48, P2 * 64, P2 * 64,
                                     P3 * 64, P3 * 80, P3 * 80, P4 * 80, P4 * 96, P3 * 80, P2 * 64, P1 * 48, P0 * 32,
-                                    P0 * 8, P0 * 176, P0 * 176};
-    const long long gsz_[G_COUNT] = {P0 * 8, P0 * 32, P0 * 32, P1 * 48, P2 * 64, P3 * 80, P4 * 96, P0 * 32, P1 * 48,
-                                     P2 * 64, P3 * 80, P4 * 80, P3 * 80, P3 * 64, P2 * 64, P2 * 48, P1 * 48, P1 * 32,
-                                     P0 * 32};
+                                    P0 * 8, P0 * 32, P0 * 32, P3 * 176, P2 * 144, P1 * 112, P0 * 80};
     long long o = 0;
     for (int i = 0; i < T_COUNT; ++i) { u.act_off[i] = o; o += (asz[i] + 63) / 64 * 64; }
     SALTY_TRY_CUDA(ctx->err, u.act.ensure((size_t)o));
-    o = 0;
-    for (int i = 0; i < G_COUNT; ++i) { u.g_off[i] = o; o += (gsz_[i] + 63) / 64 * 64; }
-    SALTY_TRY_CUDA(ctx->err, u.gbuf.ensure((size_t)o));
     size_t ws = 0;
     for (int i = 0; i < kNumLayers; ++i) {
         const UnetLayer& L = u.layers[i];
@@ -886,27 +864,34 @@ salty_status forward(salty_ctx* ctx, Unet& u, const float* d_feat, int N, int H,
     return SALTY_OK;
 }
 
-// One conv layer backward.  dy: FP32 [npx][cout] gradient of the layer output y.  Adds the
-// weight and bias gradients; leaves dL/d(input) in BF16 in F.t[T_G2] ([npx][cin]) when
-// want_dx.
-salty_status conv_backward(salty_ctx* ctx, Unet& u, Fwd& F, int li, const ConvSrc& x, int y, const float* dy, int N,
-                           int h, int w, bool want_dx, const bf16* dy16 = nullptr, int dy16_cs = 0) {
+// Blocks of a gradient pass over `work` units of 8 channels x C / 8 groups (4 per SM: the bias
+// partials of 4 blocks per SM are what the workspace holds).
+int grad_blocks(salty_ctx* ctx, long long work, int per) {
+    return (int)std::min<long long>((long long)ctx->num_sms * 4, (work + per - 1) / per);
+}
+
+// The output gradient of layer li in T_G (BF16), with its bias gradient added.
+template <int KIND>
+salty_status grad_in(salty_ctx* ctx, Unet& u, Fwd& F, int li, int y, const GradSrc& src, int N, int h, int w) {
     const UnetLayer& L = u.layers[li];
-    const long long npx = (long long)N * h * w;
-    cudaStream_t st = ctx->stream;
-    bf16* g = F.t[T_G];
-    // ReLU backward and the bias gradient's per-block partial sums in one pass (4 blocks per
-    // SM), then the partials added in block order
-    const int per = 256 / (L.cout_pad / 8);
-    const int bias_blocks = (int)std::min<long long>((long long)ctx->num_sms * 4, (npx + per - 1) / per);
-    k_relu_bwd_bias<<<bias_blocks, 256, (size_t)per * L.cout * sizeof(float), st>>>(
-        F.t[y], L.cout, dy, dy16, dy16_cs, L.cout, L.relu, npx, g, L.cout_pad, u.wg_ws.p);
-    k_bias_reduce<<<(L.cout + 127) / 128, 128, 0, st>>>(u.wg_ws.p, bias_blocks, L.cout, u.grads.p + L.b_off);
-    SALTY_TRY(launch_wgrad(ctx, u, g, L.cout_pad, L.cout, x, L.cin, u.grads.p + L.w_off, N, h, w));
-    if (want_dx)
-        SALTY_TRY(launch_conv(ctx, u.conv_kind, conv_src(g, L.cout_pad, L.cout_pad), L.cout_pad, u.wb.p + L.wb_off,
-                              L.rows_bwd, L.nt_b, nullptr, F.t[T_G2], L.cin, L.cin, N, h, w, 0));
+    const long long npx = (long long)N * h * w, work = KIND == GRAD_SKIP ? npx / 4 : npx;
+    const int per = 256 / (L.cout / 8), blocks = grad_blocks(ctx, work, per);
+    k_grad_in<KIND><<<blocks, 256, (size_t)per * L.cout * sizeof(float), ctx->stream>>>(F.t[y], src, L.cout, N, h, w,
+                                                                                      F.t[T_G], u.wg_ws.p);
+    k_bias_reduce<<<L.cout / 8, 256, 0, ctx->stream>>>(u.wg_ws.p, blocks, L.cout, u.grads.p + L.b_off);
     SALTY_TRY_CUDA(ctx->err, cudaGetLastError());
+    return SALTY_OK;
+}
+
+// Weight gradient of layer li from its output gradient in T_G, and, with dx >= 0, the gradient
+// of its input in that tensor ([npx][cin], BF16).
+salty_status conv_backward(salty_ctx* ctx, Unet& u, Fwd& F, int li, const ConvSrc& x, int N, int h, int w, int dx) {
+    const UnetLayer& L = u.layers[li];
+    bf16* g = F.t[T_G];
+    SALTY_TRY(launch_wgrad(ctx, u, g, L.cout_pad, L.cout, x, L.cin, u.grads.p + L.w_off, N, h, w));
+    if (dx >= 0)
+        SALTY_TRY(launch_conv(ctx, u.conv_kind, conv_src(g, L.cout_pad, L.cout_pad), L.cout_pad, u.wb.p + L.wb_off,
+                              L.rows_bwd, L.nt_b, nullptr, F.t[dx], L.cin, L.cin, N, h, w, 0));
     return SALTY_OK;
 }
 
@@ -914,57 +899,60 @@ salty_status conv_backward(salty_ctx* ctx, Unet& u, Fwd& F, int li, const ConvSr
 salty_status backward(salty_ctx* ctx, Unet& u, Fwd& F, const float* d_target, int N, int H, int W, double* loss) {
     cudaStream_t st = ctx->stream;
     const long long P0 = (long long)N * H * W;
-    float* G[G_COUNT];
-    for (int i = 0; i < G_COUNT; ++i) G[i] = u.gbuf.p + u.g_off[i];
     SALTY_TRY_CUDA(ctx->err, cudaMemsetAsync(u.grads.p, 0, u.n_params * sizeof(float), st));
     SALTY_TRY_CUDA(ctx->err, u.loss.ensure(1));
     SALTY_TRY_CUDA(ctx->err, cudaMemsetAsync(u.loss.p, 0, sizeof(double), st));
-    k_loss<<<gsz(P0), 256, 0, st>>>(F.t[T_OUT], F.t[T_X], d_target, P0, G[G_OUT], u.loss.p);
     const int H1 = H / 2, W1 = W / 2, H2 = H / 4, W2 = W / 4, H3 = H / 8, W3 = W / 8, H4 = H / 16, W4 = W / 16;
-    const long long P1 = P0 / 4, P2 = P0 / 16, P3 = P0 / 64, P4 = P0 / 256;
     auto x = [&](int t, int c) { return conv_src(F.t[t], c, c); };
     auto cat = [&](int coarse, int cc, int skip, int cs) { return conv_src_cat(F.t[coarse], cc, F.t[skip], cs); };
-    auto to_f32 = [&](int cs, int off, int c, long long np, float* dst, int acc) {
-        k_grad_to_f32<<<gsz(np * c / 8), 256, 0, st>>>(F.t[T_G2], cs, off, c, np, dst, acc);
+    auto plain = [&](int li, int y, int h, int w) {
+        return grad_in<GRAD_PLAIN>(ctx, u, F, li, y, GradSrc{F.t[T_G2], u.layers[li].cout, 0, nullptr}, N, h, w);
     };
-    // decoder: a conv's input gradient splits into the up-sampled part and the skip part
-    auto split = [&](int cc, int cs, int h, int w, float* g_coarse, float* g_skip) {
-        const long long np = (long long)N * h * w;
-        k_upsample_bwd<<<gsz(np / 4 * cc / 8), 256, 0, st>>>(F.t[T_G2], cc + cs, g_coarse, cc, N, h, w);
-        to_f32(cc + cs, cc, cs, np, g_skip, 0);
+    auto up = [&](int li, int y, int dcat, int ch, int h, int w) {
+        return grad_in<GRAD_UP>(ctx, u, F, li, y, GradSrc{F.t[dcat], ch, 0, nullptr}, N, h, w);
     };
-    SALTY_TRY(conv_backward(ctx, u, F, 13, x(T_D0, 32), T_OUT, G[G_OUT], N, H, W, true));
-    SALTY_TRY(conv_backward(ctx, u, F, 12, cat(T_D1, 48, T_E0, 32), T_D0, nullptr, N, H, W, true, F.t[T_G2], 32));
-    split(48, 32, H, W, G[G_D1], G[G_E0]);
-    SALTY_TRY(conv_backward(ctx, u, F, 11, cat(T_D2, 64, T_E1, 48), T_D1, G[G_D1], N, H1, W1, true));
-    split(64, 48, H1, W1, G[G_D2], G[G_E1]);
-    SALTY_TRY(conv_backward(ctx, u, F, 10, cat(T_D3, 80, T_E2, 64), T_D2, G[G_D2], N, H2, W2, true));
-    split(80, 64, H2, W2, G[G_D3], G[G_E2]);
-    SALTY_TRY(conv_backward(ctx, u, F, 9, cat(T_B, 96, T_E3, 80), T_D3, G[G_D3], N, H3, W3, true));
-    split(96, 80, H3, W3, G[G_B], G[G_E3]);
-    SALTY_TRY(conv_backward(ctx, u, F, 8, x(T_P3, 80), T_B, G[G_B], N, H4, W4, true));
-    to_f32(80, 0, 80, P4, G[G_P3], 0);
-    k_pool_bwd<<<gsz(P4 * 80 / 8), 256, 0, st>>>(F.t[T_E3], G[G_P3], G[G_E3], N, H3, W3, 80);
-    SALTY_TRY(conv_backward(ctx, u, F, 7, x(T_A3, 80), T_E3, G[G_E3], N, H3, W3, true));
-    SALTY_TRY(conv_backward(ctx, u, F, 6, x(T_P2, 64), T_A3, nullptr, N, H3, W3, true, F.t[T_G2], 80));
-    to_f32(64, 0, 64, P3, G[G_P2], 0);
-    k_pool_bwd<<<gsz(P3 * 64 / 8), 256, 0, st>>>(F.t[T_E2], G[G_P2], G[G_E2], N, H2, W2, 64);
-    SALTY_TRY(conv_backward(ctx, u, F, 5, x(T_A2, 64), T_E2, G[G_E2], N, H2, W2, true));
-    SALTY_TRY(conv_backward(ctx, u, F, 4, x(T_P1, 48), T_A2, nullptr, N, H2, W2, true, F.t[T_G2], 64));
-    to_f32(48, 0, 48, P2, G[G_P1], 0);
-    k_pool_bwd<<<gsz(P2 * 48 / 8), 256, 0, st>>>(F.t[T_E1], G[G_P1], G[G_E1], N, H1, W1, 48);
-    SALTY_TRY(conv_backward(ctx, u, F, 3, x(T_A1, 48), T_E1, G[G_E1], N, H1, W1, true));
-    SALTY_TRY(conv_backward(ctx, u, F, 2, x(T_P0, 32), T_A1, nullptr, N, H1, W1, true, F.t[T_G2], 48));
-    to_f32(32, 0, 32, P1, G[G_P0], 0);
-    k_pool_bwd<<<gsz(P1 * 32 / 8), 256, 0, st>>>(F.t[T_E0], G[G_P0], G[G_E0], N, H, W, 32);
-    SALTY_TRY(conv_backward(ctx, u, F, 1, x(T_A0, 32), T_E0, G[G_E0], N, H, W, true));
-    SALTY_TRY(conv_backward(ctx, u, F, 0, x(T_X, 16), T_A0, nullptr, N, H, W, false, F.t[T_G2], 32));
+    auto skip = [&](int li, int y, int dcat, int ch, int off, int h, int w) {
+        return grad_in<GRAD_SKIP>(ctx, u, F, li, y, GradSrc{F.t[dcat], ch, off, F.t[T_G2]}, N, h, w);
+    };
+    auto back = [&](int li, const ConvSrc& in, int h, int w, int dx) {
+        return conv_backward(ctx, u, F, li, in, N, h, w, dx);
+    };
+    // the loss, its gradient and the output layer's bias gradient
+    const int lb = grad_blocks(ctx, P0, 256);
+    k_loss_bwd<<<lb, 256, 256 * 8 * sizeof(float), st>>>(F.t[T_OUT], F.t[T_X], d_target, P0, F.t[T_G], u.wg_ws.p, u.loss.p);
+    k_bias_reduce<<<1, 256, 0, st>>>(u.wg_ws.p, lb, 8, u.grads.p + u.layers[13].b_off);
+    SALTY_TRY(back(13, x(T_D0, 32), H, W, T_G2));
+    SALTY_TRY(plain(12, T_D0, H, W));
+    SALTY_TRY(back(12, cat(T_D1, 48, T_E0, 32), H, W, T_C0));
+    SALTY_TRY(up(11, T_D1, T_C0, 80, H1, W1));
+    SALTY_TRY(back(11, cat(T_D2, 64, T_E1, 48), H1, W1, T_C1));
+    SALTY_TRY(up(10, T_D2, T_C1, 112, H2, W2));
+    SALTY_TRY(back(10, cat(T_D3, 80, T_E2, 64), H2, W2, T_C2));
+    SALTY_TRY(up(9, T_D3, T_C2, 144, H3, W3));
+    SALTY_TRY(back(9, cat(T_B, 96, T_E3, 80), H3, W3, T_C3));
+    SALTY_TRY(up(8, T_B, T_C3, 176, H4, W4));
+    SALTY_TRY(back(8, x(T_P3, 80), H4, W4, T_G2));
+    SALTY_TRY(skip(7, T_E3, T_C3, 176, 96, H3, W3));
+    SALTY_TRY(back(7, x(T_A3, 80), H3, W3, T_G2));
+    SALTY_TRY(plain(6, T_A3, H3, W3));
+    SALTY_TRY(back(6, x(T_P2, 64), H3, W3, T_G2));
+    SALTY_TRY(skip(5, T_E2, T_C2, 144, 80, H2, W2));
+    SALTY_TRY(back(5, x(T_A2, 64), H2, W2, T_G2));
+    SALTY_TRY(plain(4, T_A2, H2, W2));
+    SALTY_TRY(back(4, x(T_P1, 48), H2, W2, T_G2));
+    SALTY_TRY(skip(3, T_E1, T_C1, 112, 64, H1, W1));
+    SALTY_TRY(back(3, x(T_A1, 48), H1, W1, T_G2));
+    SALTY_TRY(plain(2, T_A1, H1, W1));
+    SALTY_TRY(back(2, x(T_P0, 32), H1, W1, T_G2));
+    SALTY_TRY(skip(1, T_E0, T_C0, 80, 48, H, W));
+    SALTY_TRY(back(1, x(T_A0, 32), H, W, T_G2));
+    SALTY_TRY(plain(0, T_A0, H, W));
+    SALTY_TRY(back(0, x(T_X, 16), H, W, -1));
     SALTY_TRY_CUDA(ctx->err, cudaGetLastError());
     double l = 0.0;
     SALTY_TRY_CUDA(ctx->err, cudaMemcpyAsync(&l, u.loss.p, sizeof(double), cudaMemcpyDeviceToHost, st));
     SALTY_TRY_CUDA(ctx->err, cudaStreamSynchronize(st));
     *loss = l / (3.0 * (double)P0);
-    (void)P1; (void)P2; (void)P3; (void)W4; (void)H4;
     return SALTY_OK;
 }
 
