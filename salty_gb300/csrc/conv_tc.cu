@@ -51,7 +51,7 @@
 //   warps 2-9 the epilogue: TMEM -> bias, ReLU, BF16 -> global, two warps per TMEM lane
 //             quarter, then release the accumulator; optionally also the 2x2 max-pooled
 //             output (rows paired in the strip, columns by a shuffle)
-//   warps 10-13 (decoder layers only) fill the chunks that come from the coarse level: each
+//   warps 10-17 (decoder layers only) fill the chunks that come from the coarse level: each
 //             coarse pixel is loaded once and stored to its up to four places in the
 //             swizzled halo, so the up-sampled tensor is never written
 // Two accumulators of R x Npad columns (512 TMEM columns) let the epilogue of one strip
@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_conv3x3_tc(const TcConvArgs a
 constexpr int kMaxStages = 4;
 constexpr int kTmaMmaWarps = 1;
 constexpr int kTmaEpiWarps = 8;            // two per TMEM lane quarter
-constexpr int kTmaCoarseWarps = 4;         // expand the coarse level (decoder layers)
+constexpr int kTmaCoarseWarps = 8;         // expand the coarse level (decoder layers)
 constexpr int kTmaThreads = 32 * (1 + kTmaMmaWarps + kTmaEpiWarps);
 constexpr int kTmaMaxChunks = 16;          // input channel chunks with their own weight barrier
 constexpr int kTmaHeader = 2048;   // barriers, TMEM address, abort flag, bias
@@ -603,7 +603,7 @@ k_conv3x3_tma(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__
         }
     } else {
         // coarse chunks: halo pixel (hy, hx) shows coarse pixel ((y0 - 1 + hy) >> 1, (x0 - 1 + hx) >> 1)
-        constexpr int kJobs = 7;  // coarse pixel halves per thread: up to 6 rows x 66 pixels x 2 halves / 128 threads
+        constexpr int kJobs = 4;  // coarse pixel halves per thread: up to 6 rows x 66 pixels x 2 halves / 256 threads
         constexpr int kCoarseW = kStrip / 2 + 2;
         const int ct = tid - kTmaThreads;
         const int Hc = a.H >> 1, Wc = a.W >> 1;
@@ -647,7 +647,8 @@ k_conv3x3_tma(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__
                     const int hy0 = 2 * (cy0 + p / kCoarseW) - (y0 - 1), hx0 = 2 * (cx0 + p % kCoarseW) - (x0 - 1);
 #pragma unroll
                     for (int d = 0; d < 4; ++d) {
-                        const int hy = hy0 + (d >> 1), hx = hx0 + (d & 1);
+                        // pairs of pixels swap their left and right copies, so that a warp's 512 bytes cover all banks
+                        const int hy = hy0 + (d >> 1), hx = hx0 + ((d ^ (p >> 1)) & 1);
                         if (hy < 0 || hy >= R + 2 || hx < 0 || hx >= kHaloW) continue;
                         const int px = hy * kHaloW + hx;
                         *reinterpret_cast<uint4*>(dst + px * 32 + ((half ^ ((px >> 2) & 1)) << 4)) = v[u];
@@ -698,7 +699,7 @@ EncodeTiledFn tensor_map_encoder() {
 // its start moved to row r + ky, pixel kx -- the copy engine has zero-filled the image
 // border -- so the input is read once per strip, not once per tap.  CTAs of a group split
 // the strips between them (K-split): each writes its partial sums to its own slice of a
-// workspace, and k_wgrad_reduce adds the slices in order -- the result does not depend on
+// workspace, and k_grad_reduce adds the slices in a fixed order -- the result does not depend on
 // scheduling, unlike atomics.
 //
 // Warp roles: one lane of warp 0 issues the TMA copies of each strip into a ring of
@@ -713,6 +714,8 @@ constexpr int kWgHaloW = kWgStrip + 2;
 constexpr int kWgChunk = 48;
 constexpr int kWgStages = 3;
 constexpr int kWgThreads = 128;
+constexpr int kWgCoarseWarps = 8;  // warps 2 .. 9 of a decoder layer's blocks expand the coarse level
+constexpr int kWgCoarseThreads = 64 + 32 * kWgCoarseWarps;
 constexpr int kWgHeader = 1024;
 constexpr int kWgDyBox = kWgRows * kWgStrip * 32;                                   // 16 channels
 constexpr int kWgXBox = ((kWgRows + 2) * kWgHaloW * 32 + 1023) / 1024 * 1024;  // 16 channels, padded
@@ -737,10 +740,12 @@ struct WgradArgs {
     int cpad, cout, cin, N, H, W;
     int strips;   // N * ceil(H / kWgRows) * ceil(W / kWgStrip)
     float* part;  // [gridDim.x slices][9][cpad][cin]
+    const bf16* coarse;  // decoder layers: input channels [0, coarse_ch) at half resolution
+    int coarse_cs, coarse_ch;
     int* status;
 };
 
-__global__ void __launch_bounds__(kWgThreads, 1)
+__global__ void __launch_bounds__(kWgCoarseThreads, 1)
 k_wgrad_tc(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_dy, const WgradArgs a) {
     extern __shared__ __align__(1024) unsigned char smem[];
     uint64_t* full = reinterpret_cast<uint64_t*>(smem);  // [kWgStages]
@@ -757,13 +762,14 @@ k_wgrad_tc(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUt
     const int c0 = blockIdx.y * kWgChunk;                    // this group's input channels
     const int ch = min(kWgChunk, a.cin - c0);               // 16, 32 or 48
     const int ndy = a.cpad / 16, nx = ch / 16;
+    const int ncx = min(max(a.coarse_ch - c0, 0), ch) / 16;  // boxes expanded from the coarse level, before the others
     const int sx = (a.W + kWgStrip - 1) / kWgStrip, sy = (a.H + kWgRows - 1) / kWgRows;
     const int first = blockIdx.x;
     const int count = first < a.strips ? (a.strips - 1 - first) / (int)gridDim.x + 1 : 0;
 
     if (tid == 0) {
         for (int k = 0; k < kWgStages; ++k) {
-            mbar_init(saddr(full + k), 1);
+            mbar_init(saddr(full + k), ncx ? 1 + kWgCoarseWarps : 1);  // the TMA thread, and the expanding warps
             mbar_init(saddr(empty + k), 1);
         }
         mbar_init(saddr(acc), 1);
@@ -783,7 +789,7 @@ k_wgrad_tc(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUt
     if (warp == 0 && lane == 0) {
         asm volatile("prefetch.tensormap [%0];" :: "l"(reinterpret_cast<uint64_t>(&tm_x)) : "memory");
         asm volatile("prefetch.tensormap [%0];" :: "l"(reinterpret_cast<uint64_t>(&tm_dy)) : "memory");
-        const uint32_t tx = (uint32_t)ndy * kWgDyBox + (uint32_t)nx * ((kWgRows + 2) * kWgHaloW * 32);
+        const uint32_t tx = (uint32_t)ndy * kWgDyBox + (uint32_t)(nx - ncx) * ((kWgRows + 2) * kWgHaloW * 32);
         for (int it = 0; it < count; ++it) {
             const int b = it % kWgStages;
             if (!wait_or_abort(saddr(empty + b), ((uint32_t)(it / kWgStages) & 1u) ^ 1u, abort_flag, a.status)) {
@@ -798,7 +804,8 @@ k_wgrad_tc(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUt
             mbar_expect_tx(bar, tx);
             const uint32_t dyb = saddr(stage0 + b * kWgStage), xb = dyb + 8 * kWgDyBox;
             for (int k = 0; k < ndy; ++k) tma_load_4d(dyb + k * kWgDyBox, &tm_dy, k * 16, x0, y0, n, bar);
-            for (int k = 0; k < nx; ++k) tma_load_4d(xb + k * kWgXBox, &tm_x, c0 + k * 16, x0 - 1, y0 - 1, n, bar);
+            for (int k = ncx; k < nx; ++k)
+                tma_load_4d(xb + k * kWgXBox, &tm_x, c0 + k * 16 - a.coarse_ch, x0 - 1, y0 - 1, n, bar);
         }
     } else if (warp == 1) {  // converged, one elected lane issues (see k_conv3x3_tma)
         const uint32_t el = elect_lane();
@@ -826,11 +833,57 @@ k_wgrad_tc(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUt
             umma_commit_elect(saddr(empty + b), el);
         }
         if (ok && count > 0) umma_commit_elect(saddr(acc), el);
+    } else if (warp >= 2 && ncx) {
+        // the coarse level's boxes: each coarse pixel loaded once and stored to its up to four
+        // places in the swizzled halo (as in k_conv3x3_tma), so no concatenation is written
+        constexpr int kCx = kWgStrip / 2 + 2, kCy = kWgRows / 2 + 2, kBoxJobs = kCx * kCy * 2;
+        constexpr int kT = 32 * kWgCoarseWarps, kJobs = (kBoxJobs * (kWgChunk / 16) + kT - 1) / kT;
+        const int ct = tid - 64, Hc = a.H >> 1, Wc = a.W >> 1;
+        for (int it = 0; it < count; ++it) {
+            const int b = it % kWgStages;
+            const int s = first + it * (int)gridDim.x;
+            const int xs = s % sx, t = s / sx;
+            const int y0 = (t % sy) * kWgRows, n = t / sy, x0 = xs * kWgStrip;
+            const int cy0 = (y0 - 1) >> 1, cx0 = (x0 - 1) >> 1;
+            uint4 v[kJobs];
+#pragma unroll
+            for (int u = 0; u < kJobs; ++u) {
+                const int i = ct + u * kT, box = i / kBoxJobs, j = i % kBoxJobs, half = j & 1, p = j >> 1;
+                const int cy = cy0 + p / kCx, cx = cx0 + p % kCx;
+                v[u] = make_uint4(0, 0, 0, 0);
+                if (box < ncx && cy >= 0 && cy < Hc && cx >= 0 && cx < Wc)
+                    v[u] = __ldg(reinterpret_cast<const uint4*>(a.coarse + (((size_t)n * Hc + cy) * Wc + cx) * a.coarse_cs + c0 +
+                                                                box * 16 + half * 8));
+            }
+            if (!warp_wait(saddr(empty + b), ((uint32_t)(it / kWgStages) & 1u) ^ 1u, abort_flag, a.status)) {
+                ok = false;
+                break;
+            }
+            unsigned char* xb = stage0 + b * kWgStage + 8 * kWgDyBox;
+#pragma unroll
+            for (int u = 0; u < kJobs; ++u) {
+                const int i = ct + u * kT, box = i / kBoxJobs, j = i % kBoxJobs, half = j & 1, p = j >> 1;
+                if (box >= ncx) continue;
+                const int hy0 = 2 * (cy0 + p / kCx) - (y0 - 1), hx0 = 2 * (cx0 + p % kCx) - (x0 - 1);
+#pragma unroll
+                for (int d = 0; d < 4; ++d) {
+                    const int hy = hy0 + (d >> 1), hx = hx0 + ((d ^ (p >> 1)) & 1);
+                    if (hy < 0 || hy >= kWgRows + 2 || hx < 0 || hx >= kWgHaloW) continue;
+                    const int px = hy * kWgHaloW + hx;
+                    *reinterpret_cast<uint4*>(xb + box * kWgXBox + px * 32 + ((half ^ ((px >> 2) & 1)) << 4)) = v[u];
+                }
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // these stores -> tensor core reads
+            __syncwarp();
+            if (lane == 0) mbar_arrive(saddr(full + b));
+        }
     }
     __syncwarp();
     // epilogue: TMEM lane (warp * 32 + lane) holds output channel co for every tap
     const bool got = count == 0 || wait_or_abort(saddr(acc), 0u, abort_flag, a.status);
-    if (__all_sync(0xffffffffu, got && !*abort_flag)) {  // warp-uniform: tcgen05.ld is .aligned
+    if (warp >= 4) {
+        // an expanding warp: the four warps below move the accumulators
+    } else if (__all_sync(0xffffffffu, got && !*abort_flag)) {  // warp-uniform: tcgen05.ld is .aligned
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         // M = 128: row i in TMEM lane i.  M = 64: rows 16w..16w+15 in lanes 32w..32w+15 of
         // warp w's quarter (the upper 16 lanes of each quarter are unused)
@@ -856,50 +909,37 @@ k_wgrad_tc(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUt
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" :: "r"(tmem) : "memory");
 }
 
-// [up2(coarse) | skip] (a decoder convolution's input) written out as one NHWC tensor
-__global__ void k_concat_src(const ConvSrc x, int cin, int N, int H, int W, bf16* __restrict__ out) {
-    const int c8 = cin / 8;
-    const long long n8 = (long long)N * H * W * c8;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n8; i += (long long)gridDim.x * blockDim.x) {
-        const int o = (int)(i % c8);
-        const long long px = i / c8;
-        const int xx = (int)(px % W);
-        const long long r = px / W;
-        const int yy = (int)(r % H), n = (int)(r / H);
-        *reinterpret_cast<uint4*>(out + px * cin + o * 8) =
-            __ldg(reinterpret_cast<const uint4*>(src_at(x, n, yy, xx, H, W, o * 8)));
-    }
-}
-
-// dw[tap][co][ci] += sum over slices s of part[s][tap][co][ci].  A block takes 32 groups of four
-// neighbouring input channels; its 8 rows of threads add a strided share of the slices each, and
-// the shares are added in row order (one thread per output walked up to 152 slices one after
-// another: 16 us per layer, latency).
-__global__ void __launch_bounds__(256) k_wgrad_reduce(const float* __restrict__ part, int slices, int cpad, int cin,
-                                                      int cout, float* __restrict__ dw) {
+// Adds every entry's partial slices to its destination: a block takes 32 groups of four
+// neighbouring outputs of one entry; its 8 rows of threads add a strided share of the slices
+// each, and the shares are added in row order.  One launch for a whole backward pass: one per
+// layer (8 us each, latency) took 190 us of 1.73 ms at 16 x 256 x 256.
+__global__ void __launch_bounds__(256) k_grad_reduce(const __grid_constant__ GradReduceTable T) {
     __shared__ float4 sm[8][32];
+    int e = 0;
+    while (e + 1 < T.n && (int)blockIdx.x >= T.e[e + 1].block0) ++e;
+    const GradReduceTable::Entry E = T.e[e];
     const int col = threadIdx.x & 31, row = threadIdx.x >> 5;
-    const int i = blockIdx.x * 32 + col;  // (tap, co, ci / 4), ci fastest
-    const int c4 = cin / 4, n = 9 * cout * c4;
+    const int i = ((int)blockIdx.x - E.block0) * 32 + col;
     float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (i < n) {
-        const int ci = (i % c4) * 4, r = i / c4, co = r % cout, tap = r / cout;
-        const size_t stride = (size_t)9 * cpad * cin;
-        const float* p = part + ((size_t)tap * cpad + co) * cin + ci;
+    if (i < E.groups) {
+        // output group i = (r, j) of the destination's rows of E.row4 groups, E.rows rows per
+        // tap; a slice has E.pad_rows rows per tap
+        const int j = i % E.row4, r = i / E.row4;
+        const float* p = E.part + ((size_t)(r / E.rows) * E.pad_rows + r % E.rows) * E.row4 * 4 + j * 4;
 #pragma unroll 4
-        for (int k = row; k < slices; k += 8) {
-            const float4 v = __ldg(reinterpret_cast<const float4*>(p + k * stride));
+        for (int k = row; k < E.slices; k += 8) {
+            const float4 v = __ldg(reinterpret_cast<const float4*>(p + (size_t)k * E.stride));
             s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
         }
     }
     sm[row][col] = s;
     __syncthreads();
-    if (row != 0 || i >= n) return;
+    if (row != 0 || i >= E.groups) return;
     for (int k = 1; k < 8; ++k) {
         const float4 v = sm[k][col];
         s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
     }
-    float* d = dw + (size_t)i * 4;  // a layer's gradients start on any 4-byte boundary
+    float* d = E.dst + (size_t)i * 4;  // a layer's gradients start on any 4-byte boundary
     d[0] += s.x;
     d[1] += s.y;
     d[2] += s.z;
@@ -1007,10 +1047,14 @@ size_t conv_wgrad_tc_workspace(int num_sms, int cin, int cpad, int N, int H, int
 }
 
 salty_status conv_wgrad_tc(salty_ctx* ctx, const bf16* dy, int cpad, int cout, const ConvSrc& x, int cin, float* dw,
-                           int N, int H, int W, float* ws, size_t ws_floats, bf16* cat_ws, size_t cat_elems,
-                           int* d_status) {
-    if (cin % 16 || cin <= 0 || cpad % 16 || cpad < 16 || cpad > 128 || cout > cpad || cout < 1 ||
-        reinterpret_cast<uintptr_t>(dy) % 16 || reinterpret_cast<uintptr_t>(ws) % 16)
+                           int N, int H, int W, float* ws, size_t ws_floats, int* d_status, GradReduceTable& table) {
+    const bool coarse = x.a_ch < cin;  // [up2(a) | b]
+    const bf16* src = coarse ? x.b : x.a;
+    const int src_cs = coarse ? x.b_cs : x.a_cs;
+    if (cin % 16 || cin <= 0 || cpad % 16 || cpad < 16 || cpad > 128 || cout > cpad || cout < 1 || src_cs % 16 ||
+        (coarse ? x.a_shift != 1 || x.a_ch % 16 || x.a_cs % 8 || H % 2 || W % 2 || reinterpret_cast<uintptr_t>(x.a) % 16
+                : x.a_shift != 0) ||
+        reinterpret_cast<uintptr_t>(src) % 16 || reinterpret_cast<uintptr_t>(dy) % 16 || reinterpret_cast<uintptr_t>(ws) % 16)
         return ctx->err.fail(SALTY_ERR_INVALID_ARG, "conv_wgrad_tc: unsupported shape (cin %d, cout %d)", cin, cout);
     EncodeTiledFn enc = tensor_map_encoder();
     if (!enc) return ctx->err.fail(SALTY_ERR_CUDA, "conv_wgrad_tc: cuTensorMapEncodeTiled is not available");
@@ -1018,27 +1062,12 @@ salty_status conv_wgrad_tc(salty_ctx* ctx, const bf16* dy, int cpad, int cout, c
     wgrad_plan(ctx->num_sms, cin, N, H, W, &groups, &slices, &strips);
     if ((size_t)slices * 9 * cpad * cin > ws_floats)
         return ctx->err.fail(SALTY_ERR_CAPACITY, "conv_wgrad_tc: workspace too small");
-    // the input as one NHWC tensor: as given, or the decoder's concatenation written out
-    const bf16* xin = x.a;
-    int xcs = x.a_cs;
-    const long long npx = (long long)N * H * W;
-    if (x.a_shift != 0 || x.a_ch < cin) {
-        if ((size_t)(npx * cin) > cat_elems)
-            return ctx->err.fail(SALTY_ERR_CAPACITY, "conv_wgrad_tc: concatenation workspace too small");
-        const long long n8 = npx * (cin / 8);
-        k_concat_src<<<(unsigned)std::min<long long>((n8 + 255) / 256, (long long)ctx->num_sms * 16), 256, 0,
-                       ctx->stream>>>(x, cin, N, H, W, cat_ws);
-        xin = cat_ws;
-        xcs = cin;
-    }
-    if (reinterpret_cast<uintptr_t>(xin) % 16 || xcs % 16)
-        return ctx->err.fail(SALTY_ERR_INVALID_ARG, "conv_wgrad_tc: input not 16-byte aligned");
     CUtensorMap tm_x, tm_dy;
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     const cuuint32_t xbox[4] = {16, (cuuint32_t)kWgHaloW, (cuuint32_t)(kWgRows + 2), 1};
-    const cuuint64_t xdim[4] = {(cuuint64_t)cin, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)N};
-    const cuuint64_t xstr[3] = {(cuuint64_t)xcs * 2, (cuuint64_t)W * xcs * 2, (cuuint64_t)H * W * xcs * 2};
-    if (enc(&tm_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<bf16*>(xin), xdim, xstr, xbox, estr,
+    const cuuint64_t xdim[4] = {(cuuint64_t)src_cs, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)N};
+    const cuuint64_t xstr[3] = {(cuuint64_t)src_cs * 2, (cuuint64_t)W * src_cs * 2, (cuuint64_t)H * W * src_cs * 2};
+    if (enc(&tm_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<bf16*>(src), xdim, xstr, xbox, estr,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return ctx->err.fail(SALTY_ERR_CUDA, "conv_wgrad_tc: input tensor map");
@@ -1051,10 +1080,23 @@ salty_status conv_wgrad_tc(salty_ctx* ctx, const bf16* dy, int cpad, int cout, c
         return ctx->err.fail(SALTY_ERR_CUDA, "conv_wgrad_tc: gradient tensor map");
     const size_t smem = (size_t)kWgHeader + (size_t)kWgStages * kWgStage;
     SALTY_TRY_CUDA(ctx->err, cudaFuncSetAttribute(k_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    WgradArgs a{cpad <= 64 ? 64 : 128, cpad, cout, cin, N, H, W, strips, ws, d_status};
-    k_wgrad_tc<<<dim3(slices, groups), kWgThreads, smem, ctx->stream>>>(tm_x, tm_dy, a);
-    const int groups4 = 9 * cout * (cin / 4);
-    k_wgrad_reduce<<<(unsigned)((groups4 + 31) / 32), 256, 0, ctx->stream>>>(ws, slices, cpad, cin, cout, dw);
+    WgradArgs a{cpad <= 64 ? 64 : 128, cpad, cout, cin, N, H, W, strips, ws, coarse ? x.a : nullptr,
+                coarse ? x.a_cs : 0, coarse ? x.a_ch : 0, d_status};
+    k_wgrad_tc<<<dim3(slices, groups), coarse ? kWgCoarseThreads : kWgThreads, smem, ctx->stream>>>(tm_x, tm_dy, a);
+    SALTY_TRY_CUDA(ctx->err, cudaGetLastError());
+    return grad_reduce_add(ctx, table, {ws, dw, slices, 9 * cpad * cin, cin / 4, cout, cpad, 9 * cout * (cin / 4), 0});
+}
+
+salty_status grad_reduce_add(salty_ctx* ctx, GradReduceTable& table, GradReduceTable::Entry e) {
+    if (table.n >= GradReduceTable::kMax) return ctx->err.fail(SALTY_ERR_CAPACITY, "gradient reduction table full");
+    e.block0 = table.blocks;
+    table.blocks += (e.groups + 31) / 32;
+    table.e[table.n++] = e;
+    return SALTY_OK;
+}
+
+salty_status grad_reduce_run(salty_ctx* ctx, const GradReduceTable& table) {
+    if (table.blocks > 0) k_grad_reduce<<<table.blocks, 256, 0, ctx->stream>>>(table);
     SALTY_TRY_CUDA(ctx->err, cudaGetLastError());
     return SALTY_OK;
 }

@@ -361,7 +361,7 @@ __global__ void k_pool(const bf16* __restrict__ in, bf16* __restrict__ out, int 
 }
 
 // Block sums of the bias gradient: per-thread sums s[8] (8-channel group j of G, thread row r of
-// `per`) added in shared memory in row order into part[blockIdx.x][c], c < C; k_bias_reduce adds
+// `per`) added in shared memory in row order into part[blockIdx.x][c], c < C; k_grad_reduce adds
 // the blocks' partials.
 __device__ __forceinline__ void bias_partials(float* sb, const float (&s)[8], int j, int r, int per, int C,
                                               float* __restrict__ part) {
@@ -520,22 +520,6 @@ __global__ void __launch_bounds__(256) k_grad_in(const bf16* __restrict__ y, Gra
         }
     }
     bias_partials(sb, s, j, r, per, C, part);
-}
-
-// db[c] += the blocks' partials: 32 threads per channel, each a strided share, then their sums
-// in a fixed order (one thread per channel took 36 us per layer for 608 blocks).
-__global__ void __launch_bounds__(256) k_bias_reduce(const float* __restrict__ part, int blocks, int C,
-                                                     float* __restrict__ db) {
-    __shared__ float sm[32][9];
-    const int cl = threadIdx.x & 7, r = threadIdx.x >> 3, c = blockIdx.x * 8 + cl;
-    float t = 0.0f;
-    for (int b = r; b < blocks; b += 32) t += part[(size_t)b * C + c];
-    sm[r][cl] = t;
-    __syncthreads();
-    if (r != 0) return;
-    t = 0.0f;
-    for (int i = 0; i < 32; ++i) t += sm[i][cl];
-    db[c] += t;
 }
 
 // Up to four symmetries of one shape, as the self-ensemble's forward passes take them.
@@ -704,7 +688,7 @@ struct Unet {
     DevBuf<float> film_ws;  // a film's input records and the denoised image (salty_denoise_unet)
     DevBuf<double> loss;
     DevBuf<float> wg_ws;    // per-CTA partial weight and bias gradients (fixed-order sums)
-    DevBuf<bf16> cat_ws;    // a decoder convolution's concatenated input, for its weight gradient
+    size_t wg_off[kNumLayers], wg_len[kNumLayers], bias_off[kNumLayers], wg_floats;  // each layer's, in floats
     int conv_kind = SALTY_CONV_TCGEN05;  // convolution kernels (forward, backward-data, weights)
 };
 
@@ -772,11 +756,11 @@ salty_status launch_conv(salty_ctx* ctx, int kind, const ConvSrc& in, int cin, c
     return SALTY_OK;
 }
 
-salty_status launch_wgrad(salty_ctx* ctx, Unet& u, const bf16* dy, int cpad, int cout, const ConvSrc& x, int cin,
-                          float* dw, int N, int H, int W) {
+salty_status launch_wgrad(salty_ctx* ctx, Unet& u, int li, const bf16* dy, int cpad, int cout, const ConvSrc& x, int cin,
+                          float* dw, int N, int H, int W, GradReduceTable& table) {
     if (u.conv_kind != SALTY_CONV_MMA_SYNC)
-        return conv_wgrad_tc(ctx, dy, cpad, cout, x, cin, dw, N, H, W, u.wg_ws.p, u.wg_ws.cap, u.cat_ws.p,
-                             u.cat_ws.cap, ctx->status.p + 8);
+        return conv_wgrad_tc(ctx, dy, cpad, cout, x, cin, dw, N, H, W, u.wg_ws.p + u.wg_off[li], u.wg_len[li],
+                             ctx->status.p + 8, table);
     const size_t smem = ((size_t)kTileX * kTileY * (kWgradCo + 8) + (size_t)kHaloX * kHaloY * 24) * sizeof(bf16);
     const int tiles = N * ((W + kTileX - 1) / kTileX) * ((H + kTileY - 1) / kTileY);
     const int mg = (cpad + kWgradCo - 1) / kWgradCo;
@@ -799,20 +783,18 @@ salty_status ensure_workspace(salty_ctx* ctx, Unet& u, int N, int H, int W) {
     long long o = 0;
     for (int i = 0; i < T_COUNT; ++i) { u.act_off[i] = o; o += (asz[i] + 63) / 64 * 64; }
     SALTY_TRY_CUDA(ctx->err, u.act.ensure((size_t)o));
+    // per layer: the weight gradient's slices, and 4 blocks per SM of bias partials
     size_t ws = 0;
     for (int i = 0; i < kNumLayers; ++i) {
         const UnetLayer& L = u.layers[i];
         const int lv = kLayerLevel[i];
-        ws = std::max(ws, conv_wgrad_tc_workspace(ctx->num_sms, L.cin, L.cout_pad, N, H >> lv, W >> lv));
+        u.wg_off[i] = ws;
+        u.wg_len[i] = conv_wgrad_tc_workspace(ctx->num_sms, L.cin, L.cout_pad, N, H >> lv, W >> lv);
+        ws += (u.wg_len[i] + 63) / 64 * 64;
+        u.bias_off[i] = ws;
+        ws += ((size_t)ctx->num_sms * 4 * L.cout + 63) / 64 * 64;
     }
-    // the bias gradients' per-block partials use the same workspace: up to 4 blocks per SM
-    // x 128 channels
-    ws = std::max(ws, (size_t)ctx->num_sms * 4 * 128);
-    SALTY_TRY_CUDA(ctx->err, u.wg_ws.ensure(ws));
-    size_t cat = 0;
-    for (int i = 0; i < kNumLayers; ++i)
-        cat = std::max(cat, (size_t)N * (H >> kLayerLevel[i]) * (W >> kLayerLevel[i]) * u.layers[i].cin);
-    SALTY_TRY_CUDA(ctx->err, u.cat_ws.ensure(cat));
+    u.wg_floats = ws;
     u.N = N; u.H = H; u.W = W;
     return SALTY_OK;
 }
@@ -870,25 +852,33 @@ int grad_blocks(salty_ctx* ctx, long long work, int per) {
     return (int)std::min<long long>((long long)ctx->num_sms * 4, (work + per - 1) / per);
 }
 
-// The output gradient of layer li in T_G (BF16), with its bias gradient added.
+salty_status bias_reduce_add(salty_ctx* ctx, Unet& u, int li, int blocks, GradReduceTable& table) {
+    const UnetLayer& L = u.layers[li];
+    return grad_reduce_add(ctx, table, {u.wg_ws.p + u.bias_off[li], u.grads.p + L.b_off, blocks, L.cout, L.cout / 4, 1, 1,
+                                        L.cout / 4, 0});
+}
+
+// The output gradient of layer li in T_G (BF16) and its bias gradient's partial sums.
 template <int KIND>
-salty_status grad_in(salty_ctx* ctx, Unet& u, Fwd& F, int li, int y, const GradSrc& src, int N, int h, int w) {
+salty_status grad_in(salty_ctx* ctx, Unet& u, Fwd& F, int li, int y, const GradSrc& src, int N, int h, int w,
+                     GradReduceTable& table) {
     const UnetLayer& L = u.layers[li];
     const long long npx = (long long)N * h * w, work = KIND == GRAD_SKIP ? npx / 4 : npx;
     const int per = 256 / (L.cout / 8), blocks = grad_blocks(ctx, work, per);
     k_grad_in<KIND><<<blocks, 256, (size_t)per * L.cout * sizeof(float), ctx->stream>>>(F.t[y], src, L.cout, N, h, w,
-                                                                                      F.t[T_G], u.wg_ws.p);
-    k_bias_reduce<<<L.cout / 8, 256, 0, ctx->stream>>>(u.wg_ws.p, blocks, L.cout, u.grads.p + L.b_off);
+                                                                                      F.t[T_G],
+                                                                                      u.wg_ws.p + u.bias_off[li]);
     SALTY_TRY_CUDA(ctx->err, cudaGetLastError());
-    return SALTY_OK;
+    return bias_reduce_add(ctx, u, li, blocks, table);
 }
 
 // Weight gradient of layer li from its output gradient in T_G, and, with dx >= 0, the gradient
 // of its input in that tensor ([npx][cin], BF16).
-salty_status conv_backward(salty_ctx* ctx, Unet& u, Fwd& F, int li, const ConvSrc& x, int N, int h, int w, int dx) {
+salty_status conv_backward(salty_ctx* ctx, Unet& u, Fwd& F, int li, const ConvSrc& x, int N, int h, int w, int dx,
+                           GradReduceTable& table) {
     const UnetLayer& L = u.layers[li];
     bf16* g = F.t[T_G];
-    SALTY_TRY(launch_wgrad(ctx, u, g, L.cout_pad, L.cout, x, L.cin, u.grads.p + L.w_off, N, h, w));
+    SALTY_TRY(launch_wgrad(ctx, u, li, g, L.cout_pad, L.cout, x, L.cin, u.grads.p + L.w_off, N, h, w, table));
     if (dx >= 0)
         SALTY_TRY(launch_conv(ctx, u.conv_kind, conv_src(g, L.cout_pad, L.cout_pad), L.cout_pad, u.wb.p + L.wb_off,
                               L.rows_bwd, L.nt_b, nullptr, F.t[dx], L.cin, L.cin, N, h, w, 0));
@@ -899,6 +889,8 @@ salty_status conv_backward(salty_ctx* ctx, Unet& u, Fwd& F, int li, const ConvSr
 salty_status backward(salty_ctx* ctx, Unet& u, Fwd& F, const float* d_target, int N, int H, int W, double* loss) {
     cudaStream_t st = ctx->stream;
     const long long P0 = (long long)N * H * W;
+    GradReduceTable table;
+    SALTY_TRY_CUDA(ctx->err, u.wg_ws.ensure(u.wg_floats));
     SALTY_TRY_CUDA(ctx->err, cudaMemsetAsync(u.grads.p, 0, u.n_params * sizeof(float), st));
     SALTY_TRY_CUDA(ctx->err, u.loss.ensure(1));
     SALTY_TRY_CUDA(ctx->err, cudaMemsetAsync(u.loss.p, 0, sizeof(double), st));
@@ -906,21 +898,22 @@ salty_status backward(salty_ctx* ctx, Unet& u, Fwd& F, const float* d_target, in
     auto x = [&](int t, int c) { return conv_src(F.t[t], c, c); };
     auto cat = [&](int coarse, int cc, int skip, int cs) { return conv_src_cat(F.t[coarse], cc, F.t[skip], cs); };
     auto plain = [&](int li, int y, int h, int w) {
-        return grad_in<GRAD_PLAIN>(ctx, u, F, li, y, GradSrc{F.t[T_G2], u.layers[li].cout, 0, nullptr}, N, h, w);
+        return grad_in<GRAD_PLAIN>(ctx, u, F, li, y, GradSrc{F.t[T_G2], u.layers[li].cout, 0, nullptr}, N, h, w, table);
     };
     auto up = [&](int li, int y, int dcat, int ch, int h, int w) {
-        return grad_in<GRAD_UP>(ctx, u, F, li, y, GradSrc{F.t[dcat], ch, 0, nullptr}, N, h, w);
+        return grad_in<GRAD_UP>(ctx, u, F, li, y, GradSrc{F.t[dcat], ch, 0, nullptr}, N, h, w, table);
     };
     auto skip = [&](int li, int y, int dcat, int ch, int off, int h, int w) {
-        return grad_in<GRAD_SKIP>(ctx, u, F, li, y, GradSrc{F.t[dcat], ch, off, F.t[T_G2]}, N, h, w);
+        return grad_in<GRAD_SKIP>(ctx, u, F, li, y, GradSrc{F.t[dcat], ch, off, F.t[T_G2]}, N, h, w, table);
     };
     auto back = [&](int li, const ConvSrc& in, int h, int w, int dx) {
-        return conv_backward(ctx, u, F, li, in, N, h, w, dx);
+        return conv_backward(ctx, u, F, li, in, N, h, w, dx, table);
     };
     // the loss, its gradient and the output layer's bias gradient
     const int lb = grad_blocks(ctx, P0, 256);
-    k_loss_bwd<<<lb, 256, 256 * 8 * sizeof(float), st>>>(F.t[T_OUT], F.t[T_X], d_target, P0, F.t[T_G], u.wg_ws.p, u.loss.p);
-    k_bias_reduce<<<1, 256, 0, st>>>(u.wg_ws.p, lb, 8, u.grads.p + u.layers[13].b_off);
+    k_loss_bwd<<<lb, 256, 256 * 8 * sizeof(float), st>>>(F.t[T_OUT], F.t[T_X], d_target, P0, F.t[T_G],
+                                                         u.wg_ws.p + u.bias_off[13], u.loss.p);
+    SALTY_TRY(bias_reduce_add(ctx, u, 13, lb, table));
     SALTY_TRY(back(13, x(T_D0, 32), H, W, T_G2));
     SALTY_TRY(plain(12, T_D0, H, W));
     SALTY_TRY(back(12, cat(T_D1, 48, T_E0, 32), H, W, T_C0));
@@ -948,6 +941,7 @@ salty_status backward(salty_ctx* ctx, Unet& u, Fwd& F, const float* d_target, in
     SALTY_TRY(back(1, x(T_A0, 32), H, W, T_G2));
     SALTY_TRY(plain(0, T_A0, H, W));
     SALTY_TRY(back(0, x(T_X, 16), H, W, -1));
+    SALTY_TRY(grad_reduce_run(ctx, table));
     SALTY_TRY_CUDA(ctx->err, cudaGetLastError());
     double l = 0.0;
     SALTY_TRY_CUDA(ctx->err, cudaMemcpyAsync(&l, u.loss.p, sizeof(double), cudaMemcpyDeviceToHost, st));

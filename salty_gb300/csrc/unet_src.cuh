@@ -4,7 +4,7 @@
 // [0, a_ch) are the coarse level's, nearest-up-sampled (read at (y >> 1, x >> 1) of an image
 // half as tall and wide), channels [a_ch, cin) the skip connection's at (y, x).  The
 // convolution kernels read both where they stage their input tiles, so the concatenated
-// tensor is never written in a forward pass.  A plain input is source a alone (a_shift 0, a_ch = cin).
+// tensor is never written.  A plain input is source a alone (a_shift 0, a_ch = cin).
 #pragma once
 
 #include <cuda_bf16.h>
@@ -51,15 +51,32 @@ salty_status conv3x3_tma(salty_ctx* ctx, const ConvSrc& in, int cin, const __nv_
                          const float* bias, __nv_bfloat16* out, __nv_bfloat16* pool, int out_cs, int cout, int N,
                          int H, int W, int relu, int* d_status);
 
-// Weight gradient of a 3x3 convolution on tcgen05, deterministic (partial sums per CTA,
-// added in a fixed order): dw[9][cout][cin] += sum over pixels of dY x X(tap).  dy
-// [N][H][W][cpad] (cpad = cout rounded up to 16, <= 128, zero beyond cout, 16-byte
-// aligned); x the layer's input (cin % 16 == 0; a decoder's concatenation is first written
-// out into cat_ws, N*H*W*cin elements); ws a workspace of at least
-// conv_wgrad_tc_workspace(...) floats.
+// Partial sums of a backward pass waiting to be added to the gradients: slices of
+// [taps][pad_rows][row4 float4] floats, `stride` floats apart; the destination's rows are the
+// first `rows` of each tap.  Filled as the layers' kernels are launched, added up by one launch.
+struct GradReduceTable {
+    static constexpr int kMax = 32;
+    struct Entry {
+        const float* part;  // 16-byte aligned
+        float* dst;
+        int slices, stride, row4, rows, pad_rows;
+        int groups;         // float4 groups of the destination
+        int block0;
+    };
+    int n = 0, blocks = 0;
+    Entry e[kMax];
+};
+salty_status grad_reduce_add(salty_ctx* ctx, GradReduceTable& table, GradReduceTable::Entry e);
+salty_status grad_reduce_run(salty_ctx* ctx, const GradReduceTable& table);
+
+// Weight gradient of a 3x3 convolution on tcgen05, deterministic (partial sums per CTA, added
+// in a fixed order): dw[9][cout][cin] += sum over pixels of dY x X(tap) once the table has been
+// run.  dy [N][H][W][cpad] (cpad = cout rounded up to 16, <= 128, zero beyond cout, 16-byte
+// aligned); x the layer's input (cin % 16 == 0), one tensor or [up2(coarse) | skip]; ws a
+// workspace of its own of at least conv_wgrad_tc_workspace(...) floats.
 size_t conv_wgrad_tc_workspace(int num_sms, int cin, int cpad, int N, int H, int W);
 salty_status conv_wgrad_tc(salty_ctx* ctx, const __nv_bfloat16* dy, int cpad, int cout, const ConvSrc& x, int cin,
-                           float* dw, int N, int H, int W, float* ws, size_t ws_floats, __nv_bfloat16* cat_ws,
-                           size_t cat_elems, int* d_status);
+                           float* dw, int N, int H, int W, float* ws, size_t ws_floats, int* d_status,
+                           GradReduceTable& table);
 
 }  // namespace salty
