@@ -58,9 +58,10 @@
 // overlap the MMAs of the next.  Waits are bounded as above; a wait that gives up raises
 // a shared abort flag that ends every role's loop.
 // Measured (GB300; film denoise at 1080p, 8 symmetries as two batches of 4 images): all
-// convolutions 5.81 -> 3.05 ms against one N = Npad MMA per tap and row from eight diverged
-// lanes, with the decoder inputs staged by k_conv3x3_tc.  The 32 -> 32 layer at full
-// resolution now moves 1.2 GB in 213 us (5.6 TB/s, 0.83 of the copy peak).
+// convolutions 5.81 -> 2.64 ms against one N = Npad MMA per tap and row from eight diverged
+// lanes, with the decoder inputs staged by k_conv3x3_tc.  The full-resolution 32 -> 32 layer
+// with its pooled output moves 1.2 GB in 196 us (6.1 TB/s, 0.90 of the copy peak); the
+// decoder's up(48) + 32 -> 32 takes 310 us, bound by the MMAs' operand reads.
 #include <cuda.h>  // CUtensorMap and its enums (the encoder is fetched from the driver at run time)
 #include <cuda_bf16.h>
 
@@ -148,6 +149,21 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
           "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// The same load without its wait, and the wait, which the values depend on.
+__device__ __forceinline__ void tmem_ld16_issue(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+                 :: "memory");
 }
 
 struct TcConvArgs {
@@ -460,7 +476,9 @@ k_conv3x3_tma(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__
         if (lane == 0) {
             asm volatile("prefetch.tensormap [%0];" :: "l"(reinterpret_cast<uint64_t>(&tm_in)) : "memory");
             asm volatile("prefetch.tensormap [%0];" :: "l"(reinterpret_cast<uint64_t>(&tm_w)) : "memory");
-            int k = 0;
+            int s = 0;
+            uint32_t ph = 0;
+            auto next = [&]() { if (++s == S) { s = 0; ph ^= 1u; } };
             for (int t = blockIdx.x; t < a.tiles; t += gridDim.x) {
                 int tt = t;
                 const int sx = tt % strips_x;
@@ -469,14 +487,12 @@ k_conv3x3_tma(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__
                 const int n = tt / strips_y;
                 const int x0 = sx * kStrip, y0 = sy * R;
                 bool ok = true;
-                for (int c = 0; c < nchunks; ++c, ++k) {
+                for (int c = 0; c < nchunks; ++c, next()) {
                     if (a.resident && t == (int)blockIdx.x) {  // the chunk's weights, once
                         const uint32_t wb = saddr(hd.wbar + c);
                         mbar_expect_tx(wb, wchunk);
                         load_weights(saddr(wres) + c * wchunk, c, wb);
                     }
-                    const int s = k % S;
-                    const uint32_t ph = (uint32_t)(k / S) & 1u;
                     // every chunk's stage is waited for, whoever fills it: a parity tells two
                     // successive uses of a stage apart, not a use from the next but one
                     if (!wait_or_abort(saddr(hd.empty + s), ph ^ 1u, abort_flag, a.status)) { ok = false; break; }
@@ -496,17 +512,17 @@ k_conv3x3_tma(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__
         const uint64_t d0 = sdesc_sw32(0);
         const uint32_t dlo = (uint32_t)d0, dhi = (uint32_t)(d0 >> 32);
         const uint32_t idesc = idesc_bf16(kStrip, 0), nbit = (uint32_t)(npad >> 3) << 17;  // + n * nbit: N = n * npad
-        int k = 0, i = 0;
+        int s = 0, i = 0;
+        uint32_t ph = 0;  // parity of the ring position's use
         for (int t = blockIdx.x; t < a.tiles; t += gridDim.x, ++i) {
             const int ab = i & 1;
             if (!warp_wait(saddr(hd.acc_empty + ab), ((uint32_t)(i >> 1) & 1u) ^ 1u, abort_flag, a.status)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t acc = tmem + (uint32_t)ab * 256u;  // row r in columns (R - 1 - r) npad ..
             bool ok = true;
-            for (int c = 0; c < nchunks; ++c, ++k) {
-                const int s = k % S;
+            for (int c = 0; c < nchunks; ++c) {
                 if (a.resident && i == 0) ok = warp_wait(saddr(hd.wbar + c), 0u, abort_flag, a.status);
-                if (!ok || !warp_wait(saddr(hd.full + s), (uint32_t)(k / S) & 1u, abort_flag, a.status)) { ok = false; break; }
+                if (!ok || !warp_wait(saddr(hd.full + s), ph, abort_flag, a.status)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t hs = saddr(ring + s * sbytes);
                 const uint32_t ws = a.resident ? saddr(wres) + c * wchunk : hs + hbytes;
@@ -528,13 +544,19 @@ k_conv3x3_tma(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__
                     umma_elect(col, ah + 4u, bh + 2u * kxs, dhi, idesc + (uint32_t)n * nbit, el, 1u);
                 }
                 umma_commit_elect(saddr(hd.empty + s), el);
+                if (++s == S) { s = 0; ph ^= 1u; }
             }
             if (!ok) break;
             umma_commit_elect(saddr(hd.acc_full + ab), el);
         }
     } else if (!COARSE || warp < 2 + kTmaEpiWarps) {
+        // The operand reads of the MMAs keep shared memory busy, so a load from it takes hundreds
+        // of cycles here: the bias stays in registers for a strip's rows of 16 channels.
         const int q = warp & 3, sub = (warp - 2) >> 2;  // TMEM lane quarter; which of its two warps
         const int J = npad / 16;
+        // the quarter's two warps share the rows (pooled: row pairs), or the channels of a single one
+        const int rstep = a.pool ? 2 : 1, units = R / rstep;
+        const int u0 = units > 1 ? sub : 0, ustep = units > 1 ? 2 : 1, j0 = units > 1 ? 0 : sub, jstep = units > 1 ? 1 : 2;
         int i = 0;
         for (int t = blockIdx.x; t < a.tiles; t += gridDim.x, ++i) {
             const int ab = i & 1;
@@ -547,35 +569,37 @@ k_conv3x3_tma(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__
             const int n = tt / strips_y;
             const int x = sx * kStrip + q * 32 + lane;
             const uint32_t acc = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)ab * 256u;
-            // 16 channels of row r of this lane's pixel, stored; left in pk
-            auto item = [&](int r, int j, uint32_t (&pk)[8]) {
-                uint32_t v[16];
-                tmem_ld16(acc + (uint32_t)((R - 1 - r) * npad + j * 16), v);
+            bf16* const orow = a.out + (((size_t)n * a.H + sy * R) * a.W + x) * a.out_cs;
+            const size_t rpitch = (size_t)a.W * a.out_cs;
+            for (int j = j0; j < J; j += jstep) {
+                float bias[16];
                 const float4* b4 = reinterpret_cast<const float4*>(sbias + j * 16);
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const float4 b = b4[e];
-                    float f0 = __uint_as_float(v[4 * e]) + b.x, f1 = __uint_as_float(v[4 * e + 1]) + b.y;
-                    float f2 = __uint_as_float(v[4 * e + 2]) + b.z, f3 = __uint_as_float(v[4 * e + 3]) + b.w;
-                    if (a.relu) {
-                        f0 = fmaxf(f0, 0.0f); f1 = fmaxf(f1, 0.0f);
-                        f2 = fmaxf(f2, 0.0f); f3 = fmaxf(f3, 0.0f);
-                    }
-                    const __nv_bfloat162 p0 = __floats2bfloat162_rn(f0, f1), p1 = __floats2bfloat162_rn(f2, f3);
-                    pk[2 * e] = *reinterpret_cast<const uint32_t*>(&p0);
-                    pk[2 * e + 1] = *reinterpret_cast<const uint32_t*>(&p1);
+                    bias[4 * e] = b.x; bias[4 * e + 1] = b.y; bias[4 * e + 2] = b.z; bias[4 * e + 3] = b.w;
                 }
-                const int y = sy * R + r;
-                if (y < a.H && x < a.W && j * 16 < a.cout)
-                    store_pixel16(a.out + (((size_t)n * a.H + y) * a.W + x) * a.out_cs + j * 16, pk, j * 16 + 16 <= a.cout);
-            };
-            if (a.pool) {
-                for (int r = 0; r < R; r += 2)
-                    for (int j = 0; j < J; ++j) {
-                        if ((((r >> 1) * J + j) & 1) != sub) continue;
-                        uint32_t p0[8], p1[8];
-                        item(r, j, p0);
-                        item(r + 1, j, p1);
+                const bool live = x < a.W && j * 16 < a.cout, full = j * 16 + 16 <= a.cout;
+                auto finish = [&](const uint32_t (&v)[16], int r, uint32_t (&pk)[8]) {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        float f0 = __uint_as_float(v[2 * e]) + bias[2 * e], f1 = __uint_as_float(v[2 * e + 1]) + bias[2 * e + 1];
+                        if (a.relu) { f0 = fmaxf(f0, 0.0f); f1 = fmaxf(f1, 0.0f); }
+                        const __nv_bfloat162 p2 = __floats2bfloat162_rn(f0, f1);
+                        pk[e] = *reinterpret_cast<const uint32_t*>(&p2);
+                    }
+                    if (live && sy * R + r < a.H) store_pixel16(orow + r * rpitch + j * 16, pk, full);
+                };
+                const uint32_t col = acc + (uint32_t)((R - 1) * npad + j * 16);  // row r: npad columns further down each
+                if (a.pool) {
+                    for (int r = 2 * u0; r < R; r += 2 * ustep) {
+                        uint32_t v0[16], v1[16], p0[8], p1[8];
+                        tmem_ld16_issue(col - (uint32_t)(r * npad), v0);
+                        tmem_ld16_issue(col - (uint32_t)((r + 1) * npad), v1);
+                        tmem_ld_wait(v0);
+                        tmem_ld_wait(v1);
+                        finish(v0, r, p0);
+                        finish(v1, r + 1, p1);
                         const int y = sy * R + r;
 #pragma unroll
                         for (int e = 0; e < 8; ++e) {
@@ -585,17 +609,24 @@ k_conv3x3_tma(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__
                             m = __hmax2(m, *reinterpret_cast<const __nv_bfloat162*>(&o));
                             p0[e] = *reinterpret_cast<uint32_t*>(&m);
                         }
-                        if (y < a.H && x < a.W && !(lane & 1) && j * 16 < a.cout)
+                        if (live && y < a.H && !(lane & 1))
                             store_pixel16(a.pool + (((size_t)n * (a.H / 2) + y / 2) * (a.W / 2) + x / 2) * a.out_cs + j * 16,
-                                          p0, j * 16 + 16 <= a.cout);
+                                          p0, full);
                     }
-            } else {
-                for (int r = 0; r < R; ++r)
-                    for (int j = 0; j < J; ++j) {
-                        if (((r * J + j) & 1) != sub) continue;
-                        uint32_t pk[8];
-                        item(r, j, pk);
+                } else {
+                    for (int r = u0; r < R; r += 2 * ustep) {  // two rows' loads in flight
+                        const int r1 = r + ustep;
+                        uint32_t v0[16], v1[16], pk[8];
+                        tmem_ld16_issue(col - (uint32_t)(r * npad), v0);
+                        if (r1 < R) tmem_ld16_issue(col - (uint32_t)(r1 * npad), v1);
+                        tmem_ld_wait(v0);
+                        finish(v0, r, pk);
+                        if (r1 < R) {
+                            tmem_ld_wait(v1);
+                            finish(v1, r1, pk);
+                        }
                     }
+                }
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
@@ -607,7 +638,8 @@ k_conv3x3_tma(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__
         constexpr int kCoarseW = kStrip / 2 + 2;
         const int ct = tid - kTmaThreads;
         const int Hc = a.H >> 1, Wc = a.W >> 1;
-        int k = 0;
+        int s = 0;
+        uint32_t ph = 0;
         for (int t = blockIdx.x; t < a.tiles; t += gridDim.x) {
             int tt = t;
             const int sx = tt % strips_x;
@@ -616,47 +648,50 @@ k_conv3x3_tma(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__
             const int n = tt / strips_y;
             const int x0 = sx * kStrip, y0 = sy * R;
             const int cy0 = (y0 - 1) >> 1, cx0 = (x0 - 1) >> 1, ncy = ((y0 + R) >> 1) - cy0 + 1;
+            // this strip's coarse pixels (-1: outside the image) and the places of their copies (-1: none)
+            int from[kJobs], to[kJobs][4];
+#pragma unroll
+            for (int u = 0; u < kJobs; ++u) {
+                const int i = ct + u * 32 * kTmaCoarseWarps, half = i & 1, p = i >> 1, ry = p / kCoarseW, rx = p % kCoarseW;
+                const int cy = cy0 + ry, cx = cx0 + rx;
+                from[u] = ry < ncy && cy >= 0 && cy < Hc && cx >= 0 && cx < Wc ? (cy * Wc + cx) * a.coarse_cs + half * 8 : -1;
+                const int hy0 = 2 * cy - (y0 - 1), hx0 = 2 * cx - (x0 - 1);
+#pragma unroll
+                for (int d = 0; d < 4; ++d) {
+                    // pairs of pixels swap their left and right copies, so that a warp's 512 bytes cover all banks
+                    const int hy = hy0 + (d >> 1), hx = hx0 + ((d ^ (p >> 1)) & 1), px = hy * kHaloW + hx;
+                    const bool in = ry < ncy && hy >= 0 && hy < R + 2 && hx >= 0 && hx < kHaloW;
+                    to[u][d] = in ? px * 32 + ((half ^ ((px >> 2) & 1)) << 4) : -1;
+                }
+            }
+            const bf16* img = a.coarse + (size_t)n * Hc * Wc * a.coarse_cs;
             bool ok = true;
-            for (int c = 0; c < nchunks; ++c, ++k) {
-                const int s = k % S;
-                if (c >= ncoarse) {  // filled by TMA; waited for here too (see warp 0)
-                    if (!warp_wait(saddr(hd.empty + s), ((uint32_t)(k / S) & 1u) ^ 1u, abort_flag, a.status)) { ok = false; break; }
-                    continue;
-                }
+            for (int c = 0; c < nchunks; ++c) {
+                const bool mine = c < ncoarse;  // the others are filled by TMA; waited for here too (see warp 0)
                 uint4 v[kJobs];
+                if (mine) {
 #pragma unroll
-                for (int u = 0; u < kJobs; ++u) {
-                    const int i = ct + u * 32 * kTmaCoarseWarps, half = i & 1, p = i >> 1;
-                    const int cy = cy0 + p / kCoarseW, cx = cx0 + p % kCoarseW;
-                    v[u] = make_uint4(0, 0, 0, 0);
-                    if (p < ncy * kCoarseW && cy >= 0 && cy < Hc && cx >= 0 && cx < Wc)
-                        v[u] = __ldg(reinterpret_cast<const uint4*>(a.coarse + (((size_t)n * Hc + cy) * Wc + cx) * a.coarse_cs +
-                                                                    c * 16 + half * 8));
+                    for (int u = 0; u < kJobs; ++u)
+                        v[u] = from[u] >= 0 ? __ldg(reinterpret_cast<const uint4*>(img + from[u] + c * 16)) : make_uint4(0, 0, 0, 0);
                 }
-                if (!warp_wait(saddr(hd.empty + s), ((uint32_t)(k / S) & 1u) ^ 1u, abort_flag, a.status)) { ok = false; break; }
-                const uint32_t bar = saddr(hd.full + s);
-                unsigned char* dst = ring + s * sbytes;
-                if (!a.resident && ct == 0) {
-                    asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" :: "r"(bar), "r"(wchunk) : "memory");
-                    load_weights(saddr(dst + hbytes), c, bar);
-                }
-#pragma unroll
-                for (int u = 0; u < kJobs; ++u) {
-                    const int i = ct + u * 32 * kTmaCoarseWarps, half = i & 1, p = i >> 1;
-                    if (p >= ncy * kCoarseW) continue;
-                    const int hy0 = 2 * (cy0 + p / kCoarseW) - (y0 - 1), hx0 = 2 * (cx0 + p % kCoarseW) - (x0 - 1);
-#pragma unroll
-                    for (int d = 0; d < 4; ++d) {
-                        // pairs of pixels swap their left and right copies, so that a warp's 512 bytes cover all banks
-                        const int hy = hy0 + (d >> 1), hx = hx0 + ((d ^ (p >> 1)) & 1);
-                        if (hy < 0 || hy >= R + 2 || hx < 0 || hx >= kHaloW) continue;
-                        const int px = hy * kHaloW + hx;
-                        *reinterpret_cast<uint4*>(dst + px * 32 + ((half ^ ((px >> 2) & 1)) << 4)) = v[u];
+                if (!warp_wait(saddr(hd.empty + s), ph ^ 1u, abort_flag, a.status)) { ok = false; break; }
+                if (mine) {
+                    const uint32_t bar = saddr(hd.full + s);
+                    unsigned char* dst = ring + s * sbytes;
+                    if (!a.resident && ct == 0) {
+                        asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" :: "r"(bar), "r"(wchunk) : "memory");
+                        load_weights(saddr(dst + hbytes), c, bar);
                     }
+#pragma unroll
+                    for (int u = 0; u < kJobs; ++u)
+#pragma unroll
+                        for (int d = 0; d < 4; ++d)
+                            if (to[u][d] >= 0) *reinterpret_cast<uint4*>(dst + to[u][d]) = v[u];
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // these stores -> tensor core reads
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar);
                 }
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // these stores -> tensor core reads
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar);
+                if (++s == S) { s = 0; ph ^= 1u; }
             }
             if (!ok) break;
         }
