@@ -263,3 +263,38 @@ def test_build_at_size_limits(ctx, oracle, kind, n, bins, max_leaf):
     np.testing.assert_array_equal(res.ids, oid)
     np.testing.assert_array_equal(res.t[oid >= 0], ot[oid >= 0])
     s.close()
+
+
+# The queueing walk (postpone 1) against the walk in which lanes test their own triangles
+# (postpone 2), bit for bit: ray counts around a warp, its least share of rays and its refill
+# size; leaf-heavy and empty regions; the rays' own limits.
+@pytest.mark.parametrize("n", [1, 5, 6, 31, 33, 700, 40000])
+@pytest.mark.parametrize("watertight", [False, True])
+def test_queueing_walk_matches_own_tests(ctx, n, watertight):
+    import salty_gb300
+    tris = salty_gb300.microbench_soup(17, 40000)
+    tris[:500] = tris[0]                      # equal distances
+    sc = _scene(ctx, tris)
+    assert sc.info["depth"] > 3
+    rays = salty_gb300.microbench_rays(n, n, 1e-4)
+    rays[::3, 7] = 2.0                        # tmax among the hits
+    rays[1::5, 3] = 1.9                       # tmin too
+    if n > 30:
+        rays[7, 7] = -1.0                     # nothing can be hit
+        rays[8, 7] = np.nan                   # bounds nothing
+        rays[9, 3] = -5.0                     # taken as 0
+        rays[10, 4:7] = (0.0, 0.0, 1.0)
+    base = ctx.tuning
+    try:
+        got, occ = {}, {}
+        for post in (1, 2):
+            ctx.tuning = {"trace_postpone": post}
+            got[post] = sc.trace(rays, watertight=watertight)
+            occ[post] = sc.trace(rays, any_hit=True, watertight=watertight).ids >= 0
+    finally:
+        ctx.tuning = base
+    for f in ("ids", "t", "u", "v"):
+        np.testing.assert_array_equal(getattr(got[1], f), getattr(got[2], f))
+    np.testing.assert_array_equal(occ[1], got[1].ids >= 0)
+    np.testing.assert_array_equal(occ[1], occ[2])
+    sc.close()
