@@ -444,23 +444,30 @@ salty_status salty_trace(salty_ctx* ctx, salty_scene* sc, const salty_ray* rays,
     const bool din = is_device_ptr(rays) && ((uintptr_t)rays % 16 == 0);
     const bool dout = is_device_ptr(hits) && ((uintptr_t)hits % 16 == 0);
     cudaStream_t st = ctx->stream;
-    SALTY_TRY_CUDA(E, cudaMemsetAsync(ctx->status.p, 0, sizeof(int), st));
-    cudaEvent_t t0 = ctx->ev[2], k0 = ctx->ev[3], k1 = ctx->ev[4], t1 = ctx->ev[5];
-    SALTY_TRY_CUDA(E, cudaEventRecord(t0, st));
+    cudaEvent_t t0 = ctx->ev[2], k1 = ctx->ev[4], t1 = ctx->ev[5];
     unsigned long long counts[3] = {0, 0, 0};
     double kernel_ms = 0.0;
+    int status = 0;
+    // The control block of a slot: cursor, node and triangle counts, then the status word; one
+    // memset before and one copy into pinned memory after the launches.
+    constexpr int kCtl = 4;
+    unsigned long long* ctl = ctx->counters.p;
+    auto* ctl_host = static_cast<unsigned long long*>(ctx->pinned);
+    auto status_of = [&](int s) { return reinterpret_cast<int*>(ctl + kCtl * s + 3); };
+    SALTY_TRY_CUDA(E, cudaEventRecord(t0, st));
+    SALTY_TRY_CUDA(E, cudaMemsetAsync(ctl, 0, 2 * kCtl * sizeof(unsigned long long), st));
     if (din && dout) {
-        SALTY_TRY_CUDA(E, cudaEventRecord(k0, st));
-        SALTY_TRY(trace_launch(ctx, sc, (const float4*)rays, n, nullptr, flags, (float4*)hits, ctx->counters.p, st,
-                               ctx->status.p));
+        SALTY_TRY(trace_launch(ctx, sc, (const float4*)rays, n, nullptr, flags, (float4*)hits, ctl, st, status_of(0)));
         stats.launches = 1;
         SALTY_TRY_CUDA(E, cudaEventRecord(k1, st));
-        SALTY_TRY_CUDA(E, cudaMemcpyAsync(counts, ctx->counters.p, sizeof counts, cudaMemcpyDeviceToHost, st));
+        SALTY_TRY_CUDA(E, cudaMemcpyAsync(ctl_host, ctl, kCtl * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
         SALTY_TRY_CUDA(E, cudaEventRecord(t1, st));
         SALTY_TRY_CUDA(E, cudaEventSynchronize(t1));
         float ms = 0;
-        cudaEventElapsedTime(&ms, k0, k1);
+        cudaEventElapsedTime(&ms, t0, k1);
         kernel_ms = ms;
+        for (int k = 0; k < 3; ++k) counts[k] = ctl_host[k];
+        status = (int)ctl_host[3];
     } else {
         // Host arrays: chunks alternate between two device slots so the copies of one
         // chunk overlap the traversal of the other.
@@ -470,7 +477,7 @@ salty_status salty_trace(salty_ctx* ctx, salty_scene* sc, const salty_ray* rays,
         SALTY_TRY_CUDA(E, ctx->ray_buf.ensure((size_t)2 * 2 * slot_rays));
         SALTY_TRY_CUDA(E, ctx->hit_buf.ensure((size_t)2 * slot_rays));
         cudaStream_t ss[2] = {ctx->stream, ctx->copy_stream};
-        cudaEvent_t slot_free[2] = {ctx->ev[6], ctx->ev[7]};
+        cudaEvent_t k0 = ctx->ev[3];
         SALTY_TRY_CUDA(E, cudaEventRecord(k0, st));
         SALTY_TRY_CUDA(E, cudaStreamWaitEvent(ss[1], k0, 0));
         for (long long c = 0; c < nch; ++c) {
@@ -484,34 +491,28 @@ salty_status salty_trace(salty_ctx* ctx, salty_scene* sc, const salty_ray* rays,
                 SALTY_TRY_CUDA(E, cudaMemcpyAsync(rb, rays + b, (size_t)m * sizeof(salty_ray), cudaMemcpyDefault, ss[s]));
                 stats.h2d_bytes += m * (int64_t)sizeof(salty_ray);
             }
-            SALTY_TRY(trace_launch(ctx, sc, rin, m, nullptr, flags, hout, ctx->counters.p + 4 * s, ss[s], ctx->status.p));
+            if (c >= 2)  // rewind the slot's cursor; its counts go on
+                SALTY_TRY_CUDA(E, cudaMemsetAsync(ctl + kCtl * s, 0, sizeof(unsigned long long), ss[s]));
+            SALTY_TRY(trace_launch(ctx, sc, rin, m, nullptr, flags, hout, ctl + kCtl * s, ss[s], status_of(s)));
             ++stats.launches;
             if (!dout) {
                 SALTY_TRY_CUDA(E, cudaMemcpyAsync(hits + b, hb, (size_t)m * sizeof(salty_hit), cudaMemcpyDefault, ss[s]));
                 stats.d2h_bytes += m * (int64_t)sizeof(salty_hit);
             }
-            SALTY_TRY_CUDA(E, cudaEventRecord(slot_free[s], ss[s]));
-            (void)slot_free;
-            if (flags & SALTY_TRACE_COUNTERS) {
-                SALTY_TRY_CUDA(E, cudaStreamSynchronize(ss[s]));
-                unsigned long long cc[3];
-                SALTY_TRY_CUDA(E, cudaMemcpy(cc, ctx->counters.p + 4 * s, sizeof cc, cudaMemcpyDeviceToHost));
-                counts[1] += cc[1];
-                counts[2] += cc[2];
-            }
         }
         SALTY_TRY_CUDA(E, cudaEventRecord(ctx->ev[6], ss[1]));
         SALTY_TRY_CUDA(E, cudaStreamWaitEvent(st, ctx->ev[6], 0));
         SALTY_TRY_CUDA(E, cudaEventRecord(k1, st));
+        SALTY_TRY_CUDA(E, cudaMemcpyAsync(ctl_host, ctl, 2 * kCtl * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
         SALTY_TRY_CUDA(E, cudaEventRecord(t1, st));
         SALTY_TRY_CUDA(E, cudaEventSynchronize(t1));
         float ms = 0;
         cudaEventElapsedTime(&ms, k0, k1);
         kernel_ms = ms;
+        for (int k = 1; k < 3; ++k) counts[k] = ctl_host[k] + ctl_host[kCtl + k];
+        status = (int)(ctl_host[3] | ctl_host[kCtl + 3]);
     }
     SALTY_TRY_CUDA(E, cudaGetLastError());
-    int status = 0;
-    SALTY_TRY_CUDA(E, cudaMemcpy(&status, ctx->status.p, sizeof(int), cudaMemcpyDeviceToHost));
     float total = 0;
     cudaEventElapsedTime(&total, t0, t1);
     stats.kernel_ms = kernel_ms;
@@ -637,6 +638,7 @@ salty_status salty_autotune_trace(salty_ctx* ctx, salty_scene* sc, const salty_r
     auto time_of = [&](float* ms) -> salty_status {
         float best = 1e30f;
         for (int r = 0; r < 3; ++r) {
+            SALTY_TRY_CUDA(E, cudaMemsetAsync(ctx->counters.p, 0, 3 * sizeof(unsigned long long), st));
             SALTY_TRY_CUDA(E, cudaEventRecord(ctx->ev[3], st));
             SALTY_TRY(trace_launch(ctx, sc, d_rays, n, nullptr, flags, hits.p, ctx->counters.p, st, ctx->status.p));
             SALTY_TRY_CUDA(E, cudaEventRecord(ctx->ev[4], st));

@@ -281,6 +281,15 @@ struct BatchArena {
 };
 }  // namespace salty
 
+namespace salty {
+// A traversal kernel's resident blocks per SM at one size of dynamic shared memory.
+struct ResidentBlocks {
+    const void* kern;
+    size_t smem;
+    int per_sm;
+};
+}  // namespace salty
+
 struct salty_ctx {
     int device = 0;
     int num_sms = 0;
@@ -303,6 +312,7 @@ struct salty_ctx {
     salty::WaveStore waves;
     salty::BatchArena arena;
     salty::DevBuf<unsigned char> slots;  // SceneSlot table of the current render
+    std::vector<salty::ResidentBlocks> resident;  // a few entries: kernels x stack depths used
     salty::DevBuf<unsigned char> build_ws;  // BVH build workspace (bvh_build.cu)
 };
 

@@ -201,22 +201,24 @@ struct WaveBuffers {
     float4* shits;
     float4* lbuf;      // per wave-local sample: radiance xyz
     float4* abuf;      // per wave-local sample, first hit: 2 x float4 (albedo, 1/(1+t)) (normal, 0)
-    int* counts;       // [0] queue A len, [1] queue B len, [2] shadow len
+    int* counts;       // [0] queue A len, [1] queue B len, [2] shadow len, [3] blocks of k_shade2 done
     long long* ctl;    // the sample stream, see enum Ctl (shared by the halves)
     long long* gen;    // this half's pending generation: first sample, count, first queue slot
+    unsigned long long *tc_ext, *tc_sh;  // this half's traversal cursors
+    int* acc_blocks;   // blocks of k_accumulate done (shared by the halves)
     int* done;         // per ring chunk: its samples whose paths have ended
     unsigned long long* stats;  // [0] rays traced, [1] paths
 };
 
 constexpr long long kMaxRingChunks = 16;  // per-sample buffers: at most 16 chunks of half a queue
 constexpr long long kMinSplit = 1 << 16;  // queues of at least this many paths run as two halves
+constexpr int kDirectDepth = 16;           // longest paths of a render launched without a graph
 constexpr int kLaunchIters = 256;          // iterations per graph launch (cancellation granularity)
 
 // Control words of the regenerating wavefront (ctl[]).
 enum Ctl : int {
     kNext = 0,      // next global sample to start
     kAccBase = 1,   // samples below this are in the films
-    kAccN = 2,      // samples [kAccBase, kAccBase + kAccN) are ready to accumulate
     kIters = 3,     // iterations run
     kLaunchEnd = 4, // this graph launch stops after iteration kLaunchEnd
     kGenA = 5,      // half A's pending generation (3 words, WaveBuffers::gen)
@@ -1081,17 +1083,25 @@ __global__ void __maxnreg__(64) k_shade2(WaveParams P, WaveBuffers B, int q) {
             if (B.roots[q ^ 1]) B.roots[q ^ 1][qi] = root;
         }
     }
+    // the last block closes the half's iteration: counts its rays, empties queue q and the
+    // shadow queue and rewinds the traversal cursors (every thread has read n by then)
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(&B.counts[3], 1) == (int)gridDim.x - 1) {
+            atomicAdd(&B.stats[0], (unsigned long long)n + (unsigned long long)B.counts[2]);
+            B.counts[q] = 0;
+            B.counts[2] = 0;
+            B.counts[3] = 0;
+            B.tc_ext[0] = 0;
+            B.tc_sh[0] = 0;
+        }
+    }
 }
 
-// After the shading of queue q in both halves: counts their rays, empties those queues and
-// the shadow queues, and finds the samples ready for the films -- the longest run of whole
-// chunks, from the first sample not yet accumulated, whose paths have all ended.
-__global__ void k_iter_end(WaveParams P, WaveBuffers A, WaveBuffers B, int q) {
-    A.stats[0] += (unsigned long long)(A.counts[q] + A.counts[2] + B.counts[q] + B.counts[2]);
-    A.counts[q] = 0;
-    A.counts[2] = 0;
-    B.counts[q] = 0;
-    B.counts[2] = 0;
+// The samples ready for the films: the longest run of whole chunks, from the first sample not
+// yet accumulated, whose paths have all ended.
+__device__ long long ready_samples(const WaveParams& P, const WaveBuffers& A) {
     const long long base = A.ctl[kAccBase];
     long long n = 0;
     for (int k = 0; k < P.ring_chunks; ++k) {
@@ -1101,7 +1111,7 @@ __global__ void k_iter_end(WaveParams P, WaveBuffers A, WaveBuffers B, int q) {
         if (A.done[(c0 / P.chunk) % P.ring_chunks] != (int)size) break;
         n += size;
     }
-    A.ctl[kAccN] = n;
+    return n;
 }
 
 // New samples for the halves' queues q: up to the free slots of half A, then of half B, as
@@ -1125,15 +1135,13 @@ __device__ void plan_generation(const WaveParams& P, WaveBuffers& A, WaveBuffers
     A.stats[1] += (unsigned long long)(add_a + add_b);
 }
 
-// After the accumulation: frees the accumulated chunks, plans the next generation (queues
+// After the accumulation of n samples: frees their chunks, plans the next generation (queues
 // q ^ 1) and decides whether the graph launch runs another iteration.
-__global__ void k_iter_next(WaveParams P, WaveBuffers A, WaveBuffers B, int q, cudaGraphConditionalHandle more,
-                            int last) {
+__device__ void iteration_done(const WaveParams& P, WaveBuffers& A, WaveBuffers& B, long long n, int q,
+                               cudaGraphConditionalHandle more, int last) {
     long long* c = A.ctl;
-    const long long n = c[kAccN];
     for (long long g = c[kAccBase]; g < c[kAccBase] + n; g += P.chunk) A.done[(g / P.chunk) % P.ring_chunks] = 0;
     c[kAccBase] += n;
-    c[kAccN] = 0;
     plan_generation(P, A, B, q ^ 1);
     c[kIters] += 1;
     if (c[kIters] > P.iter_limit) c[kStuck] = 1;
@@ -1147,10 +1155,12 @@ __global__ void k_iter_next(WaveParams P, WaveBuffers A, WaveBuffers B, int q, c
 __global__ void k_render_init(WaveParams P, WaveBuffers A, WaveBuffers B) {
     for (int k = 0; k < kCtlWords; ++k) A.ctl[k] = 0;
     for (int k = 0; k < P.ring_chunks; ++k) A.done[k] = 0;
-    for (int k = 0; k < 3; ++k) {
+    for (int k = 0; k < 4; ++k) {
         A.counts[k] = 0;
         B.counts[k] = 0;
     }
+    A.tc_ext[0] = A.tc_sh[0] = B.tc_ext[0] = B.tc_sh[0] = 0;
+    *A.acc_blocks = 0;
     A.stats[0] = 0;
     A.stats[1] = 0;
     plan_generation(P, A, B, 0);
@@ -1159,11 +1169,10 @@ __global__ void k_render_init(WaveParams P, WaveBuffers A, WaveBuffers B) {
 // Start of a graph launch: run at most launch_iters iterations.
 __global__ void k_launch_begin(WaveParams P, WaveBuffers B) { B.ctl[kLaunchEnd] = B.ctl[kIters] + P.launch_iters; }
 
-// Adds the wave's samples to the films: one thread per film pixel of the slots the wave
-// touches, that pixel's samples in index order.
-__global__ void k_accumulate(WaveParams P, WaveBuffers B) {
+// Adds the ready samples to the films: one thread per film pixel of the slots they touch, that
+// pixel's samples in index order.
+__device__ void accumulate(const WaveParams& P, const WaveBuffers& B, const long long n) {
     const long long g0 = B.ctl[kAccBase];
-    const long long n = B.ctl[kAccN];
     if (n <= 0) return;
     const int s0 = P.n_slots == 1 ? 0 : find_slot(P.sample_off, 0, P.n_slots - 1, g0);
     const int s1 = P.n_slots == 1 ? 0 : find_slot(P.sample_off, s0, P.n_slots - 1, g0 + n - 1);
@@ -1225,6 +1234,24 @@ __global__ void k_accumulate(WaveParams P, WaveBuffers B) {
     }
 }
 
+// End of an iteration: accumulates the samples that are ready; the last block plans the next
+// iteration.  (One kernel instead of three: a small frame's iteration is a chain of launches of
+// a few microseconds each.)
+__global__ void k_accumulate(WaveParams P, WaveBuffers A, WaveBuffers B, int q, cudaGraphConditionalHandle more,
+                             int last) {
+    __shared__ long long ready;
+    if (threadIdx.x == 0) ready = ready_samples(P, A);
+    __syncthreads();
+    accumulate(P, A, ready);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(A.acc_blocks, 1) == (int)gridDim.x - 1) {
+            *A.acc_blocks = 0;
+            iteration_done(P, A, B, ready, q, more, last);
+        }
+    }
+}
 
 // Mean first-hit features of the film: albedo W*H*3, normal W*H*3, 1/(1+t) W*H.
 __global__ void k_aov_out(const float* __restrict__ aov, long long npx, double count, float* albedo, float* normal,
@@ -1663,7 +1690,7 @@ salty_status render_batch(salty_ctx* ctx, salty_scene* const* scenes, const salt
 
     // the halves' views of the queues: half B starts cap_a paths in (2 rays and 2 shadow
     // rays per path), with its own queue lengths and generation plan
-    auto half = [&](long long off, int counts_off, int gen_word) {
+    auto half = [&](long long off, int counts_off, int gen_word, unsigned long long* tc_ext, unsigned long long* tc_sh) {
         WaveBuffers h;
         for (int i = 0; i < 2; ++i) {
             h.rays[i] = S.rays[i].p + 2 * off;
@@ -1682,9 +1709,12 @@ salty_status render_batch(salty_ctx* ctx, salty_scene* const* scenes, const salt
         h.gen = S.ctl.p + gen_word;
         h.done = S.done.p;
         h.stats = S.stats.p;
+        h.tc_ext = tc_ext;
+        h.tc_sh = tc_sh;
+        h.acc_blocks = S.counts.p + 15;
         return h;
     };
-    WaveBuffers BA = half(0, 0, kGenA), BB = half(P.cap_a, 8, kGenB);
+    WaveBuffers BA = half(0, 0, kGenA, S.tc0.p, S.tc1.p), BB = half(P.cap_a, 8, kGenB, S.tc2.p, S.tc3.p);
 
     const bool compat = opts[0].profile == SALTY_PROFILE_COMPAT;
     const uint32_t ext_flags = compat ? 0u : (uint32_t)SALTY_TRACE_WATERTIGHT;
@@ -1710,41 +1740,59 @@ salty_status render_batch(salty_ctx* ctx, salty_scene* const* scenes, const salt
     const bool host_loop = hl && std::atoi(hl) != 0;
     cudaGraphConditionalHandle more = 0;
     // one half's shading and traversal for queue q, on stream hs
-    auto run_half = [&](const WaveBuffers& H, long long hcap, unsigned long long* tc_ext, unsigned long long* tc_sh,
-                        cudaStream_t hs, int q) -> salty_status {
+    auto run_half = [&](const WaveBuffers& H, long long hcap, cudaStream_t hs, int q, bool generate) -> salty_status {
         const int hgrid = grid_of(hcap, 2048 / sb, ctx->num_sms, sb);
         TraceTarget ext = tgt, shd = tgt;
         ext.roots = H.roots[q];
         shd.roots = H.sroots;
-        k_generate<<<hgrid, sb, 0, hs>>>(P, H, q);
-        SALTY_TRY(trace_launch(ctx, ext, T.trace, H.rays[q], hcap, &H.counts[q], ext_flags, H.hits, tc_ext, hs,
+        if (generate) k_generate<<<hgrid, sb, 0, hs>>>(P, H, q);
+        SALTY_TRY(trace_launch(ctx, ext, T.trace, H.rays[q], hcap, &H.counts[q], ext_flags, H.hits, H.tc_ext, hs,
                                ctx->status.p));
         k_shade1<<<hgrid, sb, 0, hs>>>(P, H, q);
-        SALTY_TRY(trace_launch(ctx, shd, T.trace, H.srays, 2 * hcap, &H.counts[2], sh_flags, H.shits, tc_sh, hs,
+        SALTY_TRY(trace_launch(ctx, shd, T.trace, H.srays, 2 * hcap, &H.counts[2], sh_flags, H.shits, H.tc_sh, hs,
                                ctx->status.p));
         k_shade2<<<hgrid, sb, 0, hs>>>(P, H, q);
         return SALTY_OK;
     };
     const bool split = P.cap_b > 0;
+    // half B's stream, forked from st and joined back into it
+    auto fork = [&]() -> salty_status {
+        SALTY_TRY_CUDA(E, cudaEventRecord(ctx->fork_ev, st));
+        SALTY_TRY_CUDA(E, cudaStreamWaitEvent(ctx->aux_stream, ctx->fork_ev, 0));
+        return SALTY_OK;
+    };
+    auto join = [&]() -> salty_status {
+        SALTY_TRY_CUDA(E, cudaEventRecord(ctx->join_ev, ctx->aux_stream));
+        SALTY_TRY_CUDA(E, cudaStreamWaitEvent(st, ctx->join_ev, 0));
+        return SALTY_OK;
+    };
     auto iteration_pair = [&](bool in_graph) -> salty_status {
         for (int q = 0; q < 2; ++q) {
-            // half B on the auxiliary stream, forked from and joined back into st (in the
-            // host loop both halves run on st, one after the other)
-            const cudaStream_t sb_stream = in_graph && split ? ctx->aux_stream : st;
-            if (in_graph && split) {
-                SALTY_TRY_CUDA(E, cudaEventRecord(ctx->fork_ev, st));
-                SALTY_TRY_CUDA(E, cudaStreamWaitEvent(sb_stream, ctx->fork_ev, 0));
-            }
-            SALTY_TRY(run_half(BA, P.cap_a, S.tc0.p, S.tc1.p, st, q));
-            if (split) SALTY_TRY(run_half(BB, P.cap_b, S.tc2.p, S.tc3.p, sb_stream, q));
-            if (in_graph && split) {
-                SALTY_TRY_CUDA(E, cudaEventRecord(ctx->join_ev, sb_stream));
-                SALTY_TRY_CUDA(E, cudaStreamWaitEvent(st, ctx->join_ev, 0));
-            }
-            k_iter_end<<<1, 1, 0, st>>>(P, BA, BB, q);
-            k_accumulate<<<agrid, 256, 0, st>>>(P, BA);
-            k_iter_next<<<1, 1, 0, st>>>(P, BA, BB, q, more, in_graph && q == 1 ? 1 : 0);
+            // half B on the auxiliary stream (in the host loop both halves run on st, one after
+            // the other)
+            const bool both = in_graph && split;
+            if (both) SALTY_TRY(fork());
+            SALTY_TRY(run_half(BA, P.cap_a, st, q, true));
+            if (split) SALTY_TRY(run_half(BB, P.cap_b, both ? ctx->aux_stream : st, q, true));
+            if (both) SALTY_TRY(join());
+            k_accumulate<<<agrid, 256, 0, st>>>(P, BA, BB, q, more, in_graph && q == 1 ? 1 : 0);
         }
+        return SALTY_OK;
+    };
+    // A render whose samples all start at once (one generation) and whose paths are short ends
+    // after max_depth iterations and a single accumulation, so its launches go straight into
+    // the streams: nothing to instantiate, no generation or control launch per iteration, and
+    // the halves meet only at the end.  (256 x 256 Cornell box at 16 spp: 1.67 -> 1.40 ms; a 16 x 16
+    // frame at depth 8: 0.61 -> 0.29 ms.)  Longer paths keep the graph, which stops once all paths have ended.
+    const bool direct = !host_loop && samples <= cap && ring >= samples && max_depth <= kDirectDepth;
+    auto run_direct = [&]() -> salty_status {
+        if (split) SALTY_TRY(fork());
+        for (int it = 0; it < max_depth; ++it) {
+            SALTY_TRY(run_half(BA, P.cap_a, st, it & 1, it == 0));
+            if (split) SALTY_TRY(run_half(BB, P.cap_b, ctx->aux_stream, it & 1, it == 0));
+        }
+        if (split) SALTY_TRY(join());
+        k_accumulate<<<agrid, 256, 0, st>>>(P, BA, BB, (max_depth - 1) & 1, more, 0);
         return SALTY_OK;
     };
     cudaGraph_t graph = nullptr;
@@ -1757,7 +1805,7 @@ salty_status render_batch(salty_ctx* ctx, salty_scene* const* scenes, const salt
             if (g) cudaGraphDestroy(g);
         }
     } guard{graph, exec};
-    if (!host_loop) {
+    if (!host_loop && !direct) {
         SALTY_TRY_CUDA(E, cudaGraphCreate(&graph, 0));
         SALTY_TRY_CUDA(E, cudaGraphConditionalHandleCreate(&more, graph, 1, cudaGraphCondAssignDefault));
         cudaGraphNode_t begin_node, loop_node;
@@ -1796,7 +1844,10 @@ salty_status render_batch(salty_ctx* ctx, salty_scene* const* scenes, const salt
     const long long max_launches = P.iter_limit / (host_loop ? 2 * pairs_per_step : kLaunchIters) + 2;
     for (long long launch = 0;; ++launch) {
         if (launch > max_launches) { rs = E.fail(SALTY_ERR_TIMEOUT, "render made no progress"); break; }
-        if (host_loop) {
+        if (direct) {
+            rs = launch == 0 ? run_direct() : E.fail(SALTY_ERR_TIMEOUT, "render left samples behind");
+            if (rs != SALTY_OK) break;
+        } else if (host_loop) {
             k_launch_begin<<<1, 1, 0, st>>>(P, BA);
             for (int k = 0; k < pairs_per_step && rs == SALTY_OK; ++k) rs = iteration_pair(false);
             if (rs != SALTY_OK) break;

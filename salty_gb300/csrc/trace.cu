@@ -25,6 +25,11 @@ constexpr int kMaxStack = 63;  // stack entries per thread: BVHs up to 31 levels
 // ones); longer arrays are traced in consecutive launches of at most this many rays.
 constexpr long long kMaxLaunchRays = 1ll << 30;
 
+// A launch with fewer rays than lanes spreads them: a warp takes no more than its share of the
+// rays, but at least kMinPool (30k triangles, 4,096 rays: 173 us per call at 64 rays per warp,
+// 159 at 1, 134 at 16).
+constexpr int kMinPool = 16;
+
 // k_trace: lanes test their own triangles -- two-level scenes, spheres, counting walks,
 // postponing and shallow trees; k_trace_queue below walks the rest.
 // counters: [0] ray cursor, [1] node fetches, [2] triangle fetches.  The register budget
@@ -51,6 +56,8 @@ k_trace(const Bvh8Node* __restrict__ nodes, const float4* __restrict__ tris, con
     // queue length from device memory when given (wavefront queues), else the argument
     // (at most kMaxLaunchRays either way)
     const int n = n_dev ? *n_dev : (int)n_arg;
+    const int warps = (int)gridDim.x * (TB / 32);
+    pool = min(pool, max(kMinPool, (n + warps - 1) / warps));
     TravCount cnt{0, 0};
     int overflow = 0;
     // Warp-uniform pool of ray indices [pool_next, pool_end), refilled `pool` at a time
@@ -194,10 +201,6 @@ k_trace(const Bvh8Node* __restrict__ nodes, const float4* __restrict__ tris, con
 // reference's test 3.14 -> 3.00 ms.
 constexpr int kQueue = 64;    // pairs per warp: fewer than 32 before a push of at most 32
 constexpr int kRefill = 6;    // idle lanes that start a refill
-// A launch with fewer rays than lanes spreads them: a warp takes no more than its share of the
-// rays, but at least kMinPool (30k triangles, 4,096 rays: 173 us per call at 64 rays per warp,
-// 159 at 1, 134 at 16).
-constexpr int kMinPool = 16;
 
 template <bool ANY, bool WT, int TB, bool CAP>
 __global__ void __launch_bounds__(TB, (CAP ? 896 : 1024) / TB)
@@ -346,6 +349,20 @@ struct Launch {
     int* status;
 };
 
+// Resident blocks per SM of a kernel at a block size and shared memory, asked for once per
+// context (the query costs as much as a launch).
+salty_status resident_blocks(salty_ctx* ctx, const void* kern, int block, size_t smem, int* per_sm) {
+    for (const auto& r : ctx->resident)
+        if (r.kern == kern && r.smem == smem) {
+            *per_sm = r.per_sm;
+            return SALTY_OK;
+        }
+    SALTY_TRY_CUDA(ctx->err, cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kern, block, smem));
+    if (*per_sm < 1) *per_sm = 1;
+    ctx->resident.push_back({kern, smem, *per_sm});
+    return SALTY_OK;
+}
+
 template <bool ANY, bool WT, bool COUNT, int TB, bool CAP, bool INST, bool SPH = false>
 salty_status launch(salty_ctx* ctx, const Launch& L) {
     auto kern = k_trace<ANY, WT, COUNT, TB, CAP, INST, SPH>;
@@ -353,8 +370,7 @@ salty_status launch(salty_ctx* ctx, const Launch& L) {
     if (smem > 48 * 1024)
         SALTY_TRY_CUDA(ctx->err, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
-    SALTY_TRY_CUDA(ctx->err, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, TB, smem));
-    if (per_sm < 1) per_sm = 1;
+    SALTY_TRY(resident_blocks(ctx, reinterpret_cast<const void*>(kern), TB, smem, &per_sm));
     if (L.n_dev && L.n > kMaxLaunchRays)
         return ctx->err.fail(SALTY_ERR_CAPACITY, "ray queue capacity %lld exceeds %lld", L.n, kMaxLaunchRays);
     // consecutive launches of at most kMaxLaunchRays rays; each restarts the ray cursor
@@ -381,8 +397,7 @@ salty_status launch_queue(salty_ctx* ctx, const Launch& L) {
     if (smem > 48 * 1024)
         SALTY_TRY_CUDA(ctx->err, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
-    SALTY_TRY_CUDA(ctx->err, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, TB, smem));
-    if (per_sm < 1) per_sm = 1;
+    SALTY_TRY(resident_blocks(ctx, reinterpret_cast<const void*>(kern), TB, smem, &per_sm));
     if (L.n_dev && L.n > kMaxLaunchRays)
         return ctx->err.fail(SALTY_ERR_CAPACITY, "ray queue capacity %lld exceeds %lld", L.n, kMaxLaunchRays);
     for (long long off = 0; off == 0 || off < L.n; off += kMaxLaunchRays) {
@@ -458,11 +473,11 @@ salty_status dispatch_count(salty_ctx* ctx, const Launch& L, uint32_t flags) {
 }  // namespace
 
 // Traces rays already resident on the device: n of them, or *n_dev when n_dev is given
-// (then n is the capacity used to size the grid).  counters (3 x u64) are zeroed here.
+// (then n is the capacity used to size the grid).  counters (3 x u64) are zero on entry; the
+// caller rewinds them.
 salty_status trace_launch(salty_ctx* ctx, const TraceTarget& tgt, const TraceTuning& tune, const float4* d_rays,
                           long long n, const int* n_dev, uint32_t flags, float4* d_hits,
                           unsigned long long* d_counters, cudaStream_t st, int* d_status) {
-    SALTY_TRY_CUDA(ctx->err, cudaMemsetAsync(d_counters, 0, 3 * sizeof(unsigned long long), st));
     const bool wt = flags & SALTY_TRACE_WATERTIGHT;
     // Without postponing, the walk keeps at most one pending node group per BVH level
     // (it pushes the rest of a group before descending into one of its children, and puts
