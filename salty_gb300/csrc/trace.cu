@@ -31,7 +31,7 @@ constexpr long long kMaxLaunchRays = 1ll << 30;
 constexpr int kMinPool = 16;
 
 // k_trace: lanes test their own triangles -- two-level scenes, spheres, counting walks,
-// postponing and shallow trees; k_trace_queue below walks the rest.
+// postponing, shallow trees and few rays; k_trace_queue below walks the rest.
 // counters: [0] ray cursor, [1] node fetches, [2] triangle fetches.  The register budget
 // is set through the resident blocks asked for: 1024 / TB caps registers at 64 per thread,
 // CAP's 1152 / TB at 56 for blocks of up to 128 threads (36 instead of 32 warps per SM to
@@ -56,8 +56,6 @@ k_trace(const Bvh8Node* __restrict__ nodes, const float4* __restrict__ tris, con
     // queue length from device memory when given (wavefront queues), else the argument
     // (at most kMaxLaunchRays either way)
     const int n = n_dev ? *n_dev : (int)n_arg;
-    const int warps = (int)gridDim.x * (TB / 32);
-    pool = min(pool, max(kMinPool, (n + warps - 1) / warps));
     TravCount cnt{0, 0};
     int overflow = 0;
     // Warp-uniform pool of ray indices [pool_next, pool_end), refilled `pool` at a time
@@ -76,10 +74,15 @@ k_trace(const Bvh8Node* __restrict__ nodes, const float4* __restrict__ tris, con
         const unsigned idle_mask = __ballot_sync(0xffffffffu, idle);
         if (idle_mask) {
             if (pool_next >= pool_end && !drained) {
+                int take = pool;
+                if (n_dev) {  // the host has done this for launches whose size it knows
+                    const int warps = (int)gridDim.x * (TB / 32);
+                    take = min(take, max(kMinPool, (n + warps - 1) / warps));
+                }
                 unsigned long long base = 0;
-                if (lane == 0) base = atomicAdd(&counters[0], (unsigned long long)pool);
+                if (lane == 0) base = atomicAdd(&counters[0], (unsigned long long)take);
                 base = __shfl_sync(0xffffffffu, base, 0);
-                const long long end = (long long)base + pool;
+                const long long end = (long long)base + take;
                 pool_next = (int)min((long long)base, (long long)n);
                 pool_end = (int)min(end, (long long)n);
                 if (end >= n) drained = true;
@@ -198,7 +201,7 @@ k_trace(const Bvh8Node* __restrict__ nodes, const float4* __restrict__ tris, con
 // (7 blocks of 128 per SM; 56, 64 and 80 registers: 9, 3 and 3 % slower).  Measured (GB300):
 // 1080p terrain at 8 spp 27.4 -> 23.1 ms, 12 uneven scenes 20.3 -> 18.9 ms, 2.5M watertight
 // rays of the 1M-triangle soup from host arrays 2.81 -> 2.51 ms, 4.2M rays with the
-// reference's test 3.14 -> 3.00 ms.
+// reference's test 3.14 -> 2.96 ms.  Where it gains nothing: dispatch_flags.
 constexpr int kQueue = 64;    // pairs per warp: fewer than 32 before a push of at most 32
 constexpr int kRefill = 6;    // idle lanes that start a refill
 
@@ -215,8 +218,6 @@ k_trace_queue(const Bvh8Node* __restrict__ nodes, const float4* __restrict__ tri
     uint2* queue = sstack + (depth + 2) * TB + (threadIdx.x >> 5) * kQueue;  // (triangle, lane)
     uint2* uvs = sstack + depth * TB + (threadIdx.x & ~31);
     const int n = n_dev ? *n_dev : (int)n_arg;
-    const int warps = (int)gridDim.x * (TB / 32);
-    pool = min(pool, max(kMinPool, (n + warps - 1) / warps));
     TravCount cnt{0, 0};
     int overflow = 0;
     int pool_next = 0, pool_end = 0;
@@ -236,10 +237,15 @@ k_trace_queue(const Bvh8Node* __restrict__ nodes, const float4* __restrict__ tri
                 if (drained) {
                     if (idle_mask == 0xffffffffu) break;
                 } else {
+                    int take = pool;
+                    if (n_dev) {
+                        const int warps = (int)gridDim.x * (TB / 32);
+                        take = min(take, max(kMinPool, (n + warps - 1) / warps));
+                    }
                     unsigned long long base = 0;
-                    if (lane == 0) base = atomicAdd(&counters[0], (unsigned long long)pool);
+                    if (lane == 0) base = atomicAdd(&counters[0], (unsigned long long)take);
                     base = __shfl_sync(0xffffffffu, base, 0);
-                    const long long end = (long long)base + pool;
+                    const long long end = (long long)base + take;
                     pool_next = (int)min((long long)base, (long long)n);
                     pool_end = (int)min(end, (long long)n);
                     if (end >= n) drained = true;
@@ -349,6 +355,13 @@ struct Launch {
     int* status;
 };
 
+// Rays a warp takes at a time: few rays are spread over the launch's warps (the kernels do the
+// same for a size in device memory).
+int spread(const Launch& L, long long warps, long long n) {
+    if (L.n_dev) return L.pool;
+    return (int)std::min<long long>(L.pool, std::max<long long>(kMinPool, (n + warps - 1) / warps));
+}
+
 // Resident blocks per SM of a kernel at a block size and shared memory, asked for once per
 // context (the query costs as much as a launch).
 salty_status resident_blocks(salty_ctx* ctx, const void* kern, int block, size_t smem, int* per_sm) {
@@ -383,7 +396,7 @@ salty_status launch(salty_ctx* ctx, const Launch& L) {
         if (grid < 1) grid = 1;
         kern<<<(unsigned)grid, TB, smem, L.st>>>(L.tgt.nodes, L.tgt.tris, L.rays + 2 * off,
                                                  L.tgt.roots ? L.tgt.roots + off : nullptr, n, L.n_dev,
-                                                 L.hits + off, L.counters, L.slack, L.pool, L.postpone, L.depth,
+                                                 L.hits + off, L.counters, L.slack, spread(L, grid * (TB / 32), n), L.postpone, L.depth,
                                                  L.status, L.tgt.inst, L.tgt.sph_base);
         SALTY_TRY_CUDA(ctx->err, cudaGetLastError());
     }
@@ -406,7 +419,7 @@ salty_status launch_queue(salty_ctx* ctx, const Launch& L) {
         const long long grid = std::max(1ll, std::min((long long)ctx->num_sms * per_sm, (n + TB / 32 - 1) / (TB / 32)));
         kern<<<(unsigned)grid, TB, smem, L.st>>>(L.tgt.nodes, L.tgt.tris, L.rays + 2 * off,
                                                  L.tgt.roots ? L.tgt.roots + off : nullptr, n, L.n_dev, L.hits + off,
-                                                 L.counters, L.slack, L.pool, L.depth, L.status);
+                                                 L.counters, L.slack, spread(L, grid * (TB / 32), n), L.depth, L.status);
         SALTY_TRY_CUDA(ctx->err, cudaGetLastError());
     }
     return SALTY_OK;
@@ -415,10 +428,21 @@ salty_status launch_queue(salty_ctx* ctx, const Launch& L) {
 template <int TB, bool CAP>
 salty_status dispatch_flags(salty_ctx* ctx, const Launch& L, uint32_t flags) {
     const bool any = flags & SALTY_TRACE_ANY_HIT, wt = flags & SALTY_TRACE_WATERTIGHT;
-    // Lanes test their own triangles where that is asked for (postponing), and in trees of up to
-    // three levels, where nearly every step ends in leaves and most lanes hold triangles (the
-    // 36-triangle Cornell box, 256 x 256 at 16 spp: 1.64 ms against 1.68 with the queue).
-    const bool own = L.postpone > 1 || L.tgt.depth <= 3;
+    // Lanes test their own triangles where that is asked for (postponing), and where the queue
+    // gains nothing:
+    // - trees of up to three levels, where nearly every step ends in leaves and most lanes hold
+    //   triangles (the 36-triangle Cornell box, 256 x 256 at 16 spp: 1.64 ms against 1.68);
+    // - a caller's rays, no more of them than the chip has lanes, where the time is that of one
+    //   walk and waiting for a queue lengthens it (100k triangles, reference's test, 100,000 rays:
+    //   252 us against 289; 400,000 rays: 543 against 511);
+    // - a caller's rays in shallow trees, whose walks are so short that refilling and queueing cost
+    //   more than fuller tests save (2M rays of a soup, own against queued: reference's test 0.66
+    //   and 0.76 ms at 6,000 triangles and 6 levels, 1.67 and 1.69 at 100k and 7, 1.84 and 1.81 at
+    //   200k and 8; watertight test 1.10 and 1.14 ms at 20k and 6, 1.54 and 1.47 at 50k and 7).
+    // Renders queue from four levels on: their rays meet larger leaves (960 x 540 terrain of 8,192
+    // triangles at 8 spp: 2.78 ms against 2.51).
+    const bool caller = !L.n_dev && (L.n <= 1024ll * ctx->num_sms || L.tgt.depth <= (wt ? 6 : 7));
+    const bool own = L.postpone > 1 || L.tgt.depth <= 3 || caller;
 #define SALTY_L(A, W) \
     if (any == A && wt == W) return own ? launch<A, W, false, TB, CAP, false>(ctx, L) : launch_queue<A, W, TB, CAP>(ctx, L)
     SALTY_L(false, false); SALTY_L(false, true); SALTY_L(true, false); SALTY_L(true, true);

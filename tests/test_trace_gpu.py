@@ -298,3 +298,38 @@ def test_queueing_walk_matches_own_tests(ctx, n, watertight):
     np.testing.assert_array_equal(occ[1], got[1].ids >= 0)
     np.testing.assert_array_equal(occ[1], occ[2])
     sc.close()
+
+
+# More rays than lanes in a tree of eight levels or more take the queueing walk under either
+# test; one lane's worth past the line and a ragged larger size, bit for bit as above.
+@pytest.mark.parametrize("extra", [1, 44353])
+@pytest.mark.parametrize("watertight", [False, True])
+def test_queueing_walk_on_deep_trees(ctx, extra, watertight):
+    import salty_gb300
+    import torch
+    tris = salty_gb300.microbench_soup(17, 300000)
+    tris[:500] = tris[0]
+    sc = _scene(ctx, tris)
+    assert sc.info["depth"] >= 8
+    n = 1024 * torch.cuda.get_device_properties(0).multi_processor_count + extra
+    rays = salty_gb300.microbench_rays(5, n, 1e-4)
+    rays[::3, 7] = 2.0
+    rays[1::5, 3] = 1.9
+    rays[7, 7] = -1.0
+    rays[8, 7] = np.nan
+    rays[9, 3] = -5.0
+    rays[10, 4:7] = (0.0, 0.0, 1.0)
+    base = ctx.tuning
+    try:
+        got, occ = {}, {}
+        for post in (1, 2):
+            ctx.tuning = {"trace_postpone": post}
+            got[post] = sc.trace(rays, watertight=watertight)
+            occ[post] = sc.trace(rays, any_hit=True, watertight=watertight).ids >= 0
+    finally:
+        ctx.tuning = base
+    for f in ("ids", "t", "u", "v"):
+        np.testing.assert_array_equal(getattr(got[1], f), getattr(got[2], f))
+    np.testing.assert_array_equal(occ[1], got[1].ids >= 0)
+    np.testing.assert_array_equal(occ[1], occ[2])
+    sc.close()
