@@ -105,3 +105,58 @@ def test_variance_nlm_at_tile_edges(ctx, oracle, h, w, search_r, patch_r):
 def test_nlm_ref_at_tile_edges(ctx, oracle, h, w):
     rgba = np.random.default_rng(h).random((h, w, 4), dtype=np.float32)
     np.testing.assert_allclose(ctx.nlm_ref(rgba, 0.6), oracle.nlm_ref(rgba, 0.6), rtol=1e-5, atol=1e-6)
+
+
+def _tonemap_device(ctx, img, out, s8, kind):
+    import ctypes as C
+    import salty_gb300
+    h, w = img.shape[:2]
+    ave, mx = C.c_float(), C.c_float()
+    ctx.check(salty_gb300.lib().salty_tonemap(ctx.h, kind, w, h, img.data_ptr(), out.data_ptr() if out is not None else None,
+                                              s8.data_ptr() if s8 is not None else None, 1, C.byref(ave), C.byref(mx)), "tonemap")
+    return np.float32(ave.value), np.float32(mx.value)
+
+
+def test_tonemap_scale_is_the_hosts(ctx):
+    """The curve's scale is key / expf(mean) in the host's arithmetic, bit for bit, whatever the
+    device's own exponential rounds to: 4,000 one-pixel images, Reinhard restated in FP32."""
+    import torch
+    f = np.float32
+    rng = np.random.default_rng(31)
+    px = np.exp(rng.normal(0.0, 3.0, size=(4000, 1, 1, 3))).astype(f)
+    imgs, out = torch.from_numpy(px).cuda(), torch.empty((1, 1, 3), device="cuda")
+    for k in range(len(px)):
+        ave, mx = _tonemap_device(ctx, imgs[k], out, None, 0)
+        c = f(0.18) / ave
+        m2 = (mx * c) * (mx * c)
+        x = px[k] * c
+        y = (x * (f(1.0) + x / m2)) / (f(1.0) + x)
+        np.testing.assert_array_equal(out.cpu().numpy(), y)
+
+
+@pytest.mark.parametrize("kind", [0, 1, 2])
+@pytest.mark.parametrize("shape", [(1, 1), (1, 3), (1, 4), (5, 1), (37, 29), (33, 1024), (700, 1601)])
+def test_tonemap_layouts_agree(ctx, shape, kind):
+    """Groups of four pixels, single values, remainders, arrays off the 16-byte boundary and
+    tonemapping in place give the same bits; the scale is the same for any order of the sum
+    here (to FP32), since it is added in FP64."""
+    import torch
+    h, w = shape
+    n = h * w * 3
+    rng = np.random.default_rng(h * w)
+    img = torch.from_numpy(np.exp(rng.normal(0.0, 2.0, size=n)).astype(np.float32)).cuda()
+    img[0] = 0.0
+    got = []
+    for off in (0, 1):
+        a = torch.empty(n + 4, device="cuda")[off:off + n]
+        a.copy_(img)
+        o = torch.full((n + 4,), -1.0, device="cuda")
+        s = torch.zeros(n + 8, dtype=torch.uint8, device="cuda")
+        _tonemap_device(ctx, a.view(h, w, 3), o[off:], s[off:], kind)
+        assert (o[off + n:] == -1.0).all() and (s[off + n:] == 0).all()
+        got.append((o[off:off + n].cpu().numpy(), s[off:off + n].cpu().numpy()))
+        _tonemap_device(ctx, a.view(h, w, 3), a, None, kind)
+        got.append((a.cpu().numpy(), got[-1][1]))
+    for o, s in got[1:]:
+        np.testing.assert_array_equal(o, got[0][0])
+        np.testing.assert_array_equal(s, got[0][1])
