@@ -333,3 +333,19 @@ def test_queueing_walk_on_deep_trees(ctx, extra, watertight):
     np.testing.assert_array_equal(occ[1], got[1].ids >= 0)
     np.testing.assert_array_equal(occ[1], occ[2])
     sc.close()
+
+
+# Host arrays in one chunk, two, and two with a ragged second one: the same hits as from device
+# memory.
+@pytest.mark.parametrize("n", [1 << 18, (1 << 18) + 1, (1 << 19) + 3])
+def test_host_chunks_match_device_arrays(ctx, n):
+    import salty_gb300
+    import torch
+    sc = _scene(ctx, salty_gb300.microbench_soup(3, 2000))
+    rays = salty_gb300.microbench_rays(4, n, 1e-4)
+    host = np.full((n, 4), -7.0, np.float32)
+    sc.trace_raw(rays, host)
+    dev = torch.empty((n, 4), device="cuda")
+    sc.trace_raw(torch.from_numpy(rays).cuda(), dev)
+    np.testing.assert_array_equal(host.view(np.uint32), dev.cpu().numpy().view(np.uint32))
+    sc.close()
