@@ -197,16 +197,17 @@ k_trace(const Bvh8Node* __restrict__ nodes, const float4* __restrict__ tris, con
 // memory however many lanes it fills (1 at a time: 5 % slower).
 // Best hits live in shared memory as (t, id) keys: t >= 0, so the bits order as the floats do,
 // and equal distances go to the lowest id.
-// Bound: instruction issue and the latency of node fetches from L2.  The register budget is 72
-// (7 blocks of 128 per SM; 56, 64 and 80 registers: 9, 3 and 3 % slower).  Measured (GB300):
-// 1080p terrain at 8 spp 27.4 -> 23.1 ms, 12 uneven scenes 20.3 -> 18.9 ms, 2.5M watertight
-// rays of the 1M-triangle soup from host arrays 2.81 -> 2.51 ms, 4.2M rays with the
-// reference's test 3.14 -> 2.96 ms.  Where it gains nothing: dispatch_flags.
+// Bound: instruction issue and the latency of node fetches from L2.  64 registers, 32 warps per
+// SM, whatever the tuning's budget (56, 72 and 80 registers: 11, 1 and 1 % slower over 1080p
+// terrain and 4.2M rays).  Measured (GB300), against k_trace: 1080p terrain at 8 spp 27.4 ->
+// 21.8 ms, 12 uneven scenes 20.3 -> 18.4 ms, 2.5M watertight rays of the 1M-triangle soup from
+// host arrays 2.81 -> 2.40 ms, 4.2M rays with the reference's test 3.14 -> 2.91 ms.  Where it
+// gains nothing: dispatch_flags.
 constexpr int kQueue = 64;    // pairs per warp: fewer than 32 before a push of at most 32
 constexpr int kRefill = 6;    // idle lanes that start a refill
 
-template <bool ANY, bool WT, int TB, bool CAP>
-__global__ void __launch_bounds__(TB, (CAP ? 896 : 1024) / TB)
+template <bool ANY, bool WT, int TB>
+__global__ void __launch_bounds__(TB, 1024 / TB)
 k_trace_queue(const Bvh8Node* __restrict__ nodes, const float4* __restrict__ tris, const float4* __restrict__ rays,
               const int* __restrict__ roots, long long n_arg, const int* __restrict__ n_dev, float4* __restrict__ hits,
               unsigned long long* __restrict__ counters, float cull_slack, int pool, int depth,
@@ -403,9 +404,9 @@ salty_status launch(salty_ctx* ctx, const Launch& L) {
     return SALTY_OK;
 }
 
-template <bool ANY, bool WT, int TB, bool CAP>
+template <bool ANY, bool WT, int TB>
 salty_status launch_queue(salty_ctx* ctx, const Launch& L) {
-    auto kern = k_trace_queue<ANY, WT, TB, CAP>;
+    auto kern = k_trace_queue<ANY, WT, TB>;
     const size_t smem = ((size_t)(L.depth + 2) * TB + (size_t)(TB / 32) * kQueue) * sizeof(uint2);
     if (smem > 48 * 1024)
         SALTY_TRY_CUDA(ctx->err, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -444,7 +445,7 @@ salty_status dispatch_flags(salty_ctx* ctx, const Launch& L, uint32_t flags) {
     const bool caller = !L.n_dev && (L.n <= 1024ll * ctx->num_sms || L.tgt.depth <= (wt ? 6 : 7));
     const bool own = L.postpone > 1 || L.tgt.depth <= 3 || caller;
 #define SALTY_L(A, W) \
-    if (any == A && wt == W) return own ? launch<A, W, false, TB, CAP, false>(ctx, L) : launch_queue<A, W, TB, CAP>(ctx, L)
+    if (any == A && wt == W) return own ? launch<A, W, false, TB, CAP, false>(ctx, L) : launch_queue<A, W, TB>(ctx, L)
     SALTY_L(false, false); SALTY_L(false, true); SALTY_L(true, false); SALTY_L(true, true);
 #undef SALTY_L
     return ctx->err.fail(SALTY_ERR_INVALID_ARG, "bad trace flags");

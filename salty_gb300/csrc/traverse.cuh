@@ -227,15 +227,21 @@ __device__ __forceinline__ unsigned long long f2_pack(unsigned lo, unsigned hi) 
     return v;
 }
 
-// A child's near and far plane bytes along one axis as exact floats: each byte placed under
-// the exponent of 2^23 (one byte permute each), then 2^23 taken off both with one packed
-// subtraction (exact for 0..255) -- two issue slots fewer per child and axis than two
-// separate subtractions.
-__device__ __forceinline__ void q2(unsigned wn, unsigned wf, int k, unsigned long long off, float& qn, float& qf) {
+__device__ __forceinline__ unsigned long long f2_dup(float v) {
+    return f2_pack(__float_as_uint(v), __float_as_uint(v));
+}
+
+// The distances to a child's near and far planes along one axis: each plane byte placed under
+// the exponent of 2^23 (one byte permute each), 2^23 taken off both (exact for 0..255), then
+// byte * a + b for both -- packed, three issue slots fewer per child and axis than separate
+// operations, with the same roundings.  a and b hold one value twice.
+__device__ __forceinline__ void plane2(unsigned wn, unsigned wf, int k, unsigned long long off, unsigned long long a,
+                                       unsigned long long b, float& tn, float& tf) {
     unsigned long long q = f2_pack(__byte_perm(wn, 0x4B000000u, 0x7540u + k),
                                    __byte_perm(wf, 0x4B000000u, 0x7540u + k));
     asm("sub.rn.f32x2 %0, %0, %1;" : "+l"(q) : "l"(off));
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(qn), "=f"(qf) : "l"(q));
+    asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(q) : "l"(a), "l"(b));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(tn), "=f"(tf) : "l"(q));
 }
 
 // Intersects the 8 children of node `idx`.  Returns inner-child hits in key order
@@ -252,8 +258,9 @@ __device__ __forceinline__ void intersect_node(const Bvh8Node* __restrict__ node
     imask = w0.w >> 24;
     child_base = w1.x;
     tri_base = w1.y;
-    const float ax = sx * r.ix, ay = sy * r.iy, az = sz * r.iz;
-    const float bx = (px - r.ox) * r.ix, by = (py - r.oy) * r.iy, bz = (pz - r.oz) * r.iz;
+    const unsigned long long ax = f2_dup(sx * r.ix), ay = f2_dup(sy * r.iy), az = f2_dup(sz * r.iz);
+    const unsigned long long bx = f2_dup((px - r.ox) * r.ix), by = f2_dup((py - r.oy) * r.iy),
+                             bz = f2_dup((pz - r.oz) * r.iz);
     // near/far plane words by ray octant
     const unsigned nlx0 = (r.oct & 1) ? w3.z : w2.x, nlx1 = (r.oct & 1) ? w3.w : w2.y;
     const unsigned nhx0 = (r.oct & 1) ? w2.x : w3.z, nhx1 = (r.oct & 1) ? w2.y : w3.w;
@@ -276,13 +283,10 @@ __device__ __forceinline__ void intersect_node(const Bvh8Node* __restrict__ node
         const unsigned meta = half ? (w1.w ^ spread_hi) : (w1.z ^ spread_lo);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            float qnx, qfx, qny, qfy, qnz, qfz;
-            q2(lx, hx, k, off, qnx, qfx);
-            q2(ly, hy, k, off, qny, qfy);
-            q2(lz, hz, k, off, qnz, qfz);
-            const float tnx = fmaf(qnx, ax, bx), tfx = fmaf(qfx, ax, bx);
-            const float tny = fmaf(qny, ay, by), tfy = fmaf(qfy, ay, by);
-            const float tnz = fmaf(qnz, az, bz), tfz = fmaf(qfz, az, bz);
+            float tnx, tfx, tny, tfy, tnz, tfz;
+            plane2(lx, hx, k, off, ax, bx, tnx, tfx);
+            plane2(ly, hy, k, off, ay, by, tny, tfy);
+            plane2(lz, hz, k, off, az, bz, tnz, tfz);
             const float tn = fmax4(tnx, tny, tnz, r.tmin);
             const float tf = fmin4(tfx, tfy, tfz, tcull);
             if (tn <= tf * kBoxSlackMul) {
