@@ -434,6 +434,7 @@ k_conv3x3_tma(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     // TMA destinations and the descriptors below assume a 1024-byte aligned base
     if (saddr(smem) & 1023u) {
+        grid_turn();
         if (tid == 0) atomicOr(a.status, 2);
         return;
     }
@@ -457,11 +458,12 @@ k_conv3x3_tma(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__
         hd.abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    for (int i = tid; i < npad; i += blockDim.x) sbias[i] = (a.bias && i < a.cout) ? a.bias[i] : 0.0f;
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" :: "r"(saddr(&hd.tmem)) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    grid_turn();
+    for (int i = tid; i < npad; i += blockDim.x) sbias[i] = (a.bias && i < a.cout) ? a.bias[i] : 0.0f;
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -672,7 +674,7 @@ k_conv3x3_tma(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__
                 if (mine) {
 #pragma unroll
                     for (int u = 0; u < kJobs; ++u)
-                        v[u] = from[u] >= 0 ? __ldg(reinterpret_cast<const uint4*>(img + from[u] + c * 16)) : make_uint4(0, 0, 0, 0);
+                        v[u] = from[u] >= 0 ? *reinterpret_cast<const uint4*>(img + from[u] + c * 16) : make_uint4(0, 0, 0, 0);
                 }
                 if (!warp_wait(saddr(hd.empty + s), ph ^ 1u, abort_flag, a.status)) { ok = false; break; }
                 if (mine) {
@@ -791,6 +793,7 @@ k_wgrad_tc(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUt
     unsigned char* stage0 = smem + kWgHeader;
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     if (saddr(smem) & 1023u) {  // the swizzled boxes need 1 KB aligned destinations
+        grid_turn();
         if (tid == 0) atomicOr(a.status, 2);
         return;
     }
@@ -815,6 +818,7 @@ k_wgrad_tc(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUt
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" :: "r"(saddr(tmem_slot)) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    grid_turn();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -887,8 +891,8 @@ k_wgrad_tc(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUt
                 const int cy = cy0 + p / kCx, cx = cx0 + p % kCx;
                 v[u] = make_uint4(0, 0, 0, 0);
                 if (box < ncx && cy >= 0 && cy < Hc && cx >= 0 && cx < Wc)
-                    v[u] = __ldg(reinterpret_cast<const uint4*>(a.coarse + (((size_t)n * Hc + cy) * Wc + cx) * a.coarse_cs + c0 +
-                                                                box * 16 + half * 8));
+                    v[u] = *reinterpret_cast<const uint4*>(a.coarse + (((size_t)n * Hc + cy) * Wc + cx) * a.coarse_cs + c0 +
+                                                           box * 16 + half * 8);
             }
             if (!warp_wait(saddr(empty + b), ((uint32_t)(it / kWgStages) & 1u) ^ 1u, abort_flag, a.status)) {
                 ok = false;
@@ -950,6 +954,7 @@ k_wgrad_tc(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUt
 // layer (8 us each, latency) took 190 us of 1.73 ms at 16 x 256 x 256.
 __global__ void __launch_bounds__(256) k_grad_reduce(const __grid_constant__ GradReduceTable T) {
     __shared__ float4 sm[8][32];
+    grid_turn();
     int e = 0;
     while (e + 1 < T.n && (int)blockIdx.x >= T.e[e + 1].block0) ++e;
     const GradReduceTable::Entry E = T.e[e];
@@ -963,7 +968,7 @@ __global__ void __launch_bounds__(256) k_grad_reduce(const __grid_constant__ Gra
         const float* p = E.part + ((size_t)(r / E.rows) * E.pad_rows + r % E.rows) * E.row4 * 4 + j * 4;
 #pragma unroll 4
         for (int k = row; k < E.slices; k += 8) {
-            const float4 v = __ldg(reinterpret_cast<const float4*>(p + (size_t)k * E.stride));
+            const float4 v = *reinterpret_cast<const float4*>(p + (size_t)k * E.stride);
             s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
         }
     }
@@ -1059,8 +1064,8 @@ salty_status conv3x3_tma(salty_ctx* ctx, const ConvSrc& in, int cin, const bf16*
                   coarse ? in.a : nullptr, coarse ? in.a_cs : 0, coarse ? in.a_ch : 0, d_status};
     auto kern = coarse ? k_conv3x3_tma<true> : k_conv3x3_tma<false>;
     SALTY_TRY_CUDA(ctx->err, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<grid, kTmaThreads + (coarse ? 32 * kTmaCoarseWarps : 0), smem, ctx->stream>>>(tm_in, tm_w, a);
-    SALTY_TRY_CUDA(ctx->err, cudaGetLastError());
+    SALTY_TRY_CUDA(ctx->err, launch_early(kern, grid, kTmaThreads + (coarse ? 32 * kTmaCoarseWarps : 0), smem, ctx->stream,
+                                          tm_in, tm_w, a));
     return SALTY_OK;
 }
 
@@ -1117,8 +1122,8 @@ salty_status conv_wgrad_tc(salty_ctx* ctx, const bf16* dy, int cpad, int cout, c
     SALTY_TRY_CUDA(ctx->err, cudaFuncSetAttribute(k_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     WgradArgs a{cpad <= 64 ? 64 : 128, cpad, cout, cin, N, H, W, strips, ws, coarse ? x.a : nullptr,
                 coarse ? x.a_cs : 0, coarse ? x.a_ch : 0, d_status};
-    k_wgrad_tc<<<dim3(slices, groups), coarse ? kWgCoarseThreads : kWgThreads, smem, ctx->stream>>>(tm_x, tm_dy, a);
-    SALTY_TRY_CUDA(ctx->err, cudaGetLastError());
+    SALTY_TRY_CUDA(ctx->err, launch_early(k_wgrad_tc, dim3(slices, groups), coarse ? kWgCoarseThreads : kWgThreads, smem,
+                                          ctx->stream, tm_x, tm_dy, a));
     return grad_reduce_add(ctx, table, {ws, dw, slices, 9 * cpad * cin, cin / 4, cout, cpad, 9 * cout * (cin / 4), 0});
 }
 
@@ -1131,7 +1136,8 @@ salty_status grad_reduce_add(salty_ctx* ctx, GradReduceTable& table, GradReduceT
 }
 
 salty_status grad_reduce_run(salty_ctx* ctx, const GradReduceTable& table) {
-    if (table.blocks > 0) k_grad_reduce<<<table.blocks, 256, 0, ctx->stream>>>(table);
+    if (table.blocks > 0)
+        SALTY_TRY_CUDA(ctx->err, launch_early(k_grad_reduce, table.blocks, 256, 0, ctx->stream, table));
     SALTY_TRY_CUDA(ctx->err, cudaGetLastError());
     return SALTY_OK;
 }

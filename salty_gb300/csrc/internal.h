@@ -350,6 +350,38 @@ salty_status nlm_ref_device(salty_ctx* ctx, int w, int h, float coeff, const flo
 salty_status nlm_var_device(salty_ctx* ctx, int w, int h, int search_r, int patch_r, float k,
                             const float* d_rgb, const float* d_var, float* d_out);
 
+// Launches a kernel that may start while the kernel before it in the stream drains: its blocks
+// take the multiprocessors that come free and run up to their cudaGridDependencySynchronize(),
+// which waits for the whole of the earlier kernel and its stores.  For kernels that touch no
+// global memory before that call and read what earlier kernels wrote with plain loads (not the
+// read-only path, which asks for data that does not change while the kernel exists).  Measured
+// over the U-Net's chains of convolution and gradient kernels: a training step of 16 x 256 x 256
+// 1,548 -> 1,435 us, an eight-fold 1080p denoise (long kernels) 3,027 -> 3,008 us.
+template <class... P, class... A>
+cudaError_t launch_early(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
+#ifdef __CUDACC__
+// The point in a kernel launched with launch_early from which global memory may be touched; the
+// next kernel's blocks may come in once every block here has passed it (so at most one kernel
+// waits behind a running one).
+__device__ __forceinline__ void grid_turn() {
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
+}
+#endif
+
 inline bool is_device_ptr(const void* p) {
     if (!p) return false;
     cudaPointerAttributes a;

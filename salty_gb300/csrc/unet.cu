@@ -435,9 +435,10 @@ struct GradSrc {
 // 8-channel group t % G of the pixels (2x2 blocks for GRAD_SKIP) t / G, t / G + per, ... of
 // the block's grid stride.  C and the strides are multiples of 8.
 template <int KIND>
-__global__ void __launch_bounds__(256) k_grad_in(const bf16* __restrict__ y, GradSrc src, int C, int N, int H, int W,
-                                                 bf16* __restrict__ g, float* __restrict__ part) {
+__global__ void __launch_bounds__(256) k_grad_in(const bf16* y, GradSrc src, int C, int N, int H, int W, bf16* g,
+                                                 float* part) {
     extern __shared__ float sb[];  // [per][C]
+    grid_turn();
     const int G = C / 8, per = blockDim.x / G;
     const int j = threadIdx.x % G, r = threadIdx.x / G, c = j * 8;
     float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -452,7 +453,7 @@ __global__ void __launch_bounds__(256) k_grad_in(const bf16* __restrict__ y, Gra
 #pragma unroll
         for (int k = 0; k < 8; ++k) s[k] += w[k];
     };
-    auto ld = [](const bf16* p) { return __ldg(reinterpret_cast<const uint4*>(p)); };
+    auto ld = [](const bf16* p) { return *reinterpret_cast<const uint4*>(p); };
     if (r < per) {
         if (KIND == GRAD_SKIP) {
             const int Ho = H / 2, Wo = W / 2;
@@ -865,10 +866,8 @@ salty_status grad_in(salty_ctx* ctx, Unet& u, Fwd& F, int li, int y, const GradS
     const UnetLayer& L = u.layers[li];
     const long long npx = (long long)N * h * w, work = KIND == GRAD_SKIP ? npx / 4 : npx;
     const int per = 256 / (L.cout / 8), blocks = grad_blocks(ctx, work, per);
-    k_grad_in<KIND><<<blocks, 256, (size_t)per * L.cout * sizeof(float), ctx->stream>>>(F.t[y], src, L.cout, N, h, w,
-                                                                                      F.t[T_G],
-                                                                                      u.wg_ws.p + u.bias_off[li]);
-    SALTY_TRY_CUDA(ctx->err, cudaGetLastError());
+    SALTY_TRY_CUDA(ctx->err, launch_early(k_grad_in<KIND>, blocks, 256, (size_t)per * L.cout * sizeof(float), ctx->stream,
+                                          F.t[y], src, L.cout, N, h, w, F.t[T_G], u.wg_ws.p + u.bias_off[li]));
     return bias_reduce_add(ctx, u, li, blocks, table);
 }
 
