@@ -296,13 +296,18 @@ __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? l
 // the neighbour pixel from the staged tile.  The block's warps share the tile and take the
 // search offsets in turn (their accumulators are added at the end, in warp order), which
 // gives small images four times as many warps as tiles.  Nothing is clamped in the walk: the
-// staged tile holds the border-clamped pixels.  kNlmRows = 16 costs 1 + 2P/16 of the terms
-// of an ideal walk and keeps centre and accumulators within 255 registers (8 warps per SM).
-// Bound: instruction issue (65 % of the slots at 2 warps per scheduler, FMA pipe 41 %).
+// staged tile holds the border-clamped pixels.  A tile of r rows costs 1 + 2P/r of the terms of an
+// ideal walk; 16 (kNlmRows) keep the reference filter's centre and accumulators within 255
+// registers (8 warps per SM), and 12 (kVarRows) leave the variance-scaled one's room to load
+// ahead (1080p, radius 3: 16 rows 2.71 ms, 13 2.49, 12 2.39-2.45, 11 2.64, 10 2.58, 8 2.74, 8 at three
+// blocks per SM 2.82).
+// Bound: instruction issue and the latency that 2 warps per scheduler leave (packed FP32
+// operations 20 % slower, one reciprocal for three quotients 2 % faster and not kept).
 // Measured (GB300), against one thread per pixel with the terms and row sums in shared memory
 // (variance-scaled) or all 25 taps per offset (reference): 1920 x 1080, 21 x 21 search, 7 x 7
-// patch 10.25 -> 2.70 ms; 1279 x 719 FilterNLM 3.26 -> 0.27 ms.
+// patch 10.25 -> 2.42 ms; 1279 x 719 FilterNLM 3.26 -> 0.27 ms.
 constexpr int kNlmRows = 16;
+constexpr int kVarRows = 12;
 constexpr int kNlmWarps = 4;
 
 // Sum of the 2P+1 terms v - 2P .. v of one column, from the sums of shorter runs.
@@ -350,20 +355,20 @@ __device__ __forceinline__ float lane_sum(float v) {
 
 // Adds the warps' accumulators acc[kNlmRows][C] in warp order into warp 0's, through shared
 // memory (C * 32 floats per row; the staged tile is dead by then).
-template <int C>
-__device__ __forceinline__ void add_warps(float (&acc)[kNlmRows][C], float* sm, int warp, int lane, int warps) {
+template <int C, int ROWS>
+__device__ __forceinline__ void add_warps(float (&acc)[ROWS][C], float* sm, int warp, int lane, int warps) {
     for (int k = 1; k < warps; ++k) {
         __syncthreads();
         if (warp == k) {
 #pragma unroll
-            for (int y = 0; y < kNlmRows; ++y)
+            for (int y = 0; y < ROWS; ++y)
 #pragma unroll
                 for (int c = 0; c < C; ++c) sm[(y * C + c) * 32 + lane] = acc[y][c];
         }
         __syncthreads();
         if (warp == 0) {
 #pragma unroll
-            for (int y = 0; y < kNlmRows; ++y)
+            for (int y = 0; y < ROWS; ++y)
 #pragma unroll
                 for (int c = 0; c < C; ++c) acc[y][c] += sm[(y * C + c) * 32 + lane];
         }
@@ -414,7 +419,7 @@ __global__ void __launch_bounds__(32 * kNlmWarps, 2) k_nlm_ref(const float4* __r
             A[4] += wt;
         }
     }
-    add_warps<5>(acc, reinterpret_cast<float*>(tile), warp, lane, kNlmWarps);
+    add_warps(acc, reinterpret_cast<float*>(tile), warp, lane, kNlmWarps);
     const int x = bx + lane - P;
     if (warp != 0 || lane < P || lane >= 32 - P || x >= w) return;
 #pragma unroll
@@ -435,7 +440,7 @@ __global__ void __launch_bounds__(32 * kNlmWarps, 2) k_nlm_ref(const float4* __r
 // patch border, sums it along rows and then columns in shared memory, and every pixel reads
 // its distance: O(1) work per pixel and offset instead of O(patch).  The same sums as the
 // direct double loop in a different order, with quotients within 2 ulp.  Patch radii 1..3 run
-// as column walks (k_nlm_var_cols, 3.8x faster at radius 3); k_nlm_var keeps the others, whose
+// as column walks (k_nlm_var_cols, 4.2x faster at radius 3); k_nlm_var keeps the others, whose
 // centre pixels would not fit the registers (radius >= 4) or need no box sum (radius 0).
 constexpr int kVTile = 16;
 
@@ -511,20 +516,20 @@ __global__ void __launch_bounds__(kVTile* kVTile) k_nlm_var(const float* __restr
 }
 
 // The same filter by column walks, for patch radii up to 3 (centre pixels and variances of
-// kNlmRows + 2P rows in registers).  RM: largest search radius, the staged tile's column pitch
+// ROWS + 2P rows in registers).  RM: largest search radius, the staged tile's column pitch
 // is fixed by it.
-template <int P, int RM>
+template <int P, int RM, int ROWS>
 __global__ void __launch_bounds__(32 * kNlmWarps, 2)
 k_nlm_var_cols(const float* __restrict__ rgb, const float* __restrict__ var, int w, int h, int R, float k2, float norm,
                float* __restrict__ out) {
-    constexpr int N = kNlmRows + 2 * P, S = 32 + 2 * RM;
+    constexpr int N = ROWS + 2 * P, S = 32 + 2 * RM;
     extern __shared__ __align__(16) float sm[];
     const int rows = N + 2 * R, cols = 32 + 2 * R;
     float2* t0 = reinterpret_cast<float2*>(sm);  // (r, g), (b, var r), (var g, var b)
     float2* t1 = t0 + rows * S;
     float2* t2 = t1 + rows * S;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int bx = blockIdx.x * (32 - 2 * P), by = blockIdx.y * kNlmRows;
+    const int bx = blockIdx.x * (32 - 2 * P), by = blockIdx.y * ROWS;
     for (int i = threadIdx.x; i < rows * cols; i += 32 * kNlmWarps) {
         const int ty = i / cols, tx = i - ty * cols;
         const size_t g = ((size_t)clampi(by - P - R + ty, 0, h - 1) * w + clampi(bx - P - R + tx, 0, w - 1)) * 3;
@@ -543,9 +548,9 @@ k_nlm_var_cols(const float* __restrict__ rgb, const float* __restrict__ var, int
         a[v][0] = p0.x; a[v][1] = p0.y; a[v][2] = p1.x;
         va[v][0] = p1.y; va[v][1] = p2.x; va[v][2] = p2.y;
     }
-    float acc[kNlmRows][4];
+    float acc[ROWS][4];
 #pragma unroll
-    for (int y = 0; y < kNlmRows; ++y)
+    for (int y = 0; y < ROWS; ++y)
 #pragma unroll
         for (int c = 0; c < 4; ++c) acc[y][c] = 0.0f;
     const int side = 2 * R + 1;
@@ -575,11 +580,11 @@ k_nlm_var_cols(const float* __restrict__ rgb, const float* __restrict__ var, int
             A[3] += wt;
         }
     }
-    add_warps<4>(acc, sm, warp, lane, kNlmWarps);
+    add_warps(acc, sm, warp, lane, kNlmWarps);
     const int x = bx + lane - P;
     if (warp != 0 || lane < P || lane >= 32 - P || x >= w) return;
 #pragma unroll
-    for (int y = 0; y < kNlmRows; ++y)
+    for (int y = 0; y < ROWS; ++y)
         if (by + y < h) {
             const size_t o = ((size_t)(by + y) * w + x) * 3;
 #pragma unroll
@@ -587,14 +592,17 @@ k_nlm_var_cols(const float* __restrict__ rgb, const float* __restrict__ var, int
         }
 }
 
-template <int P, int RM>
+template <int P, int RM, int ROWS>
 salty_status launch_nlm_var_cols(salty_ctx* ctx, int w, int h, int R, float k2, float norm, const float* rgb,
                                  const float* var, float* out) {
-    const size_t tile = (size_t)(kNlmRows + 2 * P + 2 * R) * (32 + 2 * RM) * 3 * sizeof(float2);
-    const size_t smem = std::max(tile, (size_t)kNlmRows * 4 * 32 * sizeof(float));
-    auto kern = k_nlm_var_cols<P, RM>;
+    const dim3 grid((w + 31 - 2 * P) / (32 - 2 * P), (h + ROWS - 1) / ROWS);
+    // fewer tiles than SMs: shorter ones, more of them (200 x 150, radius 3: 89 -> 72 us)
+    if (ROWS > 8 && (long long)grid.x * grid.y <= ctx->num_sms)
+        return launch_nlm_var_cols<P, RM, 8>(ctx, w, h, R, k2, norm, rgb, var, out);
+    const size_t tile = (size_t)(ROWS + 2 * P + 2 * R) * (32 + 2 * RM) * 3 * sizeof(float2);
+    const size_t smem = std::max(tile, (size_t)ROWS * 4 * 32 * sizeof(float));
+    auto kern = k_nlm_var_cols<P, RM, ROWS>;
     SALTY_TRY_CUDA(ctx->err, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const dim3 grid((w + 31 - 2 * P) / (32 - 2 * P), (h + kNlmRows - 1) / kNlmRows);
     kern<<<grid, 32 * kNlmWarps, smem, ctx->stream>>>(rgb, var, w, h, R, k2, norm, out);
     SALTY_TRY_CUDA(ctx->err, cudaGetLastError());
     return SALTY_OK;
@@ -676,8 +684,8 @@ salty_status nlm_var_device(salty_ctx* ctx, int w, int h, int search_r, int patc
     const float norm = 1.0f / (3.0f * (float)((2 * patch_r + 1) * (2 * patch_r + 1)));
 #define SALTY_NLM(P)                                                                                       \
     if (patch_r == P)                                                                                      \
-        return search_r <= 10 ? launch_nlm_var_cols<P, 10>(ctx, w, h, search_r, k * k, norm, d_rgb, d_var, d_out) \
-                              : launch_nlm_var_cols<P, 32>(ctx, w, h, search_r, k * k, norm, d_rgb, d_var, d_out)
+        return search_r <= 10 ? launch_nlm_var_cols<P, 10, kVarRows>(ctx, w, h, search_r, k * k, norm, d_rgb, d_var, d_out) \
+                              : launch_nlm_var_cols<P, 32, kVarRows>(ctx, w, h, search_r, k * k, norm, d_rgb, d_var, d_out)
     SALTY_NLM(1);
     SALTY_NLM(2);
     SALTY_NLM(3);

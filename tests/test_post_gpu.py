@@ -160,3 +160,14 @@ def test_tonemap_layouts_agree(ctx, shape, kind):
     for o, s in got[1:]:
         np.testing.assert_array_equal(o, got[0][0])
         np.testing.assert_array_equal(s, got[0][1])
+
+
+# Enough tiles for the taller column walks (12 rows; the sizes above take 8), with one row, one
+# column and a full tile over.
+@pytest.mark.parametrize("h,w,patch_r", [(397, 157, 3), (396, 156, 3), (385, 169, 2), (409, 151, 1)])
+def test_variance_nlm_on_tall_tiles(ctx, oracle, h, w, patch_r):
+    rng = np.random.default_rng(h + patch_r)
+    img = rng.random((h, w, 3), dtype=np.float32)
+    var = (0.02 * rng.random((h, w, 3))).astype(np.float32)
+    out = ctx.nlm(img, var, search_r=2, patch_r=patch_r, k=0.6)
+    np.testing.assert_allclose(out, oracle.nlm_var(img, var, 2, patch_r, 0.6), rtol=1e-4, atol=1e-5)
