@@ -63,7 +63,7 @@ CPU_SAMPLE = 2_097_152      # rays of the same stream timed on the host cores (~
 # triangle postponing) on the same soup at 4,194,304 rays; the traffic (rays in, hits out,
 # L2 misses) scales with the ray count, so traffic per launch is this figure times the rays
 # of the launch.
-NCU_DRAM_BYTES_PER_RAY = (388.030208e6 + 69.070336e6) / 4_194_304
+NCU_DRAM_BYTES_PER_RAY = (344.759552e6 + 65.560576e6) / 4_194_304
 
 
 def measured_peaks_tensor() -> dict:

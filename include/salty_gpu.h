@@ -324,11 +324,12 @@ salty_status salty_render_batch(salty_ctx* ctx, salty_scene* const* scenes, cons
 typedef struct salty_tuning {
     int32_t trace_block;     /* traversal threads per block: 64, 128 or 256 */
     int32_t trace_pool;      /* rays a warp takes from the queue per refill, 32..4096 */
-    int32_t trace_postpone;  /* fewest lanes that test a triangle group together, 1..32; at 1 the
-                              * lanes of a warp queue their triangles and test them together */
+    int32_t trace_postpone;  /* fewest lanes that test a triangle group together, 1..32; at 1,
+                              * in deeper trees and for more rays than the chip has lanes, a
+                              * warp queues its triangles and tests them together */
     int32_t shade_block;     /* shading threads per block, a multiple of 32 in 64..1024 */
     int32_t trace_regs;      /* traversal registers per thread: 64, or 56 (more resident warps;
-                              * the queueing walk takes 72 instead, its fastest) */
+                              * the queueing walk always takes 64) */
     int64_t wave_paths;      /* paths in flight (queue capacity), 2^16..2^27; default 2^24
                               * (352 bytes of path state per path plus per-sample buffers of
                               * up to 7x as many samples at 48 bytes: about 11 GB for a

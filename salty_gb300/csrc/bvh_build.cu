@@ -566,7 +566,9 @@ __global__ void __launch_bounds__(1024) k_top_dp(const BNode* __restrict__ bn, C
 // primitive: lane i tries the split after its own bin (the only bins where the two sides
 // change), which finds the same split as the bins do.  Then the costs of the collapse, deepest
 // level first.  Building every level of 1M triangles with passes over all primitives took
-// 23.1 ms of kernels, a third of it below this size; here it is one launch.
+// 23.1 ms of kernels; the levels below this size are one launch of 0.87 ms here.  Bound: the
+// latency of shared-memory chains (issue 52 % at 16 warps per SM; 64 or 96 threads, five or six
+// blocks per SM, and all warps on a level's one or two large ranges are no faster).
 constexpr int kSubThreads = 128;
 constexpr int kSubWarps = kSubThreads / 32;
 constexpr unsigned short kNoLevel = 0xffff;
@@ -934,7 +936,7 @@ __device__ int collapse_children(const BNode* __restrict__ bn, const CollapseDP*
 // cnt8[level + 1].  Quantisation is exact in FP32: a plane's grid index is the floor (ceiling)
 // of (plane - origin) / 2^e, every index of 8 bits times 2^e is a float, so rounding the
 // difference down (up) first cannot move it across an index (64-bit divisions took half of
-// this kernel: 1.11 -> 0.2 ms for 1M triangles, with one atomic per warp instead of per node).
+// this kernel: 1.11 -> 0.41 ms for 1M triangles, with one atomic per warp instead of per node).
 __global__ void __launch_bounds__(128) k_collapse(int level, const BNode* __restrict__ bn, const int* __restrict__ work,
                                                   Bvh8Node* __restrict__ out, float4* __restrict__ tris,
                                                   const int* __restrict__ prim, const float* __restrict__ pos,

@@ -4,7 +4,7 @@
 // arithmetic.  For an FP32 film of fewer than 2^24 samples the same values come from pairs of
 // FP32 numbers (error-free products and differences: Dekker 1971, Knuth TAOCP 2, 4.2.2), which
 // hold 48 bits: FP64 runs at a 64th of the FP32 rate here and its three divisions per value
-// took 436 us of a 1080p film read-out, this form 23 us (bound by the film's bytes).  The mean
+// took 436 us of a 1080p film read-out, this form 32 us (bound by the film's bytes).  The mean
 // is the correctly rounded quotient either way (53 >= 2 * 24 + 2 bits).  Sums whose products
 // could overflow or lose bits to denormals take the 64-bit form.
 #pragma once

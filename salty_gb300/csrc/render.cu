@@ -11,9 +11,10 @@
 //            surviving paths into the next queue (warp ballot + one atomic per warp)
 // then, for both halves together, accumulate the samples whose paths have all ended to the
 // film in sample order (Kahan-compensated FP32, or FP64) and plan the next iteration's new
-// samples.  Queue lengths stay in device memory, so the whole frame is one CUDA graph whose
-// conditional while-node repeats the iterations; each half's launches fill the SMs the
-// other half's traversal tail leaves idle.
+// samples.  Queue lengths stay in device memory, so the host never waits within a frame: one
+// that fits the queues and whose paths are short is launched straight into the streams, any
+// other is one CUDA graph whose conditional while-node repeats the iterations.  Each half's
+// launches fill the SMs the other half's traversal tail leaves idle.
 //
 // Two estimators:
 //   SALTY_PROFILE_COMPAT reproduces the reference's estimator: pixel-centre rays, uniform
@@ -1782,8 +1783,8 @@ salty_status render_batch(salty_ctx* ctx, salty_scene* const* scenes, const salt
     // A render whose samples all start at once (one generation) and whose paths are short ends
     // after max_depth iterations and a single accumulation, so its launches go straight into
     // the streams: nothing to instantiate, no generation or control launch per iteration, and
-    // the halves meet only at the end.  (256 x 256 Cornell box at 16 spp: 1.67 -> 1.40 ms; a 16 x 16
-    // frame at depth 8: 0.61 -> 0.29 ms.)  Longer paths keep the graph, which stops once all paths have ended.
+    // the halves meet only at the end.  (256 x 256 Cornell box at 16 spp: 1.68 -> 1.36 ms; a 16 x 16
+    // frame at depth 8: 0.66 -> 0.49 ms.)  Longer paths keep the graph, which stops once all paths have ended.
     const bool direct = !host_loop && samples <= cap && ring >= samples && max_depth <= kDirectDepth;
     auto run_direct = [&]() -> salty_status {
         if (split) SALTY_TRY(fork());

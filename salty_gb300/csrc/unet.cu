@@ -21,8 +21,8 @@
 //                 nine taps of a 16-channel input slice (one dY fragment serves nine taps),
 //                 sums its pixel tiles in registers and adds the partial into FP32 gradients.
 // All three convolutions run by default on tcgen05 (conv_tc.cu: TMEM accumulators; the
-// forward and backward-data ones over 128-pixel strips, inputs in one tensor staged by TMA
-// in a persistent warp-specialised kernel, the decoder's two-source inputs by cp.async; the
+// forward and backward-data ones over 128-pixel strips staged by TMA in a persistent
+// warp-specialised kernel, where the decoder's coarse level is expanded by warps of its own; the
 // weight gradient over strips of 2 rows x 64 pixels with dY transposed as the MMA's A, the
 // input's halo as B and the taps as descriptor offsets, summed over CTAs in a fixed order);
 // the mma.sync kernels below stay selectable (salty_unet_set_conv_kernel) and are the
@@ -431,7 +431,7 @@ struct GradSrc {
 // A layer's output gradient summed in FP32, its ReLU mask (y > 0), the rounding to BF16 that
 // the next GEMMs read (g [npx][C]) and the bias gradient's partial sums, in one pass: the
 // FP32 copies of the gradients that three kernels wrote and read before are never stored
-// (gradients of 16 x 256 x 256: element-wise kernels 0.55 -> 0.2 ms).  Thread t of a block takes
+// (gradients of 16 x 256 x 256: element-wise kernels 0.55 -> 0.26 ms).  Thread t of a block takes
 // 8-channel group t % G of the pixels (2x2 blocks for GRAD_SKIP) t / G, t / G + per, ... of
 // the block's grid stride.  C and the strides are multiples of 8.
 template <int KIND>
