@@ -172,3 +172,22 @@ def test_tma_kernel_grouped_taps(k, launches):
         jobs = max(((y0 + R0) // 2 - (y0 - 1) // 2 + 1) * (k["kStrip"] // 2 + 2) * 2 for y0 in range(0, 16 * R0, R0))
         m = re.search(r"constexpr int kJobs = (\d+);", s)
         assert jobs <= int(m.group(1)) * 32 * _const(s, "kTmaCoarseWarps")
+
+
+def test_tma_kernel_grouped_taps_at_every_strip_height(k, launches):
+    """Small levels run in strips of 2 rows up to the layer's most: at each height every row gets
+    its nine taps in the same order, inside the stage and the accumulator."""
+    for _, _, cout, _ in launches:
+        R0, npad = rows(k, cout)
+        for R in range(2, R0 + 1):
+            got = {r: [] for r in range(R)}
+            for h in range(R + 2):
+                ky0 = 0 if h < R else h - R + 1
+                n = min(h, 2) - ky0 + 1
+                col = (R - 1 - h + ky0) * npad
+                assert n >= 1 and 0 <= col and col + n * npad <= 256
+                for kx in range(3):
+                    assert (h * k["kHaloW"] + kx) * 32 + k["kStrip"] * 32 <= (R + 2) * k["kHaloW"] * 32
+                    for i in range(n):
+                        got[R - 1 - (col // npad + i)].append((ky0 + i, kx))
+            assert all(g == [(ky, kx) for ky in range(3) for kx in range(3)] for g in got.values())

@@ -288,3 +288,16 @@ def test_tcgen05_full_frame_and_tiny_batch(ctx, shape):
     cos = g1 @ g2 / (np.linalg.norm(g1) * np.linalg.norm(g2))
     assert cos > 0.999, cos
     net.close()
+
+
+@pytest.mark.parametrize("h,w", [(16, 16), (48, 272), (176, 144)])
+def test_short_strips_give_the_same_output(ctx, h, w):
+    """One image has fewer strips than SMs and runs in shorter ones; 40 of them fill the GPU with
+    the layers' tallest at the upper levels.  Outputs are the same bit for bit."""
+    import salty_gb300
+    net = salty_gb300.Unet(ctx, seed=21)
+    f, _ = _batch(18, n=40, h=h, w=w)
+    many = net.forward(f)
+    for i in (0, 23, 39):
+        np.testing.assert_array_equal(net.forward(f[i:i + 1])[0], many[i])
+    net.close()
