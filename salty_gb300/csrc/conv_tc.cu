@@ -725,16 +725,20 @@ EncodeTiledFn tensor_map_encoder() {
 // the tensor cores with the pixels as its K dimension,
 //   M = output channels (dY transposed; 64 rows when they fit, else 128, of which cout
 //       are real),
-//   N = a chunk of up to 48 input channels (a CTA group's share), one accumulator of N
-//       TMEM columns per tap (9 x 48 <= 512),
+//   N = 16 input channels at a row's three horizontal taps (48), for each vertical tap and
+//       16-channel box of a CTA group's share of up to 48 channels: up to 9 x 48 <= 512 TMEM
+//       columns,
 //   K = pixels: a strip of kWgRows image rows x 64 pixels per stage, 16 per MMA.
 // A stage holds the strip's dY (boxes of 16 channels x 64 pixels x kWgRows rows) and the
 // input's halo (boxes of 16 channels x 66 pixels x kWgRows + 2 rows), both copied by TMA in
 // the 32-byte swizzle, which is the tensor core's MN-major layout: one 32-byte row (16
 // channels) per pixel, 8-pixel groups 256 bytes apart (stride byte offset), the next 16
-// channels one box further (leading byte offset).  A tap's B operand is the same halo with
-// its start moved to row r + ky, pixel kx -- the copy engine has zero-filled the image
-// border -- so the input is read once per strip, not once per tap.  CTAs of a group split
+// channels one box further (leading byte offset).  The B operand of vertical tap ky is the same
+// halo from row r + ky, and its three 16-column groups, the horizontal taps, lie one pixel apart
+// (a leading byte offset of 32) -- the copy engine has zero-filled the image border -- so the input
+// is read once per strip, not once per tap, and dY once per vertical tap: an MMA costs its
+// operand reads, 16 + N / 4 cycles at M = 64, so a 32-channel chunk takes 6 x 28 instead of the
+// 9 x 24 of one MMA per tap (gradients of 16 x 256 x 256: a training step 1,436 -> 1,410 us).  CTAs of a group split
 // the strips between them (K-split): each writes its partial sums to its own slice of a
 // workspace, and k_grad_reduce adds the slices in a fixed order -- the result does not depend on
 // scheduling, unlike atomics.
@@ -848,9 +852,9 @@ k_wgrad_tc(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUt
         }
     } else if (warp == 1) {  // converged, one elected lane issues (see k_conv3x3_tma)
         const uint32_t el = elect_lane();
-        const uint32_t idesc = idesc_bf16_mn(a.m, ch);
-        const uint64_t da = sdesc_sw32_mn(0, kWgDyBox), db = sdesc_sw32_mn(0, kWgXBox);
-        const uint32_t alo = (uint32_t)da, blo = (uint32_t)db, dhi = (uint32_t)(da >> 32);
+        const uint32_t idesc = idesc_bf16_mn(a.m, 48);
+        const uint64_t da = sdesc_sw32_mn(0, kWgDyBox), db = sdesc_sw32_mn(0, 32);
+        const uint32_t alo = (uint32_t)da, blo = (uint32_t)db, dhi = (uint32_t)(da >> 32);  // the upper halves are equal
         for (int it = 0; it < count; ++it) {
             const int b = it % kWgStages;
             if (!warp_wait(saddr(full + b), (uint32_t)(it / kWgStages) & 1u, abort_flag, a.status)) {
@@ -865,9 +869,11 @@ k_wgrad_tc(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUt
                     const uint32_t ak = a0 + (uint32_t)(r * kWgStrip + 16 * k) * 2u;
                     const uint32_t bk = b0 + (uint32_t)(r * kWgHaloW + 16 * k) * 2u;
 #pragma unroll
-                    for (int tap = 0; tap < 9; ++tap)
-                        umma_elect(tmem + tap * ch, ak, bk + (uint32_t)((tap / 3) * kWgHaloW + tap % 3) * 2u, dhi, idesc, el,
-                                   (it > 0 || r > 0 || k > 0) ? 1u : 0u);
+                    for (int ky = 0; ky < 3; ++ky)
+                        for (int j = 0; j < nx; ++j)
+                            umma_elect(tmem + (uint32_t)(ky * nx + j) * 48u, ak,
+                                       bk + (uint32_t)(j * kWgXBox / 16 + ky * kWgHaloW * 2), dhi, idesc, el,
+                                       (it > 0 || r > 0 || k > 0) ? 1u : 0u);
                 }
             umma_commit_elect(saddr(empty + b), el);
         }
@@ -931,7 +937,7 @@ k_wgrad_tc(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUt
         for (int tap = 0; tap < 9; ++tap)
             for (int j = 0; j < nx; ++j) {
                 uint32_t v[16];
-                tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + tap * ch + j * 16, v);
+                tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (tap / 3 * nx + j) * 48 + tap % 3 * 16, v);
                 if (co >= a.cout) continue;
                 float4* dst = reinterpret_cast<float4*>(part + ((size_t)tap * a.cpad + co) * a.cin + c0 + j * 16);
 #pragma unroll

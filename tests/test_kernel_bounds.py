@@ -191,3 +191,30 @@ def test_tma_kernel_grouped_taps_at_every_strip_height(k, launches):
                     for i in range(n):
                         got[R - 1 - (col // npad + i)].append((ky0 + i, kx))
             assert all(g == [(ky, kx) for ky in range(3) for kx in range(3)] for g in got.values())
+
+
+def test_weight_gradient_operands_and_columns():
+    """k_wgrad_tc's B operand is a 16-channel box at three horizontal taps one pixel apart: every
+    group of 16 columns must read pixels inside the halo box, and the accumulators of the three
+    vertical taps and up to three boxes must be disjoint, inside TMEM, and read back at the
+    columns the MMAs wrote."""
+    s = _src("conv_tc.cu")
+    strip, nrows, chunk = _const(s, "kWgStrip"), _const(s, "kWgRows"), _const(s, "kWgChunk")
+    halo = strip + 2
+    for nx in range(1, chunk // 16 + 1):
+        cols = {}
+        for ky in range(3):
+            for j in range(nx):
+                d = (ky * nx + j) * 48
+                for kx in range(3):
+                    for c in range(16):
+                        assert cols.setdefault(d + kx * 16 + c, (ky, j, kx, c)) == (ky, j, kx, c)
+                    for r in range(nrows):
+                        for k in range(strip // 16):
+                            first = (r + ky) * halo + 16 * k + kx
+                            assert (first + 15) // halo == r + ky < nrows + 2
+        assert max(cols) < 512
+        for tap in range(9):
+            for j in range(nx):
+                base = (tap // 3 * nx + j) * 48 + tap % 3 * 16
+                assert [cols[base + c] for c in range(16)] == [(tap // 3, j, tap % 3, c) for c in range(16)]
