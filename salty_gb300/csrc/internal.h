@@ -203,7 +203,7 @@ struct TraceTuning {
     int block = 128;     // threads per block: 64, 128 or 256
     int pool = 64;       // rays a warp takes from the global cursor per refill
     int postpone = 1;    // fewest lanes that test a triangle group together (1: never postpone)
-    int regs = 56;       // register budget per thread: 64, or 56 (more resident warps: 9 blocks of 128)
+    int regs = 56;       // registers per thread of the own-test walk: 64, or 56 (9 blocks of 128 per SM)
 };
 
 }  // namespace salty
@@ -248,7 +248,7 @@ struct Tuning {
     // Paths in flight (queue capacity).  Every traversal launch ends with a tail of a few
     // long walks; freed queue slots are refilled with new samples each iteration, so the
     // launches stay full and a moderate queue already amortises the tails (1080p
-    // heightfield, 64 spp: 1,360 Mrays/s at 2^22, 1,567 at 2^24, 1,633 at 2^26).  352 bytes
+    // heightfield, 64 spp: 1,984 Mrays/s at 2^22, 2,173 at 2^24, 2,235 at 2^26).  352 bytes
     // of path state per path plus 48 bytes per sample of the per-sample buffers: about 11 GB
     // at 2^24 for a depth-12 render.
     long long wave_paths = 1ll << 24;
