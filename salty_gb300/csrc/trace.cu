@@ -43,6 +43,10 @@ constexpr int kMinPool = 16;
 // Stack entry (.y) that marks where a ray entered an instance.
 constexpr unsigned kInstMarker = 0x40000000u;
 
+__device__ __forceinline__ const float* ray_tmax(const float4* rays, int rid) {
+    return &rays[2 * (long long)rid + 1].w;
+}
+
 // SPH: leaf entries with ids from sph_base on are spheres (sphere.cu).
 template <bool ANY, bool WT, bool COUNT, int TB, bool CAP, bool INST, bool SPH>
 __global__ void __launch_bounds__(TB, CAP ? 1152 / TB : 1024 / TB)
@@ -148,7 +152,7 @@ k_trace(const Bvh8Node* __restrict__ nodes, const float4* __restrict__ tris, con
             }
         }
         bool done = false;
-        if (run) done = trav_tri_step<ANY, WT, COUNT, SPH>(s, tris, r, st, cnt, vbase, sph_base);
+        if (run) done = trav_tri_step<ANY, WT, COUNT, SPH>(s, tris, r, ray_tmax(rays, rid), st, cnt, vbase, sph_base);
         bool more = true;
         if (INST && active && !done && !s.ng_hits && !s.tg_hits && s.sp > 0 &&
             st.at(s.sp - 1).y == kInstMarker) {
@@ -303,13 +307,14 @@ k_trace_queue(const Bvh8Node* __restrict__ nodes, const float4* __restrict__ tri
                     w.dz = __shfl_sync(m, r.dz, o);
                 }
                 const float tlim = __shfl_sync(m, s.hit.t, o);
+                const int orid = WT ? __shfl_sync(m, rid, o) : 0;
                 bool h = false;
                 float t = 0.0f, u = 0.0f, v = 0.0f;
                 unsigned long long key = 0;
                 if (live) {
                     const float4* tp = tris + (size_t)e.x * kTriFloat4;
                     const float4 a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
-                    h = WT ? tri_watertight(w, a, b, c, w.tmin, tlim, t, u, v)
+                    h = WT ? tri_watertight(w, a, b, c, w.tmin, tlim, ray_tmax(rays, orid), t, u, v)
                            : tri_ref(w, a, b, c, w.tmin, tlim, tlim, t, u, v);
                     if (h) {
                         key = ((unsigned long long)__float_as_uint(t + 0.0f) << 32) | __float_as_uint(a.w);

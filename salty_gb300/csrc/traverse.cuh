@@ -122,9 +122,15 @@ __device__ __forceinline__ bool tri_ref(const TravRay& r, float4 a, float4 b, fl
 }
 
 // Watertight test (Woop, Benthin, Wald, JCGT 2013) without fused operations, so an edge
-// shared by two triangles gets the same edge function with opposite sign in both.
+// shared by two triangles gets the same edge function with opposite sign in both.  A hit has
+// its rounded t in [tmin, tfar], and T, t's numerator, not beyond det times the ray's own limit
+// (*tmax).  tfar is the closest hit so far (or *tmax): it decides by t alone.  A hit of
+// exactly that distance may have T beyond fl(tfar * det) -- one in eight does -- and
+// must still meet the lowest-id rule, whichever of two coincident triangles is tested first.
+// fl(tfar * det) lies no further than fl(*tmax * det), so *tmax is read only for those.
 __device__ __forceinline__ bool tri_watertight(const TravRay& r, float4 a, float4 b, float4 c, float tmin,
-                                               float tmax, float& t, float& u, float& v) {
+                                               float tfar, const float* __restrict__ tmax, float& t, float& u,
+                                               float& v) {
     // vertices relative to the origin, components permuted to (kx, ky, kz) with selects
     // (no dynamically indexed arrays, which would live in local memory)
     auto pick = [](float x, float y, float z, int k) { return k == 0 ? x : (k == 1 ? y : z); };
@@ -150,16 +156,16 @@ __device__ __forceinline__ bool tri_watertight(const TravRay& r, float4 a, float
     if (det == 0.0f) return false;
     const float Az = __fmul_rn(r.Sz, aZ), Bz = __fmul_rn(r.Sz, bZ), Cz = __fmul_rn(r.Sz, cZ);
     const float T = __fadd_rn(__fadd_rn(__fmul_rn(U, Az), __fmul_rn(V, Bz)), __fmul_rn(W, Cz));
-    if (det > 0.0f) {
-        if (T < __fmul_rn(tmin, det) || T > __fmul_rn(tmax, det)) return false;
-    } else {
-        if (T > __fmul_rn(tmin, det) || T < __fmul_rn(tmax, det)) return false;
-    }
+    if (det > 0.0f ? T < __fmul_rn(tmin, det) : T > __fmul_rn(tmin, det)) return false;
     const float rcp = __frcp_rn(det);
     t = __fmul_rn(T, rcp);
     u = __fmul_rn(V, rcp);
     v = __fmul_rn(W, rcp);
-    if (!(t >= tmin) || t > tmax) return false;
+    if (!(t >= tmin) || t > tfar) return false;
+    if (det > 0.0f ? T > __fmul_rn(tfar, det) : T < __fmul_rn(tfar, det)) {
+        const float lim = __fmul_rn(__ldg(tmax), det);
+        if (det > 0.0f ? T > lim : T < lim) return false;
+    }
     return true;
 }
 
@@ -357,10 +363,11 @@ __device__ __forceinline__ void trav_node_step(TravState& s, const Bvh8Node* __r
 // lowest id, every candidate bounded by the best distance so far (tmax at first).
 // Returns true when an any-hit query has its answer.
 // SPH: leaf entries with ids from sph_base on are spheres, (centre, id) (radius, 0, 0, 0).
+// tmax: where the ray's own limit stands.
 template <bool ANY, bool WATERTIGHT, bool COUNT, bool SPH = false>
 __device__ __forceinline__ bool trav_tri_step(TravState& s, const float4* __restrict__ tris, const TravRay& r,
-                                              TravStack st, TravCount& cnt, int id_off = 0,
-                                              int sph_base = 0x7fffffff) {
+                                              const float* __restrict__ tmax, TravStack st, TravCount& cnt,
+                                              int id_off = 0, int sph_base = 0x7fffffff) {
     while (s.tg_hits) {
         const unsigned k = __ffs(s.tg_hits) - 1;
         s.tg_hits &= s.tg_hits - 1;
@@ -375,7 +382,7 @@ __device__ __forceinline__ bool trav_tri_step(TravState& s, const float4* __rest
             u = 0.0f;
             v = 0.0f;
         } else {
-            h = WATERTIGHT ? tri_watertight(r, a, b, c, r.tmin, tlim, t, u, v)
+            h = WATERTIGHT ? tri_watertight(r, a, b, c, r.tmin, tlim, tmax, t, u, v)
                            : tri_ref(r, a, b, c, r.tmin, tlim, tlim, t, u, v);
         }
         if (h) {

@@ -349,3 +349,49 @@ def test_host_chunks_match_device_arrays(ctx, n):
     sc.trace_raw(torch.from_numpy(rays).cuda(), dev)
     np.testing.assert_array_equal(host.view(np.uint32), dev.cpu().numpy().view(np.uint32))
     sc.close()
+
+
+def _doubled_soup(n, seed):
+    """Every triangle twice, the ids shuffled."""
+    import salty_gb300
+    t = salty_gb300.microbench_soup(seed, n)
+    return np.ascontiguousarray(np.concatenate([t, t])[np.random.default_rng(seed).permutation(2 * n)])
+
+
+# Coincident triangles: the lowest id wins under either test, whichever of the two a walk
+# tests first (the queueing walk's order depends on the rays that share a warp), so calls repeat
+# bit for bit.  More rays than lanes, so that the deep trees take the queueing walk.
+@pytest.mark.parametrize("n", [3000, 100000])
+@pytest.mark.parametrize("watertight", [False, True])
+def test_coincident_triangles_give_the_lowest_id(ctx, oracle, n, watertight):
+    import salty_gb300
+    import torch
+    tris = _doubled_soup(n, 23)
+    sc = _scene(ctx, tris)
+    assert n < 100000 or sc.info["depth"] >= 7
+    rays = salty_gb300.microbench_rays(6, 1024 * torch.cuda.get_device_properties(0).multi_processor_count + 77, 1e-4)
+    res = [sc.trace(rays, watertight=watertight) for _ in range(3)]
+    oid, ot, _, _ = oracle.trace(tris, rays, mode=1 if watertight else 0)
+    for r in res:
+        np.testing.assert_array_equal(r.ids, oid)
+        np.testing.assert_array_equal(r.t[oid >= 0], ot[oid >= 0])
+        np.testing.assert_array_equal(r.u, res[0].u)
+        np.testing.assert_array_equal(r.v, res[0].v)
+    sc.close()
+
+
+# A watertight hit at its ray's own limit: kept when both T / det as the oracle compares it and
+# the rounded t are within the limit; limits at the hit distances and one unit in the last
+# place either side.
+@pytest.mark.parametrize("step", [-1, 0, 1])
+def test_watertight_hits_at_the_ray_limit(ctx, oracle, step):
+    import salty_gb300
+    tris = _doubled_soup(20000, 29)
+    sc = _scene(ctx, tris)
+    rays = salty_gb300.microbench_rays(8, 40000, 1e-4)
+    _, ot, _, _ = oracle.trace(tris, rays, mode=1)
+    rays[:, 7] = np.where(np.isinf(ot), ot, (ot.view(np.int32) + step).view(np.float32))
+    oid, ot, _, _ = oracle.trace(tris, rays, mode=1)
+    res = sc.trace(rays, watertight=True)
+    np.testing.assert_array_equal(res.ids, np.where(ot <= rays[:, 7], oid, -1))
+    sc.close()
