@@ -200,7 +200,8 @@ k_trace(const Bvh8Node* __restrict__ nodes, const float4* __restrict__ tris, con
 // new rays kRefill at a time, since a refill costs the warp about a node step and a trip to
 // memory however many lanes it fills (1 at a time: 5 % slower).
 // Best hits live in shared memory as (t, id) keys: t >= 0, so the bits order as the floats do,
-// and equal distances go to the lowest id.
+// and equal distances go to the lowest id.  Any hit: the first of the ray's own walk, as in
+// k_trace, so the answer does not depend on the rays that share the warp.
 // Bound: instruction issue and the latency of node fetches from L2.  64 registers, 32 warps per
 // SM, whatever the tuning's budget (56, 72 and 80 registers: 11, 1 and 1 % slower over 1080p
 // terrain and 4.2M rays).  Measured (GB300), against k_trace: 1080p terrain at 8 spp 27.4 ->
@@ -316,13 +317,20 @@ k_trace_queue(const Bvh8Node* __restrict__ nodes, const float4* __restrict__ tri
                     const float4 a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
                     h = WT ? tri_watertight(w, a, b, c, w.tmin, tlim, ray_tmax(rays, orid), t, u, v)
                            : tri_ref(w, a, b, c, w.tmin, tlim, tlim, t, u, v);
-                    if (h) {
-                        key = ((unsigned long long)__float_as_uint(t + 0.0f) << 32) | __float_as_uint(a.w);
-                        atomicMin(&keys[o], key);
-                    }
+                    if (h) key = ((unsigned long long)__float_as_uint(t + 0.0f) << 32) | __float_as_uint(a.w);
                 }
-                __syncwarp();
-                if (h && keys[o] == key) uvs[o] = make_uint2(__float_as_uint(u), __float_as_uint(v));
+                if (ANY) {
+                    // a ray's pairs stand in the order of its walk: the first that hits is its answer
+                    const unsigned hs = __ballot_sync(m, h);
+                    if (h && lane == __ffs(__match_any_sync(hs, o)) - 1 && (unsigned)keys[o] == 0xffffffffu) {
+                        keys[o] = key;
+                        uvs[o] = make_uint2(__float_as_uint(u), __float_as_uint(v));
+                    }
+                } else {
+                    if (h) atomicMin(&keys[o], key);
+                    __syncwarp();
+                    if (h && keys[o] == key) uvs[o] = make_uint2(__float_as_uint(u), __float_as_uint(v));
+                }
                 __syncwarp();
                 if (pending) s.hit.t = __uint_as_float((unsigned)(keys[lane] >> 32));
             }

@@ -395,3 +395,30 @@ def test_watertight_hits_at_the_ray_limit(ctx, oracle, step):
     res = sc.trace(rays, watertight=True)
     np.testing.assert_array_equal(res.ids, np.where(ot <= rays[:, 7], oid, -1))
     sc.close()
+
+
+def _whole_and_pieces(sc, rays, **kw):
+    """The same rays in one call and in calls of no more rays than lanes: the deep trees'
+    queueing walk, and the walk in which lanes test their own triangles."""
+    import torch
+    lanes = 1024 * torch.cuda.get_device_properties(0).multi_processor_count
+    assert len(rays) > lanes
+    whole = sc.trace(rays, **kw)
+    parts = [sc.trace(rays[k:k + lanes], **kw) for k in range(0, len(rays), lanes)]
+    bits = lambda r: np.stack([r.t.view(np.int32), r.ids, r.u.view(np.int32), r.v.view(np.int32)], 1)
+    return bits(whole), np.concatenate([bits(p) for p in parts])
+
+
+# Any hit returns one and the same hit of a ray, the first of its walk, in either walk and in
+# every call, among coincident triangles too.
+@pytest.mark.parametrize("watertight", [False, True])
+def test_any_hit_is_the_same_hit_in_every_call(ctx, watertight):
+    import salty_gb300
+    sc = _scene(ctx, _doubled_soup(400000, 31))
+    assert sc.info["depth"] >= (7 if watertight else 8)
+    rays = salty_gb300.microbench_rays(9, 300001, 1e-4)
+    rays[::3, 7] = 2.0
+    for _ in range(2):
+        whole, pieces = _whole_and_pieces(sc, rays, any_hit=True, watertight=watertight)
+        np.testing.assert_array_equal(whole, pieces)
+    sc.close()
