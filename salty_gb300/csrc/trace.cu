@@ -199,7 +199,7 @@ k_trace(const Bvh8Node* __restrict__ nodes, const float4* __restrict__ tris, con
 // pairs as lanes are walking (half or a quarter as many: 1 and 5 % slower), and idle lanes take
 // new rays kRefill at a time, since a refill costs the warp about a node step and a trip to
 // memory however many lanes it fills (1 at a time: 5 % slower).
-// Best hits live in shared memory as (t, id) keys: t >= 0, so the bits order as the floats do,
+// Best hits live in shared memory as keys (hit_key): t >= 0, so the bits order as the floats do,
 // and equal distances go to the lowest id.  Any hit: the first of the ray's own walk, as in
 // k_trace, so the answer does not depend on the rays that share the warp.
 // Bound: instruction issue and the latency of node fetches from L2.  64 registers, 32 warps per
@@ -210,6 +210,13 @@ k_trace(const Bvh8Node* __restrict__ nodes, const float4* __restrict__ tris, con
 // gains nothing: dispatch_flags.
 constexpr int kQueue = 64;    // pairs per warp: fewer than 32 before a push of at most 32
 constexpr int kRefill = 6;    // idle lanes that start a refill
+constexpr unsigned kNoHit = 0xffffffffu;  // low word of a ray's key before its first hit
+
+// t, the id, and t's sign in the last bit: a hit at -0 is as near as one at +0 (ids are below 2^31).
+__device__ __forceinline__ unsigned long long hit_key(float t, float id_bits) {
+    const unsigned b = __float_as_uint(t);
+    return ((unsigned long long)(b & 0x7fffffffu) << 32) | (__float_as_uint(id_bits) << 1) | (b >> 31);
+}
 
 template <bool ANY, bool WT, int TB>
 __global__ void __launch_bounds__(TB, 1024 / TB)
@@ -263,7 +270,7 @@ k_trace_queue(const Bvh8Node* __restrict__ nodes, const float4* __restrict__ tri
                 const float4 ra = __ldcs(rays + 2 * rid), rb = __ldcs(rays + 2 * rid + 1);
                 make_trav_ray(r, ra.x, ra.y, ra.z, ra.w, rb.x, rb.y, rb.z);
                 trav_init(s, r, rb.w, roots ? (unsigned)__ldcs(roots + rid) : 0u);
-                keys[lane] = ((unsigned long long)__float_as_uint(s.hit.t) << 32) | 0xffffffffu;
+                keys[lane] = ((unsigned long long)__float_as_uint(s.hit.t) << 32) | kNoHit;
                 walking = true;
             }
             pool_next = min(pool_end, pool_next + __popc(idle_mask));
@@ -317,12 +324,12 @@ k_trace_queue(const Bvh8Node* __restrict__ nodes, const float4* __restrict__ tri
                     const float4 a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
                     h = WT ? tri_watertight(w, a, b, c, w.tmin, tlim, ray_tmax(rays, orid), t, u, v)
                            : tri_ref(w, a, b, c, w.tmin, tlim, tlim, t, u, v);
-                    if (h) key = ((unsigned long long)__float_as_uint(t + 0.0f) << 32) | __float_as_uint(a.w);
+                    if (h) key = hit_key(t, a.w);
                 }
                 if (ANY) {
                     // a ray's pairs stand in the order of its walk: the first that hits is its answer
                     const unsigned hs = __ballot_sync(m, h);
-                    if (h && lane == __ffs(__match_any_sync(hs, o)) - 1 && (unsigned)keys[o] == 0xffffffffu) {
+                    if (h && lane == __ffs(__match_any_sync(hs, o)) - 1 && (unsigned)keys[o] == kNoHit) {
                         keys[o] = key;
                         uvs[o] = make_uint2(__float_as_uint(u), __float_as_uint(v));
                     }
@@ -335,7 +342,7 @@ k_trace_queue(const Bvh8Node* __restrict__ nodes, const float4* __restrict__ tri
                 if (pending) s.hit.t = __uint_as_float((unsigned)(keys[lane] >> 32));
             }
             qn = 0;
-            if (ANY && pending && (unsigned)keys[lane] != 0xffffffffu) {
+            if (ANY && pending && (unsigned)keys[lane] != kNoHit) {
                 walking = false;
                 s.tg_hits = 0;
             }
@@ -344,9 +351,10 @@ k_trace_queue(const Bvh8Node* __restrict__ nodes, const float4* __restrict__ tri
         if (rid >= 0 && !walking && !pending && !s.tg_hits) {
             const unsigned long long key = keys[lane];
             float4 h = make_float4(INFINITY, __int_as_float(-1), 0.0f, 0.0f);
-            if ((unsigned)key != 0xffffffffu) {
+            const unsigned low = (unsigned)key;
+            if (low != kNoHit) {
                 const uint2 uv = uvs[lane];
-                h = make_float4(__uint_as_float((unsigned)(key >> 32)), __int_as_float((int)(unsigned)key),
+                h = make_float4(__uint_as_float((unsigned)(key >> 32) | (low << 31)), __uint_as_float(low >> 1),
                                 __uint_as_float(uv.x), __uint_as_float(uv.y));
             }
             __stcs(hits + rid, h);

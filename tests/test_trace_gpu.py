@@ -422,3 +422,25 @@ def test_any_hit_is_the_same_hit_in_every_call(ctx, watertight):
         whole, pieces = _whole_and_pieces(sc, rays, any_hit=True, watertight=watertight)
         np.testing.assert_array_equal(whole, pieces)
     sc.close()
+
+
+# Rays from points on the triangles themselves: distances of 0, of either sign, and a few
+# 1e-7, in both walks and under both tests.
+@pytest.mark.parametrize("watertight", [False, True])
+def test_rays_leaving_surfaces(ctx, watertight):
+    import salty_gb300
+    tris = salty_gb300.microbench_soup(37, 300000)
+    sc = _scene(ctx, tris)
+    assert sc.info["depth"] >= 8
+    rng = np.random.default_rng(3)
+    n = 1 << 20
+    w = rng.dirichlet((1, 1, 1), n).astype(np.float32)
+    rays = np.zeros((n, 8), np.float32)
+    rays[:, :3] = (tris.reshape(-1, 3, 3)[rng.integers(0, len(tris), n)] * w[:, :, None]).sum(1)
+    d = rng.normal(size=(n, 3))
+    rays[:, 4:7] = d / np.linalg.norm(d, axis=1, keepdims=True)
+    rays[:, 7] = np.inf
+    whole, pieces = _whole_and_pieces(sc, rays, watertight=watertight)
+    assert np.count_nonzero(pieces[:, 0] == np.float32(-0.0).view(np.int32)) > 50
+    np.testing.assert_array_equal(whole, pieces)
+    sc.close()
