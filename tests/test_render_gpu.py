@@ -304,3 +304,27 @@ def test_film_read_out_rounding(ctx, samples, scale):
         v = v.astype(np.float32)
     np.testing.assert_allclose(r["var"], v, rtol=2.0 ** -23, atol=2.0 ** -149)
     sc.close()
+
+
+# The variance of nearly constant pixels, down to 2^-24 of the squared mean: the exact quotient
+# of the sums rounded once (0.5 units in the last place, and 0.01 for the rounded factor), or,
+# where the sums say less than nothing, zero.
+@pytest.mark.parametrize("samples", [2, 3, 49, 1000, (1 << 24) - 1])
+@pytest.mark.parametrize("spread", [-16, -20, -22, -23, -24])
+def test_film_variance_of_nearly_constant_pixels(ctx, samples, spread):
+    from fractions import Fraction
+    from salty_gb300 import scenes
+    rng = np.random.default_rng(samples - spread)
+    w, h = 41, 3
+    s = (rng.lognormal(0.0, 1.0, (h, w, 3)) * samples).astype(np.float32).astype(np.float64)
+    q = ((s / samples) ** 2 * samples * (1.0 + 2.0 ** spread * rng.uniform(0.5, 1.0, s.shape))).astype(np.float32)
+    q = q.astype(np.float64)
+    sc = scenes.upload(ctx, scenes.cornell())
+    sc.build()
+    sc.restore({"sum": s, "sumsq": q, "comp": None, "aov": None, "samples": samples}, w, h)
+    var = sc.read(w, h)["var"].astype(np.float64)
+    sc.close()
+    for v, si, qi in zip(var.ravel(), s.ravel(), q.ravel()):
+        x = max((Fraction(qi) * samples - Fraction(si) ** 2) / (samples ** 2 * (samples - 1)), Fraction(0))
+        ulp = Fraction(float(np.spacing(np.float32(float(x)))))
+        assert abs(Fraction(v) - x) <= Fraction(51, 100) * ulp, (v, float(x))
