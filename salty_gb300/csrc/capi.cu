@@ -131,7 +131,7 @@ salty_status salty_ctx_create(salty_ctx** out, int device) {
         return SALTY_ERR_CUDA;
     }
     for (auto& e : c->ev) cudaEventCreate(&e);
-    if (c->counters.ensure(64) != cudaSuccess || c->status.ensure(16) != cudaSuccess) {
+    if (c->counters.ensure(64) != cudaSuccess || c->status.ensure(16) != cudaSuccess || tonemap_prepare(c) != SALTY_OK) {
         salty_ctx_destroy(c);
         return SALTY_ERR_OOM;
     }

@@ -343,6 +343,7 @@ salty_status film_outputs(salty_ctx* ctx, salty_scene* sc, const salty_render_op
                           float* d_mean, float* d_var, uint8_t* d_srgb);
 salty_status film_records(salty_ctx* ctx, salty_scene* sc, void* d_rec);
 // post.cu
+salty_status tonemap_prepare(salty_ctx* ctx);
 salty_status tonemap_device(salty_ctx* ctx, int type, int w, int h, const float* d_rgb,
                             float* d_out, uint8_t* d_srgb, int ref_oetf, float* ave, float* mx);
 salty_status nlm_ref_device(salty_ctx* ctx, int w, int h, float coeff, const float* d_in,

@@ -610,6 +610,17 @@ salty_status launch_nlm_var_cols(salty_ctx* ctx, int w, int h, int R, float k2, 
 
 }  // namespace
 
+// Blocks of the luminance reduction: more cost more in tickets than they hide (8 per SM: 2 us).
+static int lum_blocks(const salty_ctx* ctx) { return ctx->num_sms * 3; }
+
+// The reduction's scratch (19 KB), made with the context so that no tonemap allocates it.
+salty_status tonemap_prepare(salty_ctx* ctx) {
+    const size_t bytes = sizeof(LumScratch) + (size_t)lum_blocks(ctx) * sizeof(LumAcc);
+    SALTY_TRY_CUDA(ctx->err, ctx->lum_ws.ensure(bytes));
+    SALTY_TRY_CUDA(ctx->err, cudaMemsetAsync(ctx->lum_ws.p, 0, bytes, ctx->stream));
+    return SALTY_OK;
+}
+
 // One round trip: the reduction derives the map's parameters on the device, the map follows
 // without waiting, and the host then checks the one value that its own arithmetic defines, the
 // exponential of the mean (expf).  Where the device's differs in the last place, or where an
@@ -621,12 +632,6 @@ salty_status tonemap_device(salty_ctx* ctx, int type, int w, int h, const float*
     auto& E = ctx->err;
     cudaStream_t st = ctx->stream;
     const long long npx = (long long)w * h;
-    const int cap = ctx->num_sms * 3;  // more blocks cost more in tickets than they hide (8 per SM: 2 us)
-    const size_t bytes = sizeof(LumScratch) + (size_t)cap * sizeof(LumAcc);
-    if (!ctx->lum_ws.p) {
-        SALTY_TRY_CUDA(E, ctx->lum_ws.ensure(bytes));
-        SALTY_TRY_CUDA(E, cudaMemsetAsync(ctx->lum_ws.p, 0, bytes, st));
-    }
     LumScratch* sc = reinterpret_cast<LumScratch*>(ctx->lum_ws.p);
     LumResult* res = static_cast<LumResult*>(ctx->pinned);
     TmParams p{};
@@ -642,7 +647,7 @@ salty_status tonemap_device(salty_ctx* ctx, int type, int w, int h, const float*
     }
     const bool vec = aligned_to(d_rgb, 16);
     const long long need = ((vec ? (npx + 3) / 4 : npx) + kRedBlock - 1) / kRedBlock;
-    k_lum<<<(unsigned)std::min<long long>(cap, need), kRedBlock, 0, st>>>(d_rgb, npx, vec, p, sc, res);
+    k_lum<<<(unsigned)std::min<long long>(lum_blocks(ctx), need), kRedBlock, 0, st>>>(d_rgb, npx, vec, p, sc, res);
     auto apart = [&](const void* q, size_t len) {
         const auto a = reinterpret_cast<uintptr_t>(d_rgb), b = reinterpret_cast<uintptr_t>(q);
         return !q || b >= a + (size_t)npx * 12 || b + len <= a;

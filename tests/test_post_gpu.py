@@ -171,3 +171,23 @@ def test_variance_nlm_on_tall_tiles(ctx, oracle, h, w, patch_r):
     var = (0.02 * rng.random((h, w, 3))).astype(np.float32)
     out = ctx.nlm(img, var, search_r=2, patch_r=patch_r, k=0.6)
     np.testing.assert_allclose(out, oracle.nlm_var(img, var, 2, patch_r, 0.6), rtol=1e-4, atol=1e-5)
+
+
+# No tonemap of device arrays allocates device memory, the first of a context included.  An
+# allocation of 19 KB hides in the driver's 2 MB blocks; those of 256 contexts do not.
+def test_first_tonemap_allocates_nothing(salty_lib):
+    import torch
+    import salty_gb300
+    img = torch.rand((33, 47, 3), device="cuda")
+    out = torch.empty_like(img)
+    many = [salty_gb300.Context(0) for _ in range(257)]
+    try:
+        _tonemap_device(many[0], img, out, None, 0)  # loads the kernels
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        for c in many[1:]:
+            _tonemap_device(c, img, out, None, 0)
+        assert torch.cuda.mem_get_info()[0] == free
+    finally:
+        for c in many:
+            c.close()
