@@ -173,6 +173,67 @@ def test_variance_nlm_on_tall_tiles(ctx, oracle, h, w, patch_r):
     np.testing.assert_allclose(out, oracle.nlm_var(img, var, 2, patch_r, 0.6), rtol=1e-4, atol=1e-5)
 
 
+# The default window, the smallest and the largest radius of the wide tile's kernel, on 12-row
+# tiles (more tiles than SMs), against the direct sums in 64 bits.  Bounds as above.
+@pytest.mark.parametrize("search_r,patch_r", [(10, 3), (10, 1), (11, 3), (11, 2), (32, 3), (32, 1)])
+def test_variance_nlm_search_radii_on_tall_tiles(ctx, search_r, patch_r):
+    import torch
+    import torch.nn.functional as F
+    h, w, k = 397, 157, 0.6
+    rng = np.random.default_rng(100 * search_r + patch_r)
+    img = rng.random((h, w, 3), dtype=np.float32)
+    var = (0.02 * rng.random((h, w, 3)) + 1e-3).astype(np.float32)
+    out = ctx.nlm(img, var, search_r=search_r, patch_r=patch_r, k=k)
+    R, P = search_r, patch_r
+    pad = lambda a: F.pad(torch.from_numpy(a).cuda().double().permute(2, 0, 1)[None], (R + P,) * 4, mode="replicate")[0]
+    I, V = pad(img), pad(var)
+    cut = lambda a, dy, dx, e: a[:, R + P + dy - e:R + P + dy + h + e, R + P + dx - e:R + P + dx + w + e]
+    a, va = cut(I, 0, 0, P), cut(V, 0, 0, P)
+    acc, tot = torch.zeros((3, h, w), dtype=torch.float64, device="cuda"), torch.zeros((h, w), dtype=torch.float64, device="cuda")
+    for dy in range(-R, R + 1):
+        for dx in range(-R, R + 1):
+            b, vb = cut(I, dy, dx, P), cut(V, dy, dx, P)
+            d = (((a - b) ** 2 - (va + torch.minimum(va, vb))) / (1e-10 + k * k * (va + vb))).sum(0)
+            wt = torch.exp(-(F.avg_pool2d(d[None, None], 2 * P + 1, stride=1)[0, 0] / 3.0).clamp_min(0.0))
+            acc += wt * cut(I, dy, dx, 0)
+            tot += wt
+    np.testing.assert_allclose(out, (acc / tot).permute(1, 2, 0).cpu().numpy(), rtol=1e-4, atol=1e-5)
+
+
+def _aces_fp32(x):
+    """ACESFilm (src/s3d_tonemapper.cpp:117-130), every operation rounded to FP32."""
+    f = np.float32
+    a, b, c, d, e, g, k = f(2.51), f(0.03), f(2.43), f(0.59), f(0.14), f(0.665406), f(12.0)
+    with np.errstate(all="ignore"):
+        y = (x * (a * x * g / k + b)) / (x * g / k * (c * x * g + d) + e)
+    return np.where(y < 0, f(0), np.where(y > 1, f(1), y))
+
+
+# ACES bit for bit against the FP32 restatement with true quotients: every mantissa of a binade,
+# and scaled values on both sides of the range in which a twelfth is taken by a corrected product
+# (2^-90 from a bright channel beside tiny ones, 2^90 from a few bright pixels among black ones).
+@pytest.mark.parametrize("values", ["mantissas", "tiny", "huge"])
+def test_aces_equals_the_fp32_restatement(ctx, values):
+    import torch
+    f = np.float32
+    if values == "mantissas":
+        img = (np.arange(1 << 23, dtype=np.uint32) + np.uint32(0x3F800000)).view(f)[:3 * ((1 << 23) // 3)].reshape(1, -1, 3)
+    elif values == "tiny":
+        e = np.linspace(-100.0, -80.0, 3000)
+        img = np.stack([np.ones_like(e), 2.0 ** e, 2.0 ** -e[::-1] * 2.0 ** -180], 1).astype(f)[None]
+    else:
+        img = np.zeros((100, 1000, 3), f)
+        img[0, :, :] = (2.0 ** np.linspace(68.0, 84.0, 3000)).reshape(1000, 3)
+    d = torch.from_numpy(np.ascontiguousarray(img)).cuda()
+    out = torch.empty_like(d)
+    ave, _ = _tonemap_device(ctx, d, out, None, 2)
+    x = img * (f(0.27) / ave)
+    if values != "mantissas":
+        m = np.abs(x[x != 0])
+        assert np.count_nonzero((m > 2.0 ** 88) & (m < 2.0 ** 92) | (m > 2.0 ** -92) & (m < 2.0 ** -88)) > 300
+    np.testing.assert_array_equal(out.cpu().numpy(), _aces_fp32(x))
+
+
 # No tonemap of device arrays allocates device memory, the first of a context included.  An
 # allocation of 19 KB hides in the driver's 2 MB blocks; those of 256 contexts do not.
 def test_first_tonemap_allocates_nothing(salty_lib):
