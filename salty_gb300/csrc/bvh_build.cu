@@ -1092,7 +1092,7 @@ inline float host_o2f(int i) {
 
 }  // namespace
 
-salty_status build_bvh(salty_ctx* ctx, salty_scene* sc, const salty_build_opts& opts) {
+static salty_status build_scene(salty_ctx* ctx, salty_scene* sc, const salty_build_opts& opts) {
     if (sc->n_inst > 0) return build_instanced(ctx, sc, opts);
     if (sc->n_sph > 0) return build_with_spheres(ctx, sc, opts);
     if (sc->n_tris <= 0) return ctx->err.fail(SALTY_ERR_INVALID_ARG, "scene has no triangles");
@@ -1100,6 +1100,16 @@ salty_status build_bvh(salty_ctx* ctx, salty_scene* sc, const salty_build_opts& 
         return ctx->err.fail(SALTY_ERR_CAPACITY, "too many triangles (%lld)", (long long)sc->n_tris);
     float box[6];
     return build_bvh_tris(ctx, sc->pos.p, (int)sc->n_tris, opts, sc->bvh, box);
+}
+
+// The workspace outlives a build only for a scene that is built again (a changing scene), and
+// goes with that scene: a scene built once leaves nothing behind.
+salty_status build_bvh(salty_ctx* ctx, salty_scene* sc, const salty_build_opts& opts) {
+    const bool again = sc->bvh.generation != 0;
+    const salty_status s = build_scene(ctx, sc, opts);
+    if (again && s == SALTY_OK) ctx->build_ws_owner = sc;
+    if (!ctx->build_ws_owner) ctx->build_ws.release();
+    return s;
 }
 
 salty_status build_bvh_tris(salty_ctx* ctx, const float* d_pos, int n, const salty_build_opts& opts, Bvh& out,
@@ -1112,8 +1122,8 @@ salty_status build_bvh_tris(salty_ctx* ctx, const float* d_pos, int n, const sal
     prm.trav_cost = opts.trav_cost;
     cudaStream_t st = ctx->stream;
 
-    // Workspace: one allocation, carved up.  The context keeps it for the next build up to
-    // kKeepBuildBytes (about 2M triangles); a larger one is given back after its build.
+    // Workspace: one allocation, carved up; up to kKeepBuildBytes (about 2M triangles) the
+    // context's (build_bvh), a larger one is given back at the end.
     const size_t max_top = (size_t)n / (kSub + 1) + 2;  // tasks of one top level
     const size_t max_item = (size_t)n / kChunk + 1 + max_top;
     size_t total = 0;

@@ -401,6 +401,10 @@ void salty_scene_destroy(salty_ctx* ctx, salty_scene* scene) {
     if (ctx) {
         cudaSetDevice(ctx->device);
         cudaStreamSynchronize(ctx->stream);
+        if (ctx->build_ws_owner == scene) {
+            ctx->build_ws_owner = nullptr;
+            ctx->build_ws.release();
+        }
     }
     delete scene;
 }

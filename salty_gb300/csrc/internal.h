@@ -314,6 +314,7 @@ struct salty_ctx {
     salty::DevBuf<unsigned char> slots;  // SceneSlot table of the current render
     std::vector<salty::ResidentBlocks> resident;  // a few entries: kernels x stack depths used
     salty::DevBuf<unsigned char> build_ws;  // BVH build workspace (bvh_build.cu)
+    const salty_scene* build_ws_owner = nullptr;  // the scene it is kept for, null: given back after each build
     salty::DevBuf<unsigned char> lum_ws;    // tonemapping's partial sums and parameters (post.cu)
 };
 

@@ -444,3 +444,31 @@ def test_rays_leaving_surfaces(ctx, watertight):
     assert np.count_nonzero(pieces[:, 0] == np.float32(-0.0).view(np.int32)) > 50
     np.testing.assert_array_equal(whole, pieces)
     sc.close()
+
+
+# A scene built once leaves no build workspace behind; one built again keeps a bounded one,
+# which goes with the scene.  (Sizes to the driver's 2 MB blocks.)
+def test_build_workspace_is_given_back(salty_lib):
+    import salty_gb300
+    import torch
+    free = lambda: torch.cuda.mem_get_info()[0]
+    n, slack = 1000000, 8 << 20
+    tris = salty_gb300.microbench_soup(41, n)
+    with salty_gb300.Context(0) as c:
+        w = c.upload_scene(tris[:1000])
+        w.build()                              # loads the kernels
+        w.close()
+        before = free()
+        s = c.upload_scene(tris)
+        uploaded = free()
+        s.build()
+        tree = uploaded - free()
+        assert tree <= (n + 1) * 80 + n * 48 + slack
+        s.build()
+        kept = uploaded - free() - tree
+        assert kept <= (512 << 20) + slack
+        other = c.upload_scene(tris[:2000])
+        other.build()
+        other.close()
+        s.close()
+        assert before - free() <= slack
