@@ -529,7 +529,9 @@ k_nlm_var_cols(const float* __restrict__ rgb, const float* __restrict__ var, int
     float2* t1 = t0 + rows * S;
     float2* t2 = t1 + rows * S;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int bx = blockIdx.x * (32 - 2 * P), by = blockIdx.y * ROWS;
+    // blocks in one dimension: the second has room for 65,535 only
+    const int tiles_x = (w + 31 - 2 * P) / (32 - 2 * P);
+    const int bx = (int)(blockIdx.x % tiles_x) * (32 - 2 * P), by = (int)(blockIdx.x / tiles_x) * ROWS;
     for (int i = threadIdx.x; i < rows * cols; i += 32 * kNlmWarps) {
         const int ty = i / cols, tx = i - ty * cols;
         const size_t g = ((size_t)clampi(by - P - R + ty, 0, h - 1) * w + clampi(bx - P - R + tx, 0, w - 1)) * 3;
@@ -595,15 +597,15 @@ k_nlm_var_cols(const float* __restrict__ rgb, const float* __restrict__ var, int
 template <int P, int RM, int ROWS>
 salty_status launch_nlm_var_cols(salty_ctx* ctx, int w, int h, int R, float k2, float norm, const float* rgb,
                                  const float* var, float* out) {
-    const dim3 grid((w + 31 - 2 * P) / (32 - 2 * P), (h + ROWS - 1) / ROWS);
+    const long long tiles = (long long)((w + 31 - 2 * P) / (32 - 2 * P)) * ((h + ROWS - 1) / ROWS);
     // fewer tiles than SMs: shorter ones, more of them (200 x 150, radius 3: 89 -> 72 us)
-    if (ROWS > 8 && (long long)grid.x * grid.y <= ctx->num_sms)
+    if (ROWS > 8 && tiles <= ctx->num_sms)
         return launch_nlm_var_cols<P, RM, 8>(ctx, w, h, R, k2, norm, rgb, var, out);
     const size_t tile = (size_t)(ROWS + 2 * P + 2 * R) * (32 + 2 * RM) * 3 * sizeof(float2);
     const size_t smem = std::max(tile, (size_t)ROWS * 4 * 32 * sizeof(float));
     auto kern = k_nlm_var_cols<P, RM, ROWS>;
     SALTY_TRY_CUDA(ctx->err, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<grid, 32 * kNlmWarps, smem, ctx->stream>>>(rgb, var, w, h, R, k2, norm, out);
+    kern<<<(unsigned)tiles, 32 * kNlmWarps, smem, ctx->stream>>>(rgb, var, w, h, R, k2, norm, out);
     SALTY_TRY_CUDA(ctx->err, cudaGetLastError());
     return SALTY_OK;
 }

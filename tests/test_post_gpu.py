@@ -252,3 +252,19 @@ def test_first_tonemap_allocates_nothing(salty_lib):
     finally:
         for c in many:
             c.close()
+
+
+# An image of more rows than a grid's second dimension has tiles for, against its own bands.
+def test_variance_nlm_of_a_very_tall_image(ctx):
+    import torch
+    h, w, R, P = 800000, 3, 1, 1
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    img = torch.rand((h, w, 3), device="cuda", generator=g)
+    var = 0.02 * torch.rand((h, w, 3), device="cuda", generator=g)
+    out, band = torch.empty_like(img), torch.empty((600, w, 3), device="cuda")
+    ctx.nlm(img, var, R, P, out=out)
+    for y in (0, 400000, h - 600):
+        ctx.nlm(img[y:y + 600].contiguous(), var[y:y + 600].contiguous(), R, P, out=band)
+        lo, hi = (0 if y == 0 else 2), (600 if y == h - 600 else 598)  # rows that see the band alone
+        torch.testing.assert_close(out[y + lo:y + hi], band[lo:hi], rtol=1e-5, atol=1e-6)
