@@ -537,7 +537,8 @@ struct FlipSet {
 __global__ void __launch_bounds__(256) k_output_images(const bf16* __restrict__ out, const uint4* __restrict__ rec, int W,
                                                        int H, int Wp, int Hp, FlipSet fs, float weight, int first,
                                                        float* __restrict__ rgb) {
-    const int px = blockIdx.x * 16 + (threadIdx.x & 15), py = blockIdx.y * 16 + (threadIdx.x >> 4);
+    const int bw = (W + 15) / 16;
+    const int px = (int)(blockIdx.x % bw) * 16 + (threadIdx.x & 15), py = (int)(blockIdx.x / bw) * 16 + (threadIdx.x >> 4);
     if (px >= W || py >= H) return;
     const long long p = (long long)py * W + px;
     const uint2 xr = *reinterpret_cast<const uint2*>(rec + 2 * p);
@@ -614,16 +615,16 @@ __global__ void k_weights_to_bf16(const float* __restrict__ w, int Cout, int Cin
 // are read from L2.
 __global__ void __launch_bounds__(256) k_place_inputs(const uint4* __restrict__ rec, int W, int H, int Wp, int Hp,
                                                       FlipSet fs, uint4* __restrict__ x) {
-    const int half = threadIdx.x & 1, t = threadIdx.x >> 1, f = fs.flip[blockIdx.z];
-    // blocks run along the output's rows: (u, v) is the output pixel
-    const int Wo = (f & 4) ? Hp : Wp, Ho = (f & 4) ? Wp : Hp;
-    const int u = blockIdx.x * 16 + (t & 15), v = blockIdx.y * 8 + (t >> 4);
+    const int half = threadIdx.x & 1, t = threadIdx.x >> 1, f = fs.flip[blockIdx.y];
+    // blocks run along the output's rows, in one grid dimension: (u, v) is the output pixel
+    const int Wo = (f & 4) ? Hp : Wp, Ho = (f & 4) ? Wp : Hp, bw = Wo / 16;
+    const int u = (int)(blockIdx.x % bw) * 16 + (t & 15), v = (int)(blockIdx.x / bw) * 8 + (t >> 4);
     if (u >= Wo || v >= Ho) return;
     const int px = (f & 4) ? v : u, py = (f & 4) ? u : v;
     int sx = px < W ? px : max(2 * W - 2 - px, 0), sy = py < H ? py : max(2 * H - 2 - py, 0);
     if (f & 1) sx = W - 1 - sx;
     if (f & 2) sy = H - 1 - sy;
-    x[(((long long)blockIdx.z * Ho + v) * Wo + u) * 2 + half] = __ldg(rec + ((long long)sy * W + sx) * 2 + half);
+    x[(((long long)blockIdx.y * Ho + v) * Wo + u) * 2 + half] = __ldg(rec + ((long long)sy * W + sx) * 2 + half);
 }
 
 inline int gsz(long long n, int block = 256) {
@@ -1185,11 +1186,11 @@ salty_status salty_denoise_unet_ensemble(salty_ctx* ctx, salty_unet* net, salty_
         const bool tr = (k0 & 4) != 0;  // the transposed frames: Hp wide, Wp tall
         const int h = tr ? Wp : Hp, w = tr ? Hp : Wp;
         SALTY_TRY(ensure_workspace(ctx, u, per, h, w));
-        k_place_inputs<<<dim3(w / 16, (h + 7) / 8, per), 256, 0, ctx->stream>>>(
+        k_place_inputs<<<dim3((w / 16) * ((h + 7) / 8), per), 256, 0, ctx->stream>>>(
             rec, W, H, Wp, Hp, fs, reinterpret_cast<uint4*>(u.act.p + u.act_off[T_X]));
         Fwd F;
         SALTY_TRY(forward(ctx, u, nullptr, per, h, w, F));
-        k_output_images<<<dim3((W + 15) / 16, (H + 15) / 16), 256, 0, ctx->stream>>>(
+        k_output_images<<<((W + 15) / 16) * ((H + 15) / 16), 256, 0, ctx->stream>>>(
             F.t[T_OUT], rec, W, H, Wp, Hp, fs, 1.0f / (float)mirrors, k0 == 0, img);
     }
     SALTY_TRY_CUDA(ctx->err, cudaGetLastError());

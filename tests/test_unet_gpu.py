@@ -301,3 +301,27 @@ def test_short_strips_give_the_same_output(ctx, h, w):
     for i in (0, 23, 39):
         np.testing.assert_array_equal(net.forward(f[i:i + 1])[0], many[i])
     net.close()
+
+
+# A film of more rows than a grid's second dimension has blocks for, against a band of it: rows
+# further from the band's ends than the network sees are the same bits.
+def test_denoise_of_a_very_tall_film(ctx):
+    import salty_gb300
+    from salty_gb300 import scenes
+    w, h, n = 16, 600000, 16
+    y0, y1, margin = 399984, 404080, 512
+    rng = np.random.default_rng(12)
+    m = rng.lognormal(-1.0, 0.5, (h, w, 3)).astype(np.float32).astype(np.float64)
+    aov = (rng.random((h, w, 7), dtype=np.float32) * n).astype(np.float32)
+    film = {"sum": m * n, "sumsq": m * m * n * 1.1, "comp": np.zeros((h, w, 3), np.float32), "aov": aov, "samples": n}
+    sc = scenes.upload(ctx, scenes.cornell())
+    sc.build()
+    net = salty_gb300.Unet(ctx, seed=4)
+    sc.restore(film, w, h)
+    whole = net.denoise_film(sc, mirrors=8)
+    band = {k: np.ascontiguousarray(v[y0:y1]) if isinstance(v, np.ndarray) else v for k, v in film.items()}
+    sc.restore(band, w, y1 - y0)
+    part = net.denoise_film(sc, mirrors=8)
+    net.close()
+    sc.close()
+    np.testing.assert_array_equal(whole[y0 + margin:y1 - margin], part[margin:-margin])
