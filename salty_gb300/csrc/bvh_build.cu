@@ -935,8 +935,9 @@ __device__ int collapse_children(const BNode* __restrict__ bn, const CollapseDP*
 // and work[..] names their binary nodes; their children follow them in out, counted in
 // cnt8[level + 1].  Quantisation is exact in FP32: a plane's grid index is the floor (ceiling)
 // of (plane - origin) / 2^e, every index of 8 bits times 2^e is a float, so rounding the
-// difference down (up) first cannot move it across an index (64-bit divisions took half of
-// this kernel: 1.11 -> 0.41 ms for 1M triangles, with one atomic per warp instead of per node).
+// difference down (up) first cannot move it across an index; where the quotient is so small that
+// it rounds to zero, the ceiling of a positive difference is still one (64-bit divisions took half
+// of this kernel: 1.11 -> 0.41 ms for 1M triangles, with one atomic per warp instead of per node).
 __global__ void __launch_bounds__(128) k_collapse(int level, const BNode* __restrict__ bn, const int* __restrict__ work,
                                                   Bvh8Node* __restrict__ out, float4* __restrict__ tris,
                                                   const int* __restrict__ prim, const float* __restrict__ pos,
@@ -1024,7 +1025,8 @@ __global__ void __launch_bounds__(128) k_collapse(int level, const BNode* __rest
                 BNode c = bn[set[i]];
                 for (int a = 0; a < 3; ++a) {
                     const float lo = floorf(__fsub_rd(c.lo[a], b.lo[a]) * inv[a]);
-                    const float hi = ceilf(__fsub_ru(c.hi[a], b.lo[a]) * inv[a]);
+                    const float up = __fsub_ru(c.hi[a], b.lo[a]);
+                    const float hi = fmaxf(ceilf(up * inv[a]), up > 0.0f ? 1.0f : 0.0f);
                     qlo[a][s] = (unsigned char)fminf(fmaxf(lo, 0.0f), 255.0f);
                     qhi[a][s] = (unsigned char)fminf(fmaxf(hi, 0.0f), 255.0f);
                 }

@@ -472,3 +472,23 @@ def test_build_workspace_is_given_back(salty_lib):
         other.close()
         s.close()
         assert before - free() <= slack
+
+
+# A box of 2^-60 in a node of 2^100: its upper plane is an index of one, not of zero, so a ray
+# that starts inside meets what is there.
+@pytest.mark.parametrize("watertight", [False, True])
+def test_tiny_boxes_in_huge_nodes(ctx, watertight):
+    tris = np.zeros((20, 3, 3), np.float32)
+    tris[:, 0, 1:], tris[:, 1, 1:], tris[:, 2, 1:] = (0.0, 0.0), (0.8, 0.0), (0.0, 0.8)
+    tris[:, :, 1] += np.arange(20, dtype=np.float32)[:, None]
+    tris[:16:2, :, 0] = 2.0 ** -60
+    tris[16:, :, 0] = 2.0 ** 100
+    sc = _scene(ctx, tris.reshape(-1, 9))
+    near = np.arange(0, 16, 2)
+    rays = np.zeros((len(near), 8), np.float32)
+    rays[:, 0], rays[:, 1], rays[:, 2] = 2.0 ** -61, near + 0.2, 0.2
+    rays[:, 4], rays[:, 7] = 1.0, np.inf
+    res = sc.trace(rays, watertight=watertight)
+    np.testing.assert_array_equal(res.ids, near)
+    np.testing.assert_array_equal(res.t, np.full(len(near), 2.0 ** -61, np.float32))
+    sc.close()
