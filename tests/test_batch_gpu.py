@@ -132,3 +132,44 @@ def test_host_loop_renders_the_same_films(ctx, batch, monkeypatch):
     monkeypatch.setenv("SALTY_RENDER_HOST_LOOP", "1")
     ctx.render_batch(ss, opts)
     _same(_films(ss, opts), ref)
+
+
+# Frames launched straight into the streams (paths of up to 16 segments that all start at once) and
+# frames run as a graph (longer paths, or more samples than the queue), against the host loop.
+@pytest.mark.parametrize("depth,wave", [(1, 1 << 24), (16, 1 << 24), (17, 1 << 24), (16, 1 << 16), (17, 1 << 16)])
+def test_direct_and_graph_frames_equal_the_host_loop(ctx, batch, monkeypatch, depth, wave):
+    ss, _ = batch
+    opts = [dict(width=96, height=90, spp=8, max_depth=depth, seed=7), dict(width=40, height=30, spp=3, max_depth=depth, seed=8)]
+    two = [ss[1], ss[2]]
+    default = ctx.tuning
+    ctx.tuning = {"wave_paths": wave}
+    try:
+        got = _alone(two, opts)
+        ctx.render_batch(two, opts)
+        _same(_films(two, opts), got)
+        monkeypatch.setenv("SALTY_RENDER_HOST_LOOP", "1")
+        _same(_alone(two, opts), got)
+    finally:
+        ctx.tuning = default
+
+
+# The queueing walk (the default in trees of four levels or more) at a render's smallest queues:
+# around a warp, a refill and a warp's least share of rays, bit for bit against the walk in which
+# lanes test their own triangles.
+@pytest.mark.parametrize("w,h", [(1, 1), (5, 1), (6, 1), (31, 1), (33, 1), (28, 25)])
+@pytest.mark.parametrize("compat", [False, True])
+def test_small_queues_in_either_walk(ctx, batch, w, h, compat):
+    import salty_gb300
+    ss, _ = batch
+    default = ctx.tuning
+    for s in ss[2:4]:
+        assert s.info["depth"] > 3
+        o = [dict(width=w, height=h, spp=1, max_depth=6, seed=w,
+                  profile=salty_gb300.PROFILE_COMPAT if compat else salty_gb300.PROFILE_PHYSICAL)]
+        got = _alone([s], o)
+        ctx.tuning = {"trace_postpone": 2}
+        try:
+            own = _alone([s], o)
+        finally:
+            ctx.tuning = default
+        _same(got, own)

@@ -218,3 +218,27 @@ def test_weight_gradient_operands_and_columns():
             for j in range(nx):
                 base = (tap // 3 * nx + j) * 48 + tap % 3 * 16
                 assert [cols[base + c] for c in range(16)] == [(tap // 3, j, tap % 3, c) for c in range(16)]
+
+
+def test_tma_kernel_layout_at_every_strip_height(k, launches):
+    """k_conv3x3_tma's shared memory at every strip height the launcher can take: the header's
+    barriers, TMEM address and abort flag end before the bias table at byte 512, the table before
+    the weights, at least two stages fit, and boxes stay inside their stages."""
+    s = _src("conv_tc.cu")
+    chunks = _const(s, "kTmaMaxChunks")
+    assert "uint64_t wbar[kTmaMaxChunks];" in s and "smem + 512" in s
+    assert (2 * k["kMaxStages"] + 4 + chunks) * 8 + 8 <= 512
+    for kind, cin, cout, wrows in launches:
+        R0, npad = rows(k, cout)
+        assert 512 + 4 * npad <= k["kTmaHeader"] and cin // 16 <= chunks
+        wts, wbytes = (9 * npad * 32 + 1023) // 1024 * 1024, cin // 16 * 9 * npad * 32
+        resident = wbytes <= k["kResidentMaxBytes"]
+        wres = (wbytes + 1023) // 1024 * 1024 if resident else 0
+        for R in range(min(2, R0), R0 + 1):
+            halo = ((R + 2) * k["kHaloW"] * 32 + 1023) // 1024 * 1024
+            stage = halo if resident else halo + wts
+            S = min(k["kMaxStages"], (SMEM_MAX - k["kTmaHeader"] - wres) // stage)
+            smem = max(k["kTmaHeader"] + wres + S * stage, k["kTmaMinSmem"])
+            assert S >= 2 and SMEM_SM // 2 < smem <= SMEM_MAX, (kind, cin, cout, R)
+            assert stage % 1024 == 0 and 16 * k["kHaloW"] * (R + 2) * 2 <= halo and 2 * R * npad <= 512
+            assert 16 * k["kHaloW"] * (R + 2) * 2 + wbytes // (cin // 16) < 1 << 20  # transaction bytes of a stage
