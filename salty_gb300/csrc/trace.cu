@@ -230,6 +230,8 @@ k_trace_queue(const Bvh8Node* __restrict__ nodes, const float4* __restrict__ tri
     unsigned long long* keys = reinterpret_cast<unsigned long long*>(sstack + (depth + 1) * TB) + (threadIdx.x & ~31);
     uint2* queue = sstack + (depth + 2) * TB + (threadIdx.x >> 5) * kQueue;  // (triangle, lane)
     uint2* uvs = sstack + depth * TB + (threadIdx.x & ~31);
+    // the rays' own limits (WT), after the block's queues
+    float* tmaxs = reinterpret_cast<float*>(sstack + (depth + 2) * TB + TB / 32 * kQueue) + (threadIdx.x & ~31);
     const int n = n_dev ? *n_dev : (int)n_arg;
     TravCount cnt{0, 0};
     int overflow = 0;
@@ -271,6 +273,7 @@ k_trace_queue(const Bvh8Node* __restrict__ nodes, const float4* __restrict__ tri
                 make_trav_ray(r, ra.x, ra.y, ra.z, ra.w, rb.x, rb.y, rb.z);
                 trav_init(s, r, rb.w, roots ? (unsigned)__ldcs(roots + rid) : 0u);
                 keys[lane] = ((unsigned long long)__float_as_uint(s.hit.t) << 32) | kNoHit;
+                if (WT) tmaxs[lane] = rb.w;
                 walking = true;
             }
             pool_next = min(pool_end, pool_next + __popc(idle_mask));
@@ -315,14 +318,13 @@ k_trace_queue(const Bvh8Node* __restrict__ nodes, const float4* __restrict__ tri
                     w.dz = __shfl_sync(m, r.dz, o);
                 }
                 const float tlim = __shfl_sync(m, s.hit.t, o);
-                const int orid = WT ? __shfl_sync(m, rid, o) : 0;
                 bool h = false;
                 float t = 0.0f, u = 0.0f, v = 0.0f;
                 unsigned long long key = 0;
                 if (live) {
                     const float4* tp = tris + (size_t)e.x * kTriFloat4;
                     const float4 a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
-                    h = WT ? tri_watertight(w, a, b, c, w.tmin, tlim, ray_tmax(rays, orid), t, u, v)
+                    h = WT ? tri_watertight(w, a, b, c, w.tmin, tlim, tmaxs + o, t, u, v)
                            : tri_ref(w, a, b, c, w.tmin, tlim, tlim, t, u, v);
                     if (h) key = hit_key(t, a.w);
                 }
@@ -428,7 +430,7 @@ salty_status launch(salty_ctx* ctx, const Launch& L) {
 template <bool ANY, bool WT, int TB>
 salty_status launch_queue(salty_ctx* ctx, const Launch& L) {
     auto kern = k_trace_queue<ANY, WT, TB>;
-    const size_t smem = ((size_t)(L.depth + 2) * TB + (size_t)(TB / 32) * kQueue) * sizeof(uint2);
+    const size_t smem = ((size_t)(L.depth + 2) * TB + (size_t)(TB / 32) * kQueue) * sizeof(uint2) + (WT ? TB * sizeof(float) : 0);
     if (smem > 48 * 1024)
         SALTY_TRY_CUDA(ctx->err, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;

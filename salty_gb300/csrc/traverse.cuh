@@ -163,7 +163,7 @@ __device__ __forceinline__ bool tri_watertight(const TravRay& r, float4 a, float
     v = __fmul_rn(W, rcp);
     if (!(t >= tmin) || t > tfar) return false;
     if (det > 0.0f ? T > __fmul_rn(tfar, det) : T < __fmul_rn(tfar, det)) {
-        const float lim = __fmul_rn(__ldg(tmax), det);
+        const float lim = __fmul_rn(*tmax, det);
         if (det > 0.0f ? T > lim : T < lim) return false;
     }
     return true;
