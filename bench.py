@@ -58,12 +58,12 @@ SOUP_SEED, RAY_SEED = 20260001, 20260002
 TMIN = 1e-4
 METRIC = "Mrays/s"
 CPU_SAMPLE = 2_097_152      # rays of the same stream timed on the host cores (~10 s of CPU work)
-# DRAM bytes (read + write) per ray of the closest-hit k_trace launch, from one ncu capture
-# of that kernel at the default launch shape (128 threads, 56 registers, pool 64, no
+# DRAM bytes (read + write) per ray of the closest-hit k_trace_queue launch, from one ncu capture
+# of that kernel at the default launch shape (128 threads, 64 registers, pool 64, no
 # triangle postponing) on the same soup at 4,194,304 rays; the traffic (rays in, hits out,
 # L2 misses) scales with the ray count, so traffic per launch is this figure times the rays
 # of the launch.
-NCU_DRAM_BYTES_PER_RAY = (344.759552e6 + 65.560576e6) / 4_194_304
+NCU_DRAM_BYTES_PER_RAY = (341.545472e6 + 64.932096e6) / 4_194_304
 
 
 def measured_peaks_tensor() -> dict:
@@ -827,7 +827,10 @@ def main():
     else:
         tuning, tune_ms = scene.autotune_trace(d_rays, any_hit=any_hit)
 
-    # fetch counts (untimed): algorithmic bytes per ray
+    # fetch counts (untimed): algorithmic bytes per ray.  The counting walk is the one in which
+    # lanes test their own triangles; it culls earlier than the queueing walk that is timed (34.0
+    # nodes and 5.4 triangles per closest-hit ray against 36.2 and 6.0), so these bytes are what the
+    # work needs, not all that the timed kernel fetches.
     st = scene.trace_raw(d_rays, d_hits, any_hit=any_hit, counters=True)
     n_node = st["node_fetches"] / n_rays
     n_tri = st["tri_fetches"] / n_rays

@@ -256,7 +256,8 @@ enum {
 };
 
 /* Closest or any hit for n rays.  Closest hit: the smallest t the triangle test accepts
- * in [tmin, tmax]; equal t goes to the lowest triangle index.  Misses: id = -1, t = +inf.
+ * in [tmin, tmax]; equal t goes to the lowest triangle index.  Any hit: the first accepted one of
+ * the ray's walk, the same in every call over one BVH under one tuning.  Misses: id = -1, t = +inf.
  * u, v: barycentric weights of v1, v2.  rays/hits: host or device.  Triangle ids are
  * scene input indices. */
 salty_status salty_trace(salty_ctx* ctx, salty_scene* scene, const salty_ray* rays, int64_t n,
@@ -326,9 +327,10 @@ salty_status salty_render_batch(salty_ctx* ctx, salty_scene* const* scenes, cons
 typedef struct salty_tuning {
     int32_t trace_block;     /* traversal threads per block: 64, 128 or 256 */
     int32_t trace_pool;      /* rays a warp takes from the queue per refill, 32..4096 */
-    int32_t trace_postpone;  /* fewest lanes that test a triangle group together, 1..32; at 1,
-                              * in deeper trees and for more rays than the chip has lanes, a
-                              * warp queues its triangles and tests them together */
+    int32_t trace_postpone;  /* fewest lanes that test a triangle group together, 1..32; at 1, a
+                              * warp queues its triangles and tests them together in renders of
+                              * trees of four levels or more, and in trace calls of more rays
+                              * than the chip has lanes in deeper trees */
     int32_t shade_block;     /* shading threads per block, a multiple of 32 in 64..1024 */
     int32_t trace_regs;      /* traversal registers per thread: 64, or 56 (more resident warps;
                               * the queueing walk always takes 64) */

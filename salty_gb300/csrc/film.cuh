@@ -5,7 +5,7 @@
 // both products are 48 bits, held as pairs of FP32 numbers, and their difference keeps every
 // rounding error as a further term (error-free products and differences: Dekker 1971, Knuth
 // TAOCP 2, 4.2.2).  So the variance is the exact one rounded once, whatever cancels: 0.50 units
-// in the last place at every spread, where FP64 quotients reach 0.55 at a variance of 2^-23 of
+// in the last place at every spread, where FP64 quotients reach 0.60 at a variance of 2^-23 of
 // the squared mean and 4 at 2^-24.  FP64 runs at a 64th of the FP32 rate here and its three
 // divisions per value took 436 us of a 1080p film read-out, this form 32 us (bound by the film's
 // bytes).  The mean is the correctly rounded quotient either way (53 >= 2 * 24 + 2 bits).  Sums

@@ -248,7 +248,7 @@ struct Tuning {
     // Paths in flight (queue capacity).  Every traversal launch ends with a tail of a few
     // long walks; freed queue slots are refilled with new samples each iteration, so the
     // launches stay full and a moderate queue already amortises the tails (1080p
-    // heightfield, 64 spp: 1,984 Mrays/s at 2^22, 2,173 at 2^24, 2,235 at 2^26).  352 bytes
+    // heightfield, 64 spp: 1,979 Mrays/s at 2^22, 2,164 at 2^24, 2,227 at 2^26).  352 bytes
     // of path state per path plus 48 bytes per sample of the per-sample buffers: about 11 GB
     // at 2^24 for a depth-12 render.
     long long wave_paths = 1ll << 24;

@@ -4,8 +4,9 @@
 //   reduction, then a per-pixel curve (Reinhard, Uncharted2, ACES) fused with the clamp,
 //   OETF and 8-bit rounding of PathTracer::Capture (src/s3d_pt.cpp:145-171).  Both passes
 //   stream the image once (HBM bound); per-pixel arithmetic keeps the reference's
-//   operation order with separately rounded products.  The reduction sums log terms in
-//   double, where the reference adds them one by one in single precision.
+//   operation order with separately rounded products.  The reduction adds log terms in pairs
+//   of FP32 numbers and the pairs in double (salty_tonemap), or four by four and then in double
+//   (salty_tonemap_noalloc), where the reference adds them one by one in single precision.
 //   FilterNLM (src/s3d_denoiser.cpp:19-95): each block stages its tile plus halo in
 //   shared memory; overlapping patches share their squared differences.
 #include <algorithm>
@@ -229,7 +230,9 @@ struct LumScratch {
 // the block that finishes last adds them in index order, so one launch does it and the sum does
 // not depend on the order of the blocks.  rgb 16-byte aligned (vec): four pixels per step.  A
 // thread's logarithms are added as an unevaluated FP32 pair (Knuth's TwoSum, 48 bits), since FP64
-// runs at a 64th of the rate; pairs meet in FP64.  The average is exp of the FP32 mean; taken in
+// runs at a 64th of the rate; pairs meet in FP64.  A thread adds 18 terms at 1080p and 72 at 4K,
+// which a pair holds without any error (FP32 logarithms of images; 2,300 terms at 16,384^2: 1e-9
+// of the FP32 mean's rounding).  The average is exp of the FP32 mean; taken in
 // FP64 and rounded it is nearly always the host's expf (the caller compares).
 // Bound: the logarithms' and additions' issue and the latency of a handful of loads.
 __device__ __forceinline__ void two_sum(float& hi, float& lo, float x) {

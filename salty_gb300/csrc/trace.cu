@@ -25,9 +25,11 @@ constexpr int kMaxStack = 63;  // stack entries per thread: BVHs up to 31 levels
 // ones); longer arrays are traced in consecutive launches of at most this many rays.
 constexpr long long kMaxLaunchRays = 1ll << 30;
 
-// A launch with fewer rays than lanes spreads them: a warp takes no more than its share of the
-// rays, but at least kMinPool (30k triangles, 4,096 rays: 173 us per call at 64 rays per warp,
-// 159 at 1, 134 at 16).
+// Few rays are shared out: a warp takes no more than its share of them, but at least kMinPool, so
+// that none takes 64 and leaves the others idle (30k triangles: 4,096 rays 150 us per call
+// with pools of 64, 102 so; 100,000 rays 203 and 151; 1M triangles: 277 and 224, 354 and 312).
+// k_trace's grid holds a lane per ray, so a caller's few rays are 32 to a warp there, on as
+// many SMs as their blocks fill; the least share is for queues whose length only the device knows.
 constexpr int kMinPool = 16;
 
 // k_trace: lanes test their own triangles -- two-level scenes, spheres, counting walks,
@@ -194,8 +196,9 @@ k_trace(const Bvh8Node* __restrict__ nodes, const float4* __restrict__ tris, con
 // queue together, one (ray, triangle) pair per lane.  In k_trace a test runs with the four to
 // five lanes that hold triangles at that step, once or twice a step, a third to a half of its
 // instructions; here about once in three steps with most lanes.  A lane walks on meanwhile with
-// the best distance it knows, which never changes the answer, only how early boxes are culled;
-// when its walk is over it waits for its own pairs.  The queue is tested once it holds as many
+// the best distance it knows, which changes how early boxes are culled (36.2 nodes and 6.0
+// triangles per ray of the microbenchmark, 34.0 and 5.4 in k_trace) and not the answer: both
+// tests bound a hit by its rounded distance alone.  When its walk is over it waits for its own pairs.  The queue is tested once it holds as many
 // pairs as lanes are walking (half or a quarter as many: 1 and 5 % slower), and idle lanes take
 // new rays kRefill at a time, since a refill costs the warp about a node step and a trip to
 // memory however many lanes it fills (1 at a time: 5 % slower).
@@ -453,18 +456,21 @@ template <int TB, bool CAP>
 salty_status dispatch_flags(salty_ctx* ctx, const Launch& L, uint32_t flags) {
     const bool any = flags & SALTY_TRACE_ANY_HIT, wt = flags & SALTY_TRACE_WATERTIGHT;
     // Lanes test their own triangles where that is asked for (postponing), and where the queue
-    // gains nothing:
+    // gains nothing (us per call, own tests / queued):
     // - trees of up to three levels, where nearly every step ends in leaves and most lanes hold
-    //   triangles (the 36-triangle Cornell box, 256 x 256 at 16 spp: 1.64 ms against 1.68);
+    //   triangles (the 36-triangle Cornell box, 256 x 256 at 16 spp: 1,380 / 1,415);
     // - a caller's rays, no more of them than the chip has lanes, where the time is that of one
-    //   walk and waiting for a queue lengthens it (100k triangles, reference's test, 100,000 rays:
-    //   252 us against 289; 400,000 rays: 543 against 511);
+    //   walk and waiting for a queue lengthens it (100,000 rays: 20k triangles 129 / 174, 100k
+    //   223 / 276, 1M 313 / 375; watertight 138 / 186, 237 / 290, 336 / 386);
     // - a caller's rays in shallow trees, whose walks are so short that refilling and queueing cost
-    //   more than fuller tests save (2M rays of a soup, own against queued: reference's test 0.66
-    //   and 0.76 ms at 6,000 triangles and 6 levels, 1.67 and 1.69 at 100k and 7, 1.84 and 1.81 at
-    //   200k and 8; watertight test 1.10 and 1.14 ms at 20k and 6, 1.54 and 1.47 at 50k and 7).
-    // Renders queue from four levels on: their rays meet larger leaves (960 x 540 terrain of 8,192
-    // triangles at 8 spp: 2.78 ms against 2.51).
+    //   more than fuller tests save.  The line lies where a million rays are as fast either way:
+    //   reference's test 562 / 622 at 20k triangles and 6 levels, 908 / 938 at 100k and 7, 1,018 /
+    //   1,017 at 200k and 8, 980 / 942 at 1M and 9; watertight test 603 / 612 at 20k and 6, 820 /
+    //   788 at 50k and 7, 1,143 / 1,044 at 200k and 8.  Ray counts move it by less than 5 % (400,000
+    //   rays, 100k triangles: 499 / 498).
+    // Renders queue from four levels on, at any size: their rays meet larger leaves (terrain at 1 spp
+    // in 8 levels, 16 x 16: 506 / 480, 512 x 512: 1,242 / 1,179; in 10 levels 805 / 732 and 2,058 /
+    // 1,806; only in 7 levels or fewer up to 6 % the other way).
     const bool caller = !L.n_dev && (L.n <= 1024ll * ctx->num_sms || L.tgt.depth <= (wt ? 6 : 7));
     const bool own = L.postpone > 1 || L.tgt.depth <= 3 || caller;
 #define SALTY_L(A, W) \

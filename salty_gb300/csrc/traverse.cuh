@@ -220,9 +220,13 @@ __device__ __forceinline__ float fmin4(float a, float b, float c, float d) {
     return fminf(m, d);
 }
 
-// Widening of the far plane (tn >= tmin >= 0): covers the rounding of the decoded
-// planes, of 1/d and of the fused plane evaluation, so the quantised-box test never
-// rejects a box the exact ray segment meets.
+// Widening of the far plane (tn >= tmin >= 0) over the rounding of the decoded planes, of 1/d
+// and of the fused plane evaluation.  With M the larger of the node's extent and its distance from
+// the ray's origin along an axis, over d, that rounding is up to 2^-22 M: for t above M / 32 a
+// quantised box is met wherever the exact one is.  For nearer t the widening is smaller than the
+// rounding, and what keeps a box is the outward quantisation of its planes.  Hits at 0 to 1e-4
+// are found all the same: 2^20 rays leaving the triangles of a 300k soup, and 1e-6 to 1e-4
+// beside them, give the oracle's ids under both tests.
 constexpr float kBoxSlackMul = 1.0f + 1.0f / (1 << 17);
 
 // Two FP32 values in one 64-bit register pair, for the packed FP32 instructions of sm_100
