@@ -214,6 +214,7 @@ struct WaveBuffers {
 constexpr long long kMaxRingChunks = 16;  // per-sample buffers: at most 16 chunks of half a queue
 constexpr long long kMinSplit = 1 << 16;  // queues of at least this many paths run as two halves
 constexpr int kDirectDepth = 16;           // longest paths of a render launched without a graph
+constexpr int kDirectStep = 8;             // its iterations between looks at what is left
 constexpr int kLaunchIters = 256;          // iterations per graph launch (cancellation granularity)
 
 // Control words of the regenerating wavefront (ctl[]).
@@ -1781,19 +1782,24 @@ salty_status render_batch(salty_ctx* ctx, salty_scene* const* scenes, const salt
         return SALTY_OK;
     };
     // A render whose samples all start at once (one generation) and whose paths are short ends
-    // after max_depth iterations and a single accumulation, so its launches go straight into
-    // the streams: nothing to instantiate, no generation or control launch per iteration, and
-    // the halves meet only at the end.  (256 x 256 Cornell box at 16 spp: 1.68 -> 1.36 ms; a 16 x 16
-    // frame at depth 8: 0.66 -> 0.49 ms.)  Longer paths keep the graph, which stops once all paths have ended.
+    // after max_depth iterations, so its launches go straight into the streams: nothing to
+    // instantiate, no generation or control launch per iteration, and the halves meet only at the
+    // end.  (256 x 256 Cornell box at 16 spp: 1.68 -> 1.36 ms; a 16 x 16 frame at depth 8: 0.66 ->
+    // 0.49 ms.)  Its iterations are launched whether paths are left or not, at 15 to 30 us each, so
+    // the host looks after every kDirectStep of them: a lone triangle at depth 16, whose paths end
+    // in the second iteration, takes 306 us at 16 x 16 (443 without the look, 333 as a graph) and
+    // 967 at 512 x 512 and 16 spp (1,202, 1,041); a look where paths go on costs about 15 us.
+    // Longer paths keep the graph, which stops once all paths have ended.
     const bool direct = !host_loop && samples <= cap && ring >= samples && max_depth <= kDirectDepth;
-    auto run_direct = [&]() -> salty_status {
+    auto run_direct = [&](int first) -> salty_status {
+        const int end = std::min(first + kDirectStep, max_depth);
         if (split) SALTY_TRY(fork());
-        for (int it = 0; it < max_depth; ++it) {
+        for (int it = first; it < end; ++it) {
             SALTY_TRY(run_half(BA, P.cap_a, st, it & 1, it == 0));
             if (split) SALTY_TRY(run_half(BB, P.cap_b, ctx->aux_stream, it & 1, it == 0));
         }
         if (split) SALTY_TRY(join());
-        k_accumulate<<<agrid, 256, 0, st>>>(P, BA, BB, (max_depth - 1) & 1, more, 0);
+        k_accumulate<<<agrid, 256, 0, st>>>(P, BA, BB, (end - 1) & 1, more, 0);
         return SALTY_OK;
     };
     cudaGraph_t graph = nullptr;
@@ -1846,7 +1852,8 @@ salty_status render_batch(salty_ctx* ctx, salty_scene* const* scenes, const salt
     for (long long launch = 0;; ++launch) {
         if (launch > max_launches) { rs = E.fail(SALTY_ERR_TIMEOUT, "render made no progress"); break; }
         if (direct) {
-            rs = launch == 0 ? run_direct() : E.fail(SALTY_ERR_TIMEOUT, "render left samples behind");
+            rs = launch * kDirectStep < max_depth ? run_direct((int)launch * kDirectStep)
+                                                  : E.fail(SALTY_ERR_TIMEOUT, "render left samples behind");
             if (rs != SALTY_OK) break;
         } else if (host_loop) {
             k_launch_begin<<<1, 1, 0, st>>>(P, BA);
