@@ -445,8 +445,9 @@ salty_status salty_trace(salty_ctx* ctx, salty_scene* sc, const salty_ray* rays,
         ctx->last_trace = stats;
         return SALTY_OK;
     }
-    const bool din = is_device_ptr(rays) && ((uintptr_t)rays % 16 == 0);
-    const bool dout = is_device_ptr(hits) && ((uintptr_t)hits % 16 == 0);
+    const cudaMemoryType rays_at = memory_type(rays), hits_at = memory_type(hits);
+    const bool din = is_device_memory(rays_at) && ((uintptr_t)rays % 16 == 0);
+    const bool dout = is_device_memory(hits_at) && ((uintptr_t)hits % 16 == 0);
     cudaStream_t st = ctx->stream;
     cudaEvent_t t0 = ctx->ev[2], k1 = ctx->ev[4], t1 = ctx->ev[5];
     unsigned long long counts[3] = {0, 0, 0};
@@ -475,11 +476,28 @@ salty_status salty_trace(salty_ctx* ctx, salty_scene* sc, const salty_ray* rays,
     } else {
         // Host arrays: chunks alternate between two device slots so the copies of one
         // chunk overlap the traversal of the other.  2^21 rays each (other sizes are slower over
-        // 16M rays), or half the array where that is less, so that both slots work: 1.5M rays in
-        // 5,000 triangles 849 -> 689 us, 2.5M watertight in 1M triangles 2,479 -> 2,438; a third
-        // or a quarter of it 1 to 5 % slower, since each launch has its own drain.  Below 2^18
-        // rays another launch costs what it hides.
-        const long long chunk = std::min<long long>(1ll << 21, std::max<long long>(1ll << 18, (n + 1) / 2));
+        // 16M rays), or half the array where that is less, so that both slots work; a third
+        // or a quarter of it 1 to 5 % slower, since each launch has its own drain.  An array goes
+        // whole where the copies hidden are less than that drain, which grows with the tree (us per
+        // call, whole / in halves, reference's test):
+        // - copies of pageable memory hide nothing (1M triangles: 400,000 rays 687 / 976, a
+        //   million 1,209 / 1,493);
+        // - up to five levels: halves from 2^18 rays on whichever array is on the host (1,000
+        //   triangles, a million rays: hits on the device 361 / 298, rays 281 / 251);
+        // - both arrays pinned: six levels as five (30,000 triangles: 400,000 rays 447 / 437, a
+        //   million 882 / 804), seven from 3 2^18 (100,000: 524,288 rays 698 / 726, 2^20 1,194 /
+        //   1,156), more from 5 2^18 (1M: 2^20 rays 1,213 / 1,245, 2.5M 2,372 / 2,335);
+        // - hits on the device: six and seven levels from 2^20 (30,000: 524,288 rays 476 / 506,
+        //   2^20 824 / 788; 100,000: 1,108 / 1,110), more from 2^21 (1M: 2^20 rays 1,135 / 1,200,
+        //   2.5M 2,342 / 2,215);
+        // - rays on the device leave too little to hide (2.5M rays: 30,000 triangles 1,441 / 1,514,
+        //   1M 2,040 / 2,113).
+        constexpr long long k18 = 1ll << 18, never = 1ll << 62;
+        constexpr long long least[3][4] = {
+            {k18, k18, 3 * k18, 5 * k18}, {k18, 4 * k18, 4 * k18, 8 * k18}, {k18, never, never, never}};
+        const bool halves = n >= least[din ? 2 : dout ? 1 : 0][std::clamp(sc->bvh.depth, 5, 8) - 5] &&
+                            rays_at != cudaMemoryTypeUnregistered && hits_at != cudaMemoryTypeUnregistered;
+        const long long chunk = halves ? std::min<long long>(1ll << 21, std::max<long long>(k18, (n + 1) / 2)) : 1ll << 21;
         const long long nch = (n + chunk - 1) / chunk;
         const long long slot_rays = std::min<long long>(chunk, n);
         SALTY_TRY_CUDA(E, ctx->ray_buf.ensure((size_t)2 * 2 * slot_rays));

@@ -384,13 +384,17 @@ __device__ __forceinline__ void grid_turn() {
 }
 #endif
 
-inline bool is_device_ptr(const void* p) {
-    if (!p) return false;
+// Where an array is: device or managed memory, host memory that the copy engines reach by
+// themselves, or (cudaMemoryTypeUnregistered) pageable memory, whose copies hold the host up.
+inline cudaMemoryType memory_type(const void* p) {
+    if (!p) return cudaMemoryTypeUnregistered;
     cudaPointerAttributes a;
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         cudaGetLastError();
-        return false;
+        return cudaMemoryTypeUnregistered;
     }
-    return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
+    return a.type;
 }
+inline bool is_device_memory(cudaMemoryType t) { return t == cudaMemoryTypeDevice || t == cudaMemoryTypeManaged; }
+inline bool is_device_ptr(const void* p) { return is_device_memory(memory_type(p)); }
 }  // namespace salty

@@ -492,3 +492,26 @@ def test_tiny_boxes_in_huge_nodes(ctx, watertight):
     np.testing.assert_array_equal(res.ids, near)
     np.testing.assert_array_equal(res.t, np.full(len(near), 2.0 ** -61, np.float32))
     sc.close()
+
+
+# Pinned arrays of more than 2^18 rays go in halves in trees of six levels; pageable ones, whose
+# copies overlap nothing, and those of which one stays on the device go whole.  The hits are the same.
+@pytest.mark.parametrize("n", [1 << 18, (1 << 19) + 3])
+def test_chunks_of_pinned_and_pageable_arrays(ctx, n):
+    import salty_gb300
+    import torch
+    sc = _scene(ctx, salty_gb300.microbench_soup(3, 30000))
+    assert sc.info["depth"] == 6
+    rays = salty_gb300.microbench_rays(4, n, 1e-4)
+    pinned_rays, pinned_hits, dev_hits = ctx.pinned((n, 8)), ctx.pinned((n, 4)), torch.empty((n, 4), device="cuda")
+    pinned_rays[:] = rays
+    pageable = lambda: np.empty((n, 4), np.float32)
+    hits = {}
+    for name, r, h in (("pageable", rays, pageable()), ("pinned", pinned_rays, pinned_hits),
+                       ("rays pinned", pinned_rays, pageable()), ("to the device", pinned_rays, dev_hits)):
+        st = sc.trace_raw(r, h)
+        assert st["launches"] == (2 if name == "pinned" and n > 1 << 18 else 1), name
+        hits[name] = (h.cpu().numpy() if h is dev_hits else h).view(np.uint32).copy()
+    for name in hits:
+        np.testing.assert_array_equal(hits[name], hits["pageable"])
+    sc.close()
