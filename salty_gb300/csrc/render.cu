@@ -214,7 +214,7 @@ struct WaveBuffers {
 constexpr long long kMaxRingChunks = 16;  // per-sample buffers: at most 16 chunks of half a queue
 constexpr long long kMinSplit = 1 << 16;  // queues of at least this many paths run as two halves
 constexpr int kDirectDepth = 16;           // longest paths of a render launched without a graph
-constexpr int kDirectStep = 8;             // its iterations between looks at what is left
+constexpr int kDirectLook = 8;             // iterations after which it looks at what is left
 constexpr int kLaunchIters = 256;          // iterations per graph launch (cancellation granularity)
 
 // Control words of the regenerating wavefront (ctl[]).
@@ -1802,20 +1802,40 @@ salty_status render_batch(salty_ctx* ctx, salty_scene* const* scenes, const salt
     // instantiate, no generation or control launch per iteration, and the halves meet only at the
     // end.  (256 x 256 Cornell box at 16 spp: 1.68 -> 1.36 ms; a 16 x 16 frame at depth 8: 0.66 ->
     // 0.49 ms.)  Its iterations are launched whether paths are left or not, at 15 to 30 us each, so
-    // the host looks after every kDirectStep of them: a lone triangle at depth 16, whose paths end
-    // in the second iteration, takes 306 us at 16 x 16 (443 without the look, 333 as a graph) and
-    // 967 at 512 x 512 and 16 spp (1,202, 1,041); a look where paths go on costs about 15 us.
+    // the host looks at the queues after kDirectLook of them, with one more launched to run
+    // meanwhile: a lone triangle at depth 16, whose paths end in the second iteration, takes 312
+    // us at 16 x 16 (443 without the look, 333 as a graph) and 997 at 512 x 512 and 16 spp (1,202,
+    // 1,041); where paths go on the look costs nothing (joining the halves for it: 0.6 % of 1080p
+    // terrain at depth 12).
     // Longer paths keep the graph, which stops once all paths have ended.
     const bool direct = !host_loop && samples <= cap && ring >= samples && max_depth <= kDirectDepth;
-    auto run_direct = [&](int first) -> salty_status {
-        const int end = std::min(first + kDirectStep, max_depth);
+    auto run_direct = [&]() -> salty_status {
+        struct Side {
+            const WaveBuffers& half;
+            long long cap;
+            cudaStream_t st;
+            cudaEvent_t seen;
+        } sides[2] = {{BA, P.cap_a, st, ctx->ev[6]}, {BB, P.cap_b, ctx->aux_stream, ctx->ev[7]}};
+        const int n_sides = split ? 2 : 1;
+        volatile int* left = static_cast<int*>(ctx->pinned);
+        int it = 0;
         if (split) SALTY_TRY(fork());
-        for (int it = first; it < end; ++it) {
-            SALTY_TRY(run_half(BA, P.cap_a, st, it & 1, it == 0));
-            if (split) SALTY_TRY(run_half(BB, P.cap_b, ctx->aux_stream, it & 1, it == 0));
+        for (; it < max_depth; ++it) {
+            if (it == kDirectLook + 1) {
+                for (int k = 0; k < n_sides; ++k) SALTY_TRY_CUDA(E, cudaEventSynchronize(sides[k].seen));
+                if (left[0] == 0 && (!split || left[1] == 0)) break;
+            }
+            for (int k = 0; k < n_sides; ++k) SALTY_TRY(run_half(sides[k].half, sides[k].cap, sides[k].st, it & 1, it == 0));
+            if (it == kDirectLook - 1 && max_depth > kDirectLook + 1)
+                for (int k = 0; k < n_sides; ++k) {
+                    const Side& d = sides[k];
+                    SALTY_TRY_CUDA(E, cudaMemcpyAsync(const_cast<int*>(left + k), d.half.counts + ((it + 1) & 1), sizeof(int),
+                                                      cudaMemcpyDeviceToHost, d.st));
+                    SALTY_TRY_CUDA(E, cudaEventRecord(d.seen, d.st));
+                }
         }
         if (split) SALTY_TRY(join());
-        k_accumulate<<<agrid, 256, 0, st>>>(P, BA, BB, (end - 1) & 1, more, 0);
+        k_accumulate<<<agrid, 256, 0, st>>>(P, BA, BB, (it - 1) & 1, more, 0);
         return SALTY_OK;
     };
     cudaGraph_t graph = nullptr;
@@ -1868,8 +1888,7 @@ salty_status render_batch(salty_ctx* ctx, salty_scene* const* scenes, const salt
     for (long long launch = 0;; ++launch) {
         if (launch > max_launches) { rs = E.fail(SALTY_ERR_TIMEOUT, "render made no progress"); break; }
         if (direct) {
-            rs = launch * kDirectStep < max_depth ? run_direct((int)launch * kDirectStep)
-                                                  : E.fail(SALTY_ERR_TIMEOUT, "render left samples behind");
+            rs = launch == 0 ? run_direct() : E.fail(SALTY_ERR_TIMEOUT, "render left samples behind");
             if (rs != SALTY_OK) break;
         } else if (host_loop) {
             k_launch_begin<<<1, 1, 0, st>>>(P, BA);

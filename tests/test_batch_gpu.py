@@ -175,10 +175,11 @@ def test_small_queues_in_either_walk(ctx, batch, w, h, compat):
         _same(got, own)
 
 
-# Frames launched directly go eight iterations at a time: depths around one and two steps, with paths
-# that last (the room of mirrors and glass) and paths that are over at once (the soup under a sky).
-@pytest.mark.parametrize("depth", [7, 8, 9, 15])
-def test_direct_frames_around_their_steps(ctx, batch, monkeypatch, depth):
+# Frames launched directly look after eight iterations whether any path is left, from depth 10 on:
+# depths around that, with paths that last (the room of mirrors and glass) and paths that are over
+# at once (the soup under a sky).
+@pytest.mark.parametrize("depth", [7, 8, 9, 10, 11, 15])
+def test_direct_frames_around_their_look(ctx, batch, monkeypatch, depth):
     ss, _ = batch
     two = [ss[1], ss[3]]
     opts = [dict(width=48, height=40, spp=6, max_depth=depth, seed=9, rr_depth=depth), dict(width=33, height=21, spp=5, max_depth=depth, seed=10)]
